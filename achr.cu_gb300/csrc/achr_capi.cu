@@ -485,6 +485,10 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
         lu[i] = make_double2(model->lb[i], model->ub[i]);
     }
     ctx->bound_err = berr;
+    ctx->bound_exact = true;
+    for (int i = 0; i < n; ++i)
+        ctx->bound_exact = ctx->bound_exact && achr::f32_exact_bound(model->lb[i]) && achr::f32_exact_bound(model->ub[i]) &&
+                           std::isfinite(model->lb[i]) && std::isfinite(model->ub[i]);
     {
         double bsq = 0.0;
         for (int i = 0; i < n; ++i) bsq += std::max(model->lb[i] * model->lb[i], model->ub[i] * model->ub[i]);
@@ -722,6 +726,7 @@ ChainArgs chain_args(const achr_ctx *ctx, uint64_t seed, uint64_t chain_offset, 
     a.lbub = ctx->lbub.p;
     a.bnd = ctx->bnd.p;
     a.bound_err = ctx->bound_err;
+    a.bound_exact = ctx->bound_exact ? 1 : 0;
     a.dtol_hi = f32_up(ctx->opt.d_tol) * (1.0f + 9.5367431640625e-07f);
     a.dtol_lo = f32_down(ctx->opt.d_tol) * (1.0f - 9.5367431640625e-07f);
     a.utol32 = (float)ctx->opt.u_tol;

@@ -1,4 +1,4 @@
-// Chain-kernel instantiations with 32-128 threads per chain.
+// Chain-kernel instantiations with 32 and 64 threads per chain.
 #include "achr_chain_kernel.cuh"
 
 namespace achr {
@@ -8,11 +8,11 @@ cudaError_t launch_chain_cfg_small(int bd, int ept, const ChainArgs &a, cudaStre
         case 32 * 100 + 4: return launch_cfg<32, 4>(a, s, max_ctas, per_sm);
         case 32 * 100 + 8: return launch_cfg<32, 8>(a, s, max_ctas, per_sm);
         case 64 * 100 + 4: return launch_cfg<64, 4>(a, s, max_ctas, per_sm);
+        case 64 * 100 + 6: return launch_cfg<64, 6>(a, s, max_ctas, per_sm);
         case 64 * 100 + 8: return launch_cfg<64, 8>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 4: return launch_cfg<128, 4>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 8: return launch_cfg<128, 8>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 16: return launch_cfg<128, 16>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 32: return launch_cfg<128, 32>(a, s, max_ctas, per_sm);
+        case 64 * 100 + 12: return launch_cfg<64, 12>(a, s, max_ctas, per_sm);
+        case 64 * 100 + 16: return launch_cfg<64, 16>(a, s, max_ctas, per_sm);
+        case 64 * 100 + 20: return launch_cfg<64, 20>(a, s, max_ctas, per_sm);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -22,11 +22,11 @@ cudaError_t launch_chain_queue_small(int bd, int ept, const ChainQueue &q, cudaS
         case 32 * 100 + 4: return launch_queue_cfg<32, 4>(q, s, grid, per_sm);
         case 32 * 100 + 8: return launch_queue_cfg<32, 8>(q, s, grid, per_sm);
         case 64 * 100 + 4: return launch_queue_cfg<64, 4>(q, s, grid, per_sm);
+        case 64 * 100 + 6: return launch_queue_cfg<64, 6>(q, s, grid, per_sm);
         case 64 * 100 + 8: return launch_queue_cfg<64, 8>(q, s, grid, per_sm);
-        case 128 * 100 + 4: return launch_queue_cfg<128, 4>(q, s, grid, per_sm);
-        case 128 * 100 + 8: return launch_queue_cfg<128, 8>(q, s, grid, per_sm);
-        case 128 * 100 + 16: return launch_queue_cfg<128, 16>(q, s, grid, per_sm);
-        case 128 * 100 + 32: return launch_queue_cfg<128, 32>(q, s, grid, per_sm);
+        case 64 * 100 + 12: return launch_queue_cfg<64, 12>(q, s, grid, per_sm);
+        case 64 * 100 + 16: return launch_queue_cfg<64, 16>(q, s, grid, per_sm);
+        case 64 * 100 + 20: return launch_queue_cfg<64, 20>(q, s, grid, per_sm);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -11,31 +11,41 @@
 //
 // Design (one CTA per chain, persistent over chains):
 //   * The chain's point x and centre accumulator A = (W + t) c live in shared
-//     memory for all T steps; only the warmup column w_r is read from HBM/L2
-//     each step, staged into shared memory by a 1-D TMA bulk copy
-//     (cp.async.bulk + mbarrier) issued one step ahead.
-//   * GB300's FP64 pipe issues about 1.6 DFMA per clock per SM, 72x less than
-//     FP32, and FP64 compares cost as much as FMAs.  Per element and accepted
-//     step the kernel spends exactly three FP64 pipe instructions
-//     (d = w - A/(W+t), x += s d, A += x).  The norm is summed in FP32 (it only
-//     feeds tolerance tests, which carry margins and fall back to FP64 when a
-//     margin is not enough); the ratio test brackets every bound distance and
-//     ratio in FP32 with rigorous error bounds and evaluates in FP64 only the
-//     coordinates whose bracket can hold the minimum; clipping and the min/max
-//     reductions compare FP64 values as integers (order-preserving keys).
-//   * The brackets are formed in the same pass as d, before the block knows
-//     ||d||, so one block reduction serves the norm and the bracket minima
-//     (two barriers per accepted step: that one and the exact minima's).
+//     memory for all T steps.  The warmup column w_r is read from HBM/L2
+//     straight into the registers that hold the direction: each thread owns
+//     pairs of neighbouring reactions (16-byte loads), and as soon as the step
+//     has used a direction pair it requests the next step's column there.  A
+//     chain needs two vectors of shared memory, not the three that a staged
+//     column takes: an SM holds 4 chains of 3072 reactions, 2 of 6656.
+//   * GB300's FP64 pipe takes one warp instruction per 19 clocks and SM (64
+//     clocks for one warp alone), 72x less than FP32, and FP64 compares cost
+//     as much as FMAs.  Per element and accepted step the kernel spends exactly
+//     three FP64 pipe instructions (d = w - A/(W+t), x += s d, A += x).  The
+//     norm is summed in FP32 (it only feeds tolerance tests, which carry
+//     margins and fall back to FP64 when a margin is not enough); the ratio
+//     test brackets every ratio in FP32 with rigorous error bounds and
+//     evaluates in FP64 only the coordinates whose bracket can hold the
+//     minimum; clipping and the min/max reductions compare FP64 values as
+//     integers (order-preserving keys), and the quotients that decide the step
+//     are divided with integer arithmetic (div_rn).
+//   * The FP32 image of x that the clip test forms stays in registers for the
+//     next step's brackets (where registers allow: chain_keeps_x32).
+//   * The brackets are formed in the pass that forms d, before the block knows
+//     ||d||, so they fill the FP64 latency and one block reduction serves the
+//     norm and the bracket minima.  The few contenders meet in shared memory,
+//     and one warp computes the step length (three barriers per accepted step).
 //   * Per-step scalars (warmup index, step uniform, 1/(W+t)) come from a
-//     shared-memory table that the CTA refills once every BD steps.
+//     shared-memory table that the CTA refills once every kTbl steps.
 //   * The element loops are unrolled over compile-time BD x EPT with arrays
 //     padded to that length, so no loop carries a bounds test.
 //   * Reductions are warp shuffles plus one shared-memory exchange in a fixed
-//     order, so a launch is bitwise repeatable.
+//     order, so a launch is bitwise repeatable; a one-warp CTA skips the
+//     exchange.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
 
+#include "achr_div.cuh"
 #include "achr_internal.h"
 #include "achr_rng.cuh"
 
@@ -46,13 +56,14 @@ constexpr float kErrK = 2.384185791015625e-07f;        // 2^-22: bound on trunca
 constexpr float kTiny = 2.350988701644575e-38f;        // 2^-125: absolute error of flushed tiny values
 constexpr float kUp = 1.0f + 9.5367431640625e-07f;     // 1 + 2^-20
 constexpr float kDn = 1.0f - 9.5367431640625e-07f;     // 1 - 2^-20
+constexpr float kQUp = 1.0f + 1.9073486328125e-06f;    // 1 + 2^-19: relative error of a bracketed ratio
+constexpr float kQDn = 1.0f - 1.9073486328125e-06f;
+constexpr float kErrX = 2.4080276489257812e-07f;       // 2^-22 (1 + 2^-6.7): kErrK with room for kQUp and its rounding
 constexpr float kAdUp = 1.0f + 4.76837158203125e-07f;  // 1 + 2^-21
 constexpr float kNormUp = 1.0f + 1e-5f;                // FP32 norm relative error margin
 constexpr float kNormDn = 1.0f - 1e-5f;
-// Lower bound of u_tol ||d|| from u_tol max|d_i|: the FP32 norm of a vector is
-// at least its largest element within (1 - 1e-6), and the threshold carries
-// the kNormDn margin; 0.999 leaves room for both and the products' rounding.
-constexpr float kProvDn = 0.999f;
+constexpr float kDMin = 7.888609052210118e-31f;        // 2^-100: smallest |d| the brackets tell apart
+constexpr float kDCert = 1.5777218104420236e-30f;      // 2^-99: no smaller |d| is a certain candidate
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bounded mbarrier wait: 2 s
 constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 
@@ -68,6 +79,24 @@ __device__ __forceinline__ float f64_to_f32_rz(double v) {
     mag = (fe >= 255) ? 0x7F800000u : mag;
     return __uint_as_float((hi & 0x80000000u) | mag);
 }
+
+// The same for the hot loops, in six integer operations: the magnitude is
+// clamped to [2^LO_EXP, 2^128 (1 - 2^-20)) in its FP64 form (three spare low
+// bits of a clamped value are below the error bound), then the exponent is
+// re-biased with one addition.  |v - f| <= 2^-23 |f| inside the range; below
+// it f is +-2^LO_EXP (1 + 2^-20) at most, above it the largest magnitude.
+template <int LO_EXP>
+__device__ __forceinline__ float f64_to_f32_clamped(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v);
+    const unsigned lo = (unsigned)__double2loint(v);
+    constexpr unsigned kLo = (unsigned)(1023 + LO_EXP) << 20, kHi = 0x47EFFFFFu;
+    const unsigned h = min(max(hi & 0x7FFFFFFFu, kLo), kHi);
+    const unsigned mag = __funnelshift_l(lo, h, 3) + 0x40000000u;  // - (896 << 23)
+    return __uint_as_float((hi & 0x80000000u) | mag);
+}
+// x: clamped at 2^-126 (kTiny covers it); d: clamped at kDMin.
+__device__ __forceinline__ float x_to_f32(double v) { return f64_to_f32_clamped<-126>(v); }
+__device__ __forceinline__ float d_to_f32(double v) { return f64_to_f32_clamped<-100>(v); }
 
 // Order-preserving integer key of a double (sign-magnitude -> two's
 // complement; -0 and +0 share key 0).  a < b  <=>  key(a) < key(b) for non-NaN.
@@ -87,8 +116,6 @@ __device__ __forceinline__ double clip_exact(double x, double2 lu) {
     return r;
 }
 
-// (lb, ub) of one reaction.  A volatile load, so that the compiler keeps it
-// (and the FP64 work that depends on it) inside the rarely taken branches.
 // |v| and its bit pattern through integer operations (fabs on a double can be
 // issued to the FP64 pipe).
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
@@ -99,27 +126,53 @@ __device__ __forceinline__ bool positive_int(double v) {  // v > 0 for non-NaN v
     const long long b = __double_as_longlong(v);
     return b > 0;
 }
-
-// r[k] for a run-time k without indexing the register array dynamically.
-template <int EPT>
-__device__ __forceinline__ double pick(const double (&r)[EPT], int k) {
-    double v = r[0];
-#pragma unroll
-    for (int j = 1; j < EPT; ++j) v = (j == k) ? r[j] : v;
-    return v;
+// v > t for t >= 0 and non-NaN v (an FP64 compare would go to the FP64 pipe).
+__device__ __forceinline__ bool above_int(double v, double t) {
+    return __double_as_longlong(v) > __double_as_longlong(t);
 }
 
+// r[k] for a run-time k without indexing the register array dynamically: a
+// tree of selects on the bits of k.
+template <int N>
+__device__ __forceinline__ double pick(const double (&r)[N], int k) {
+    if constexpr (N == 1) {
+        return r[0];
+    } else {
+        double h[(N + 1) / 2];
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) h[j] = (k & 1) ? r[2 * j + 1] : r[2 * j];
+        if (N & 1) h[N / 2] = r[N - 1];
+        return pick(h, k >> 1);
+    }
+}
+
+// (lb, ub) of one reaction.  A volatile load, so that the compiler keeps it
+// (and the FP64 work that depends on it) inside the rarely taken branches.
 __device__ __forceinline__ double2 ld_lbub(const double2 *p) {
     double2 v;
     asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
     return v;
 }
 
+// (lb, ub) of one reaction in FP64: from the FP32 image when the host found
+// every bound finite and exact there (the image is in L1; the FP64 bounds come
+// from L2, several hundred clocks in the middle of a step).
+__device__ __forceinline__ double2 exact_bounds(const ChainArgs &a, int i);
+
+// A pair of a warmup column: 16 bytes, past L1 (a column is read once per
+// step; L1 keeps the FP32 bounds, which every step reads twice).  Volatile, so
+// that the request stays where it is issued, a whole phase ahead of its use.
+__device__ __forceinline__ double2 ld_column(const double2 *p) {
+    double2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
 // FP32 test that x (as its truncation x32) lies strictly inside (lb, ub):
 // true only when the bracket arithmetic proves it; false means "test exactly".
-__device__ __forceinline__ bool surely_inside(float x32, float2 b, float berr) {
+__device__ __forceinline__ bool surely_inside(float x32, float lb, float ub, float berr) {
     const float ex = fmaf(fabsf(x32), kErrK, kTiny + berr);
-    return (x32 - b.x) > ex && (b.y - x32) > ex;
+    return fminf(x32 - lb, ub - x32) > ex;
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
@@ -128,30 +181,6 @@ __device__ __forceinline__ unsigned smem_addr(const void *p) {
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void fence_mbar_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-
-// 1-D bulk copy global -> shared, completion counted on `bar`.  Both addresses
-// are 16-byte aligned and bytes is a multiple of 16 (the warmup leading
-// dimension is even and the shared buffer starts on a 128-byte boundary).
-__device__ __forceinline__ void tma_load_1d(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
@@ -186,6 +215,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {  // within 2^-22; the norm's margin is 1e-5
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -225,18 +260,66 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
     return ((unsigned long long)mhi << 32) | mlo;
 }
 
+// CTA barriers; a one-warp CTA needs only its warp's.
+template <int BD>
+__device__ __forceinline__ void cta_sync() {
+    if (BD == 32) __syncwarp();
+    else __syncthreads();
+}
+template <int BD>
+__device__ __forceinline__ bool cta_any(bool p) {
+    if (BD != 32) return __syncthreads_or(p ? 1 : 0) != 0;
+    const bool any = __any_sync(0xffffffffu, p) != 0;
+    __syncwarp();
+    return any;
+}
+
 // Shared-memory exchange slots, two sets selected by attempt parity so that
-// consecutive attempts never overwrite slots another warp may still read.
-struct RedSlots {
-    float sum1[32];
-    int flag1[32];
-    float2 min2[32];
-    int flag2[32];
-    ulonglong2 min3[32];
-    int flag3[32];
-    unsigned long long max4[32];
-    double sum5[32];
+// consecutive attempts never overwrite slots another warp may still read.  The
+// per-warp values are read back four at a time.
+template <int NW>
+struct alignas(16) RedSlots {
+    static constexpr int NW4 = (NW + 3) / 4 * 4;
+    float sum1[NW4], uh[NW4], ul[NW4];
+    unsigned long long kh, kl;  // smallest exact ratios (bits) of the attempt's contenders
+    double step;                // the step length over ||d||
+    unsigned flags;             // 1: a valid contender, 2: one needs the FP64 norm
+    unsigned pad;
+    unsigned long long max4[NW];
+    double sum5[NW];
+    __device__ void clear() {
+        kh = kl = kInfBits;
+        flags = 0;
+    }
 };
+
+// Sum of the warps' values in order / their minimum.
+template <int NW>
+__device__ __forceinline__ float slots_sum(const float *v) {
+    float s = 0.0f;
+#pragma unroll
+    for (int w = 0; w < NW; w += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(v + w);
+        s += x.x;
+        if (w + 1 < NW) s += x.y;
+        if (w + 2 < NW) s += x.z;
+        if (w + 3 < NW) s += x.w;
+    }
+    return s;
+}
+template <int NW>
+__device__ __forceinline__ float slots_min(const float *v) {
+    float m = INFINITY;
+#pragma unroll
+    for (int w = 0; w < NW; w += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(v + w);
+        m = fminf(m, x.x);
+        if (w + 1 < NW) m = fminf(m, x.y);
+        if (w + 2 < NW) m = fminf(m, x.z);
+        if (w + 3 < NW) m = fminf(m, x.w);
+    }
+    return m;
+}
 
 struct StepEntry {
     double U;      // step uniform of attempt 0
@@ -245,110 +328,112 @@ struct StepEntry {
     unsigned pad;
 };
 
-// FP32 bracket of one coordinate's ratio-test contribution (reference
-// fillrandPoint, ACHRCuda.cu:266-281: a coordinate is a candidate when
-// distUb > dTol, distLb > dTol and |u_i| > uTol).  Writes the lower ends of
-// the two ratio brackets: NaN = certainly not a candidate, -inf = undecided
-// (evaluate in FP64), else the bracket's lower end; and folds the upper ends
-// of certain candidates into the running minima.
-__device__ __forceinline__ void bracket(double x, double dk, float2 b, float berr, float dtol_hi, float dtol_lo,
-                                        float uthr_hi, float uthr_lo, float &lo_h, float &lo_l, float &uh, float &ul,
-                                        int &fl) {
-    const float x32 = f64_to_f32_rz(x);
-    const float d32 = f64_to_f32_rz(dk);
-    const float ad = fabsf(d32);
-    const float Dp = b.y - x32;  // ub - x
-    const float Dm = x32 - b.x;  // x - lb
-    const float ex = fmaf(fabsf(x32), kErrK, kTiny + berr);
-    const float Ep = fmaf(fabsf(Dp), kErrK, ex);
-    const float Em = fmaf(fabsf(Dm), kErrK, ex);
-    const bool p_ok = (Dp - Ep) > dtol_hi, p_bad = (Dp + Ep) <= dtol_lo;
-    const bool m_ok = (Dm - Em) > dtol_hi, m_bad = (Dm + Em) <= dtol_lo;
-    const bool u_ok = ad > uthr_hi, u_bad = ad * kAdUp < uthr_lo;
-    const bool bad = p_bad || m_bad || u_bad;
-    const bool ok = p_ok && m_ok && u_ok;
-    const float r = rcp_approx(ad);
-    const bool pos = d32 > 0.0f;
-    const float nh = pos ? Dp : Dm, eh = pos ? Ep : Em;
-    const float nl = pos ? Dm : Dp, el = pos ? Em : Ep;
-    const float rup = r * kUp, rdn = r * kDn;
-    const float qh_up = (nh + eh) * rup, qh_dn = (nh - eh) * rdn;
-    const float ql_up = (nl + el) * rup, ql_dn = (nl - el) * rdn;
-    if (ok) {
-        uh = fminf(uh, qh_up);
-        ul = fminf(ul, ql_up);
+// ---- ratio-test brackets
+// FP32 bracket of one coordinate's two ratios (reference fillrandPoint,
+// ACHRCuda.cu:266-281: a coordinate is a candidate when distUb > dTol,
+// distLb > dTol and |u_i| > uTol).  With r = 1 / d the ratios are
+// (bh - x) r and (x - bl) r, bh the bound the step d moves towards and bl the
+// other one, so the sign of d enters as one select per bound.
+//   live: not certainly a non-candidate (its |d| may exceed the threshold)
+//   lo_h, lo_l: lower ends; of a coordinate at a bound (within the FP32
+//        error) they are not positive, so it is looked at exactly
+//   ok: certainly a candidate; only then do the upper ends count
+// e0 = (kTiny + bound error + d_tol) rounded up, so lo > 0 implies dist > d_tol.
+struct Bracket {
+    float lo_h, lo_l, up_h, up_l;
+    bool live, ok;
+};
+__device__ __forceinline__ Bracket bracket(float x, float d, float lb, float ub, float e0, float uthr_hi,
+                                           float uthr_lo) {
+    Bracket B;
+    const float ad = fabsf(d);
+    const bool pos = d > 0.0f;
+    const float bh = pos ? ub : lb, bl = pos ? lb : ub;
+    const float r = rcp_approx(d);
+    const float qh = (bh - x) * r, ql = (x - bl) * r;
+    const float g = fmaf(fabsf(x), kErrX, e0) * fabsf(r);
+    B.lo_h = fmaf(qh, kQDn, -g);
+    B.lo_l = fmaf(ql, kQDn, -g);
+    B.up_h = fmaf(qh, kQUp, g);
+    B.up_l = fmaf(ql, kQUp, g);
+    B.live = !(ad * kAdUp < uthr_lo);
+    B.ok = B.lo_h > 0.0f && B.lo_l > 0.0f && ad > uthr_hi;
+    return B;
+}
+
+// Calls f(row, (S x)_row) for the rows thread tid owns: with the sliced-ELL
+// copy of S (32-row groups, slot-major, so each warp's loads of one nonzero
+// slot are one coalesced segment) lane l of warp w has row l of groups w, w +
+// BD/32, ...; without it (caller-owned models) rows tid, tid + BD, ... of the
+// CSR are read directly.  Both visit a row's nonzeros in the same order, so
+// the sums are bitwise equal (the ELL padding adds 0 * x_0).
+//
+// The structure comes from L2 and a row is a chain of dependent FP64
+// instructions, so both latencies are shared by two groups at a time: their
+// next kSlotLoads slots are requested before any is used, and the group offsets
+// are loaded once for all of a warp's groups.
+constexpr int kSlotLoads = 4;
+
+template <int BD, class F>
+__device__ __forceinline__ void residual_each(const ChainArgs &a, const double *xs, int tid, F &&f) {
+    if (a.sell_off) {
+        constexpr int NW = BD / 32;
+        const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll 1
+        for (int g0 = warp; g0 < a.sell_groups; g0 += 32 * NW) {
+            const int mine = g0 + lane * NW;
+            const int off0 = mine < a.sell_groups ? __ldg(a.sell_off + mine) : 0;
+            const int off1 = mine < a.sell_groups ? __ldg(a.sell_off + mine + 1) : 0;
+            const int cnt = min(32, (a.sell_groups - g0 + NW - 1) / NW);
+#pragma unroll 1
+            for (int j = 0; j < cnt; j += 2) {
+                // the second group of an odd count is the first again, not used
+                const bool two = j + 1 < cnt;
+                int b0 = __shfl_sync(0xffffffffu, off0, j), b1 = __shfl_sync(0xffffffffu, off0, two ? j + 1 : j);
+                const int n0 = (__shfl_sync(0xffffffffu, off1, j) - b0) >> 5;
+                const int n1 = two ? (__shfl_sync(0xffffffffu, off1, j + 1) - b1) >> 5 : 0;
+                if (n0 == 0) b0 = b1;  // an empty group may start at the array's end: read the other's entries
+                if (n1 == 0) b1 = b0;
+                double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 1
+                for (int t = 0; t < max(n0, n1); t += kSlotLoads) {
+                    int c0[kSlotLoads], c1[kSlotLoads];
+                    double v0[kSlotLoads], v1[kSlotLoads];
+#pragma unroll
+                    for (int u = 0; u < kSlotLoads; ++u) {  // past a row: its last slot again, not used
+                        const int o0 = b0 + lane + (max(min(t + u, n0 - 1), 0) << 5);
+                        const int o1 = b1 + lane + (max(min(t + u, n1 - 1), 0) << 5);
+                        c0[u] = __ldg(a.sell_col + o0);
+                        c1[u] = __ldg(a.sell_col + o1);
+                        v0[u] = __ldg(a.sell_val + o0);
+                        v1[u] = __ldg(a.sell_val + o1);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kSlotLoads; ++u) {  // (lengths are the warp's: uniform branches)
+                        if (t + u < n0) acc0 = fma(v0[u], xs[c0[u]], acc0);
+                        if (t + u < n1) acc1 = fma(v1[u], xs[c1[u]], acc1);
+                    }
+                }
+                f(((g0 + j * NW) << 5) + lane, acc0);
+                if (two) f(((g0 + (j + 1) * NW) << 5) + lane, acc1);
+            }
+        }
+    } else {
+        for (int row = tid; row < a.m; row += BD) {
+            double acc = 0.0;
+            const int q1 = __ldg(a.row_ptr + row + 1);
+            for (int q = __ldg(a.row_ptr + row); q < q1; ++q) acc = fma(__ldg(a.val + q), xs[__ldg(a.col_idx + q)], acc);
+            f(row, acc);
+        }
     }
-    lo_h = ok ? qh_dn : (bad ? __int_as_float(0x7fc00000) : -INFINITY);
-    lo_l = ok ? ql_dn : (bad ? __int_as_float(0x7fc00000) : -INFINITY);
-    fl |= ok ? 1 : 0;
-    fl |= (!ok && !bad) ? 2 : 0;
-    fl |= (!ok && !bad && !u_ok && !u_bad) ? 4 : 0;  // needs the FP64 norm
 }
 
 // Largest |(S x)_i| over this thread's rows, as the bits of a non-negative
-// double (reference findMaxAbs, ACHRCuda.cu:232-240, on the rows thread tid
-// owns: tid, tid + BD, ...; a warp's 32 lanes own 32 consecutive rows).  With
-// the sliced-ELL copy of S each warp's loads of one nonzero slot are one
-// coalesced segment; without it (caller-owned models) the CSR rows are read
-// directly.  Both visit a row's nonzeros in the same order, so the sums are
-// bitwise equal (the ELL padding adds 0 * x_0).
+// double (reference findMaxAbs, ACHRCuda.cu:232-240).
 template <int BD>
 __device__ __forceinline__ unsigned long long residual_max_bits(const ChainArgs &a, const double *xs, int tid) {
     unsigned long long mx = 0;
-    if (a.sell_off) {
-        const int lane = tid & 31;
-        for (int g = tid >> 5; g < a.sell_groups; g += BD / 32) {
-            const int base = __ldg(a.sell_off + g);
-            const int len = (__ldg(a.sell_off + g + 1) - base) >> 5;
-            double acc = 0.0;
-#pragma unroll 4
-            for (int t = 0; t < len; ++t) {  // unrolled so the loads of 4 slots are in flight together
-                const int q = base + (t << 5) + lane;
-                acc = fma(__ldg(a.sell_val + q), xs[__ldg(a.sell_col + q)], acc);
-            }
-            mx = umax(mx, abs_bits(acc));
-        }
-    } else {
-        for (int row = tid; row < a.m; row += BD) {
-            double acc = 0.0;
-            const int q1 = __ldg(a.row_ptr + row + 1);
-            for (int q = __ldg(a.row_ptr + row); q < q1; ++q) acc = fma(__ldg(a.val + q), xs[__ldg(a.col_idx + q)], acc);
-            mx = umax(mx, abs_bits(acc));
-        }
-    }
-    return mx;
-}
-
-// The same row sums as residual_max_bits (same rows, same order of terms, so
-// the same maximum), each stored to rr[row] (device row order) for the
-// batched reprojection of segmented sampling.
-template <int BD>
-__device__ __forceinline__ unsigned long long residual_rows(const ChainArgs &a, const double *xs, double *rr, int tid) {
-    unsigned long long mx = 0;
-    if (a.sell_off) {
-        const int lane = tid & 31;
-        for (int g = tid >> 5; g < a.sell_groups; g += BD / 32) {
-            const int base = __ldg(a.sell_off + g);
-            const int len = (__ldg(a.sell_off + g + 1) - base) >> 5;
-            double acc = 0.0;
-#pragma unroll 4
-            for (int t = 0; t < len; ++t) {
-                const int q = base + (t << 5) + lane;
-                acc = fma(__ldg(a.sell_val + q), xs[__ldg(a.sell_col + q)], acc);
-            }
-            mx = umax(mx, abs_bits(acc));
-            const int row = (g << 5) + lane;
-            if (row < a.m) rr[row] = acc;
-        }
-    } else {
-        for (int row = tid; row < a.m; row += BD) {
-            double acc = 0.0;
-            const int q1 = __ldg(a.row_ptr + row + 1);
-            for (int q = __ldg(a.row_ptr + row); q < q1; ++q) acc = fma(__ldg(a.val + q), xs[__ldg(a.col_idx + q)], acc);
-            mx = umax(mx, abs_bits(acc));
-            rr[row] = acc;
-        }
-    }
+    residual_each<BD>(a, xs, tid, [&](int, double v) { mx = umax(mx, abs_bits(v)); });
     return mx;
 }
 
@@ -374,6 +459,12 @@ __device__ __forceinline__ double f32_to_f64_exact(float f) {
         (long long)(s | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(u & 0x7FFFFFu) << 29)));
 }
 
+__device__ __forceinline__ double2 exact_bounds(const ChainArgs &a, int i) {
+    if (!a.bound_exact) return ld_lbub(a.lbub + i);
+    const float2 b = __ldg(a.bnd + i);
+    return make_double2(f32_to_f64_exact(b.x), f32_to_f64_exact(b.y));
+}
+
 // BF16 bits of f rounded to nearest even (hi) and of the remainder f - hi (lo),
 // for finite f; FP32 and integer operations only.
 __device__ __forceinline__ void split_bf16_bits(float f, unsigned short &hi, unsigned short &lo) {
@@ -385,10 +476,31 @@ __device__ __forceinline__ void split_bf16_bits(float f, unsigned short &hi, uns
     lo = (unsigned short)(ru >> 16);
 }
 
+// The same row sums as residual_max_bits (same rows, same order of terms, so
+// the same maximum), each written out for the batched reprojection of
+// segmented sampling (chain p, device row order): FP64, and the BF16 split of
+// its truncation to FP32 (no FP64 operation).
+__device__ __forceinline__ void store_residual_row(const ChainArgs &a, int p, int row, double v) {
+    unsigned short h, l;
+    split_bf16_bits(f64_to_f32_rz(v), h, l);
+    a.seg_Rh[(size_t)p * (size_t)a.kpad + (size_t)row] = h;
+    a.seg_Rl[(size_t)p * (size_t)a.kpad + (size_t)row] = l;
+    a.seg_rd[(size_t)p * (size_t)a.ld_r + (size_t)row] = v;
+}
+template <int BD>
+__device__ __forceinline__ unsigned long long residual_rows(const ChainArgs &a, const double *xs, int p, int tid) {
+    unsigned long long mx = 0;
+    residual_each<BD>(a, xs, tid, [&](int row, double v) {
+        mx = umax(mx, abs_bits(v));
+        if (row < a.m) store_residual_row(a, p, row, v);
+    });
+    return mx;
+}
+
 // x <- x - S^T z, z = (S S^T)^+ S x: the reference's N (N^T x) written through
 // the residual (equal in exact arithmetic).  S x is summed in FP64 over the
-// same rows as the check and kept as FP32 hi + lo pairs in rr (m entries of
-// the staging buffer); z = (S S^T)^+ r runs in FP32 (a warp per row of the
+// same rows as the check and kept as FP32 hi + lo pairs in rr (m entries
+// in the accumulator's place); z = (S S^T)^+ r runs in FP32 (a warp per row of the
 // pseudo-inverse, coalesced), whose relative error (~1e-7 times the condition
 // number) applies to the correction, not to x, which is at most of the size of
 // the residual's preimage; the update x_j -= sum_i S_ij z_i is FP64 (CSC).
@@ -398,31 +510,12 @@ __device__ __forceinline__ void residual_form_reproject(const ChainArgs &a, doub
     constexpr int NW = BD / 32;
     const int lane = tid & 31, warp = tid >> 5;
     const int m = a.m;
-    if (a.sell_off) {
-        for (int g = warp; g < a.sell_groups; g += NW) {
-            const int base = __ldg(a.sell_off + g);
-            const int len = (__ldg(a.sell_off + g + 1) - base) >> 5;
-            double acc = 0.0;
-#pragma unroll 4
-            for (int t = 0; t < len; ++t) {
-                const int q = base + (t << 5) + lane;
-                acc = fma(__ldg(a.sell_val + q), xs[__ldg(a.sell_col + q)], acc);
-            }
-            const int row = (g << 5) + lane;
-            if (row < m) {
-                const float hi = __double2float_rn(acc);
-                rr[row] = make_float2(hi, __double2float_rn(acc - (double)hi));
-            }
+    residual_each<BD>(a, xs, tid, [&](int row, double v) {
+        if (row < m) {
+            const float hi = __double2float_rn(v);
+            rr[row] = make_float2(hi, __double2float_rn(v - (double)hi));
         }
-    } else {
-        for (int row = tid; row < m; row += BD) {
-            double acc = 0.0;
-            const int q1 = __ldg(a.row_ptr + row + 1);
-            for (int q = __ldg(a.row_ptr + row); q < q1; ++q) acc = fma(__ldg(a.val + q), xs[__ldg(a.col_idx + q)], acc);
-            const float hi = __double2float_rn(acc);
-            rr[row] = make_float2(hi, __double2float_rn(acc - (double)hi));
-        }
-    }
+    });
     __syncthreads();
     for (int i = warp; i < m; i += NW) {
         const float *Bi = a.pinv32 + (size_t)i * (size_t)m;
@@ -445,35 +538,115 @@ __device__ __forceinline__ void residual_form_reproject(const ChainArgs &a, doub
     }
 }
 
-// Bytes of one staged warmup column (the leading dimension is even, so a
-// multiple of 16).
-__device__ __forceinline__ unsigned column_bytes(const ChainArgs &a) {
-    return (unsigned)(sizeof(double) * (size_t)a.ldw);
+// What a thread keeps of its brackets: the smallest lower and upper ends.
+struct Minima {
+    float uh = INFINITY, ul = INFINITY, lh = INFINITY, ll = INFINITY;
+    __device__ __forceinline__ void add(const Bracket &B) {
+        if (B.live) {
+            lh = fminf(lh, B.lo_h);
+            ll = fminf(ll, B.lo_l);
+        }
+        if (B.ok) {
+            uh = fminf(uh, B.up_h);
+            ul = fminf(ul, B.up_l);
+        }
+    }
+};
+
+// The ratio-test quantities phase B2 needs of an attempt.
+struct RatioTest {
+    float uh, ul, uthr_hi, uthr_lo, e0;
+    bool have_norm64;
+    double thr64;
+    unsigned long long kh, kl;  // smallest exact ratios found (bits)
+    int found;                  // 1: a valid contender, 2: one whose candidacy needs the FP64 norm
+};
+
+// FP64 evaluation of reaction i as a contender for the max step (side_h) or
+// the min step: the candidacy test where the bracket left it open, then the
+// quotient.
+__device__ __forceinline__ void evaluate(const ChainArgs &a, RatioTest &t, double xi, double dk, int i, float2 b32,
+                                         bool side_h) {
+    const bool up = side_h == positive_int(dk);  // this ratio's distance: ub - x, else x - lb
+    double2 lu;
+    if (a.bound_exact) {
+        lu.x = lu.y = f32_to_f64_exact(up ? b32.y : b32.x);
+    } else {
+        lu = ld_lbub(a.lbub + i);
+    }
+    const double num = (up ? lu.y : xi) - (up ? xi : lu.x);
+    // a certain candidate, by the bracket's own bounds (with the norm known)
+    const float x32 = x_to_f32(xi), ad = fabsf(d_to_f32(dk));
+    bool valid = !a.exact_ratio && ad > fmaxf(t.uthr_hi, kDCert) &&
+                 fminf(b32.y - x32, x32 - b32.x) * kQDn > fmaf(fabsf(x32), kErrX, t.e0);
+    if (!valid) {  // undecided: full FP64 candidacy test
+        if (a.bound_exact) lu = make_double2(f32_to_f64_exact(b32.x), f32_to_f64_exact(b32.y));
+        const double oth = (up ? xi : lu.y) - (up ? lu.x : xi);
+        bool u_pass;
+        if (t.have_norm64) {
+            u_pass = abs_bits(dk) > (unsigned long long)__double_as_longlong(t.thr64);
+        } else {
+            const float ad32 = fabsf(f64_to_f32_rz(dk));
+            // inside the FP32 norm's margin: settled with the FP64 norm
+            if (!(ad32 > t.uthr_hi) && !(ad32 * kAdUp < t.uthr_lo)) t.found |= 2;
+            u_pass = ad32 > t.uthr_hi;
+        }
+        valid = above_int(num, a.d_tol) && above_int(oth, a.d_tol) && u_pass;
+    }
+    if (valid) {
+        const unsigned long long q = (unsigned long long)__double_as_longlong(div_rn(num, abs_int(dk)));
+        if (side_h) t.kh = umin(t.kh, q);
+        else t.kl = umin(t.kl, q);
+        t.found |= 1;
+    }
 }
 
 }  // namespace
 
 constexpr int kTbl = 64;  // steps per refill of the step table
 
-// Shared memory of one CTA: xs, As, ws (NP doubles each; ws doubles as the
-// reprojection scratch), the step table and the reduction slots.
-__host__ __device__ inline size_t chain_smem_bytes_cfg(int np, int d, int bd) {
-    (void)d;
-    (void)bd;
-    return sizeof(double) * 3 * (size_t)np + sizeof(StepEntry) * kTbl + 2 * sizeof(RedSlots) + 128;
+// Shared memory of one CTA: xs, As (NP doubles each; a reprojection parks the
+// accumulator in registers and uses As as its scratch), the step table, two
+// reduction slots, then eight statistics counters, the exact-evaluation count
+// (two ints), the `never` barrier and the two worst-case words.
+template <int BD>
+__host__ __device__ constexpr size_t chain_tail_bytes() {
+    return sizeof(StepEntry) * kTbl + 2 * sizeof(RedSlots<BD / 32>) + 128;
+}
+template <int BD, int EPT>
+__host__ __device__ constexpr size_t chain_smem_bytes_cfg() {
+    return sizeof(double) * 2 * (size_t)(BD * EPT) + chain_tail_bytes<BD>();
 }
 
-// Shared-memory header of a CTA: x, A and the staging buffer (3 NP doubles),
-// the step table, two reduction slots, then the column barrier, eight
-// statistics counters, the exact-evaluation count (two ints), the `never`
-// barrier and the two worst-case words.
-template <int NP>
-__device__ __forceinline__ void chain_barriers(unsigned char *smem_raw, uint64_t *&bar, uint64_t *&never) {
-    RedSlots *rsb = reinterpret_cast<RedSlots *>(reinterpret_cast<StepEntry *>(reinterpret_cast<double *>(smem_raw) +
-                                                                               3 * (size_t)NP) +
-                                                 kTbl);
-    bar = reinterpret_cast<uint64_t *>(rsb + 2);
-    never = reinterpret_cast<uint64_t *>(reinterpret_cast<int *>(bar + 1 + 8) + 2);
+// Resident CTAs per SM a configuration is compiled for, with `regs` registers
+// per thread: what shared memory and the registers allow.  An SM's registers
+// lie in four files of 16384, one per scheduler, and the warps spread over
+// them, so the fullest file counts (18 warps allow 96 registers each, 12 allow
+// 168).
+template <int BD, int EPT>
+constexpr int chain_ctas_with(int regs) {
+    const int by_smem = (int)(227 * 1024 / (chain_smem_bytes_cfg<BD, EPT>() + 1024));
+    const int r = regs < 72 ? 72 : regs > 255 ? 255 : (regs + 7) / 8 * 8;
+    const int by_regs = 4 * (16384 / (32 * r)) / (BD / 32);
+    const int c = by_smem < by_regs ? by_smem : by_regs;
+    return c < 1 ? 1 : c > 32 ? 32 : c;
+}
+// A thread keeps its direction (2 EPT registers) and, unless that costs a
+// resident chain where there are few, the FP32 image of its point (EPT).
+template <int BD, int EPT>
+constexpr bool chain_keeps_x32() {
+    const int kept = chain_ctas_with<BD, EPT>(3 * EPT + 58);
+    return kept >= 4 || kept >= chain_ctas_with<BD, EPT>(2 * EPT + 48);
+}
+template <int BD, int EPT>
+constexpr int chain_min_ctas() {
+    return chain_ctas_with<BD, EPT>(chain_keeps_x32<BD, EPT>() ? 3 * EPT + 58 : 2 * EPT + 48);
+}
+
+template <int BD, int EPT>
+__device__ __forceinline__ uint64_t *chain_never(unsigned char *smem_raw) {
+    return reinterpret_cast<uint64_t *>(smem_raw + sizeof(double) * 2 * (size_t)(BD * EPT) + sizeof(StepEntry) * kTbl +
+                                        2 * sizeof(RedSlots<BD / 32>) + 72);
 }
 
 // Entries e = tid, tid + BD, ... < kTbl of the step table for steps s + e below
@@ -497,54 +670,68 @@ __device__ __forceinline__ void fill_step_table(const ChainArgs &a, StepEntry *t
 
 // One CTA's share of a launch: chains p_begin, p_begin + p_step, ... below
 // p_end of the model `a` describes, then the CTA's statistics into
-// a.counters.  The staging barriers live in the shared-memory header; the
-// caller initialises them once per CTA and `phase` carries their parity from
-// one call to the next.  Returns true when a bounded wait ran out.
+// a.counters.  Returns true when the launch failed (a bounded wait ran out, or
+// a warmup index outside the matrix).
 // SEG: segmented launches of the deferred reprojection (a separate
 // instantiation, so the plain kernel carries none of its code or registers).
+//
+// What bounds it: the FP64 pipe (three instructions per reaction and step, one
+// warp instruction per 19 clocks and SM), as long as other chains' FP64 work
+// fills the latency of a chain's two reductions and its contenders.  So the
+// split serves residency: as many chains per SM as two vectors of shared memory
+// and the registers allow.  2766 x 3742, two chains per SM: 10.2 K clocks of an
+// SM per chain-step (14.0 K with the column staged in shared memory, the
+// brackets formed twice and the ratios divided on the FP64 pipe), 7.8 K of them
+// the pipe's; a lone chain's step went from 16.4 K to 14.7 K.
 template <int BD, int EPT, bool SEG>
 __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p_step, int p_end,
-                                          unsigned char *smem_raw, unsigned &phase) {
-    constexpr int NP = BD * EPT;
+                                          unsigned char *smem_raw) {
+    static_assert(EPT % 2 == 0, "threads own pairs of reactions");
+    constexpr int NP = BD * EPT, KP = EPT / 2;
     constexpr int NW = BD / 32;
+    constexpr bool KX = chain_keeps_x32<BD, EPT>();
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     double *xs = reinterpret_cast<double *>(smem_raw);
     double *As = xs + NP;
-    double *ws = As + NP;
-    double *ys = ws;  // reprojection scratch (d <= n entries, below the zero padding of ws)
-    StepEntry *tbl = reinterpret_cast<StepEntry *>(ws + NP);
-    RedSlots *rsb = reinterpret_cast<RedSlots *>(tbl + kTbl);
-    uint64_t *bar, *never;  // the staged column's barrier; a barrier nothing arrives on
-    chain_barriers<NP>(smem_raw, bar, never);
-    unsigned long long *cnt = reinterpret_cast<unsigned long long *>(bar + 1);  // CTA statistics, CNT_* slots
+    double2 *xs2 = reinterpret_cast<double2 *>(xs), *As2 = reinterpret_cast<double2 *>(As);
+    double *ys = As;  // reprojection scratch (the accumulator waits in registers)
+    StepEntry *tbl = reinterpret_cast<StepEntry *>(As + NP);
+    RedSlots<NW> *rsb = reinterpret_cast<RedSlots<NW> *>(tbl + kTbl);
+    unsigned long long *cnt = reinterpret_cast<unsigned long long *>(rsb + 2);  // CTA statistics, CNT_* slots
     int *exact_count = reinterpret_cast<int *>(cnt + 8);
+    uint64_t *never = chain_never<BD, EPT>(smem_raw);  // a barrier nothing arrives on
     // largest residual and bound violation of the CTA's emitted points (bits of non-negative doubles)
     unsigned long long *worst = reinterpret_cast<unsigned long long *>(never + 1);
     // (S S^T)^+ r of the residual-form reprojection (m floats), when enabled
-    float *zs = reinterpret_cast<float *>(smem_raw + chain_smem_bytes_cfg(NP, a.d, BD));
+    float *zs = reinterpret_cast<float *>(smem_raw + chain_smem_bytes_cfg<BD, EPT>());
 
     if (tid == 0) {
         *exact_count = 0;
         for (int c = 0; c < 8; ++c) cnt[c] = 0;
         worst[0] = worst[1] = 0;
+        rsb[0].clear();
+        rsb[1].clear();
     }
-    // The TMA copy fills ws[0, ldw); the padding beyond stays zero.
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) ws[tid + k * BD] = 0.0;
-    __syncthreads();
+    cta_sync<BD>();
 
     const bool hr = a.hit_and_run != 0;  // directions are the staged columns themselves (no centre)
-    const bool merged = a.merged_ab != 0 && !a.exact_ratio;  // ratio-test brackets formed in phase A
-    const float uthr_max = a.uthr_max;
-    // A warp whose 32 elements of the last slot (k = EPT - 1) all lie in the
-    // padding (i >= n) skips that slot: its coordinates stay 0 and its d is 0,
-    // so the FP64 operations on it would change nothing.
-    const bool tail_live = warp * 32 + (EPT - 1) * BD < a.n;
-// (Not for 32 elements per thread, where the branches cost more registers than they save.)
-#define ACHR_PAD_SLOT(k) (EPT < 32 && (k) == EPT - 1 && !tail_live)
+    const bool merged = a.merged_ab != 0 && !a.exact_ratio;  // ratio-test brackets formed before ||d|| is known
+    const int npair = (a.n + 1) >> 1;
+    const int odd = (a.n & 1) ? npair - 1 : -1;  // the pair whose second reaction is padding
+    // A warp whose pairs of the last slot (k = KP - 1) all lie in the padding
+    // skips that slot: its coordinates stay 0 and its d is 0, so the FP64
+    // operations on it would change nothing.
+    const bool tail_live = warp * 32 + (KP - 1) * BD < npair;
+#define ACHR_PAD_SLOT(k) ((k) == KP - 1 && !tail_live)
+    const float e0 = (kTiny + a.bound_err + a.dtol_hi) * 1.01f;
+    const float4 *bnd2 = reinterpret_cast<const float4 *>(a.bnd);  // (lb, ub, lb, ub) of a pair
     unsigned it = 0;
     bool failed = false;
+    // The failure-detection test: a wait on a barrier nothing completes always runs out.
+    if (a.wait_never && a.T > 0 && p_begin < p_end)
+        failed = !mbar_wait_bounded(never, 0, a.wait_ns ? a.wait_ns : kWaitNs);
+    failed = cta_any<BD>(failed);
 
     // (Scalars that stay constant over a launch are read from the kernel
     // parameters where they are used rather than held in registers.)
@@ -576,8 +763,8 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 As[i] = a.A0[i];
             }
         }
-        int buf_col = -1;
-        bool inflight = false, any_accepted = a.x_in != nullptr || (sflags & SEG_ACCEPTED), stuck = false;
+        int buf_col = -1;  // the warmup column dreg holds (-1: none)
+        bool any_accepted = a.x_in != nullptr || (sflags & SEG_ACCEPTED), stuck = false;
         bool seg_pending = false;  // this launch ended the chain after a check step's update
         const bool was_stuck = (sflags & SEG_STUCK) != 0;
         if (was_stuck) stuck = true;  // stopped in an earlier launch: no more steps
@@ -594,6 +781,9 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 }
             }
         }
+        cta_sync<BD>();  // the loops above are per element, the step's per pair
+        double dreg[EPT];  // the next step's column, then the step's direction
+        float xf[KX ? EPT : 2];  // FP32 image of the point (KX; else formed where it is used)
         if (sflags & SEG_PENDING) {
             // Finish the check step the previous launch ended on (the batched
             // pass has reprojected the point if its residual was above the
@@ -601,34 +791,55 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
             unsigned edge = 0;
 #pragma unroll
             for (int k = 0; k < EPT; ++k) {
-                const int i = tid + k * BD;
-                if (ACHR_PAD_SLOT(k)) continue;
+                const int i = 2 * (tid + (k >> 1) * BD) + (k & 1);
+                if (ACHR_PAD_SLOT(k >> 1)) continue;
                 const double xv = xs[i];
-                if (surely_inside(f64_to_f32_rz(xv), __ldg(a.bnd + i), a.bound_err)) {
+                const float2 b = __ldg(a.bnd + i);
+                if (surely_inside(x_to_f32(xv), b.x, b.y, a.bound_err)) {
                     if (!hr) As[i] += xv;
                 } else {
                     edge |= 1u << k;
                 }
             }
             for (; edge; edge &= edge - 1) {
-                const int i = tid + (__ffs(edge) - 1) * BD;
-                const double xc = clip_exact(xs[i], ld_lbub(a.lbub + i));
+                const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
+                const double xc = clip_exact(xs[i], exact_bounds(a, i));
                 xs[i] = xc;
                 if (!hr) As[i] += xc;
+            }
+        }
+// Pair k of the point's image.
+#define ACHR_X32(k, f0, f1)                        \
+    float f0, f1;                                  \
+    if (KX) {                                      \
+        f0 = xf[KX ? 2 * (k) : 0];                 \
+        f1 = xf[KX ? 2 * (k) + 1 : 1];             \
+    } else {                                       \
+        const double2 xk_ = xs2[tid + (k) * BD];   \
+        f0 = x_to_f32(xk_.x);                      \
+        f1 = x_to_f32(xk_.y);                      \
+    }
+        if (KX) {
+#pragma unroll
+            for (int k = 0; k < KP; ++k) {
+                const double2 x2 = xs2[tid + k * BD];
+                xf[KX ? 2 * k : 0] = x_to_f32(x2.x);
+                xf[KX ? 2 * k + 1 : 1] = x_to_f32(x2.y);
             }
         }
         // The reference checks when the step count is a multiple of the period
         // (ACHRCuda.cu:325); a period of INT_MAX stands for "never".
         int chk = a.check_period == 0x7fffffff ? 1 : a.step0 % a.check_period;
         int tbase = a.step0 - kTbl;
+        float t_lo = 0.0f;  // lower end of the merged brackets' candidacy threshold
 
         for (int s = a.step0; s < (a.step0 + a.T) && !stuck && !failed && !seg_pending; ++s) {
             if (s - tbase >= kTbl) {
                 // refill the step table: entry e holds step tbase + e
                 tbase = s;
-                __syncthreads();
+                cta_sync<BD>();
                 fill_step_table<BD>(a, tbl, ACHR_CHAIN_ID, s, a.step0 + a.T, tid);
-                __syncthreads();
+                cta_sync<BD>();
             }
             // this step's table entry (its fields are read where they are used)
             const StepEntry *te = tbl + (s - tbase);
@@ -637,152 +848,79 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                     stuck = true;
                     break;
                 }
-                RedSlots *rs = rsb + (it & 1u);
+                RedSlots<NW> *rs = rsb + (it & 1u);
                 const int r = att == 0
                                   ? (int)te->idx
                                   : (int)warmup_index(step_draw(a.seed, ACHR_CHAIN_ID, (uint32_t)s, (uint32_t)att),
                                                                   (uint32_t)a.W);
-                if (buf_col != r) {
-                    if (inflight) {
-                        if (!mbar_wait_bounded(bar, phase)) failed = true;
-                        phase ^= 1u;
-                        inflight = false;
-                    }
-                    __syncthreads();  // every thread has seen the previous phase complete
-                    if (r < 0 || r >= a.W) {  // never copy from outside the warmup matrix
-                        failed = true;
-                        break;
-                    }
-                    if (tid == 0) {
-                        fence_proxy_async_smem();
-                        mbar_arrive_expect_tx(bar, column_bytes(a));
-                        tma_load_1d(ws, a.warmup + (size_t)r * (size_t)a.ldw, column_bytes(a), bar);
-                    }
-                    inflight = true;
-                    buf_col = r;
-                }
-                if (inflight) {
-                    // a.wait_never (failure-detection test): the wait is on a barrier
-                    // that nothing completes, so it always runs out.
-                    if (!mbar_wait_bounded(a.wait_never ? never : bar, phase, a.wait_ns ? a.wait_ns : kWaitNs)) {
-                        // The column did not arrive within the caller's limit: record it,
-                        // then let the copy land (default limit) before the buffer is left.
-                        failed = true;
-                        mbar_wait_bounded(bar, phase);
-                    }
-                    phase ^= 1u;
-                    inflight = false;
-                }
-
-                // Phase A: d = w_r - A / (W + t)  (reference ACHRCuda.cu:260-264);
-                // in hit-and-run mode the staged column is the direction itself.
-                double dreg[EPT];
-                float ss = 0.0f, admax = 0.0f;
-                if (hr) {
-#pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) {
-                            dreg[k] = 0.0;
-                            continue;
-                        }
-                        const double dk = ws[i];
-                        dreg[k] = dk;
-                        const float d32 = f64_to_f32_rz(dk);
-                        ss = fmaf(d32, d32, ss);
-                        admax = fmaxf(admax, fabsf(d32));
-                    }
-                } else {
-                    const double ninv = -te->inv;
-#pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) {
-                            dreg[k] = 0.0;
-                            continue;
-                        }
-                        const double dk = fma(As[i], ninv, ws[i]);
-                        dreg[k] = dk;
-                        const float d32 = f64_to_f32_rz(dk);
-                        ss = fmaf(d32, d32, ss);
-                        admax = fmaxf(admax, fabsf(d32));
-                    }
-                }
-                // Phase B1 folded into phase A (merged): the brackets need ||d||
-                // only for the candidacy test |d_i| > u_tol ||d||, so they are
-                // formed now with a threshold interval that holds for any norm
-                // the block sum can give: above by uthr_max (checked after the
-                // reduction), below by u_tol times this thread's largest |d_i|.
-                // A coordinate certain under both is classified; any other
-                // gets a -inf lower end and is settled exactly in phase B2.
-                float uh = INFINITY, ul = INFINITY;
-                float my_lh = INFINITY, my_ll = INFINITY;  // this thread's smallest bracket lower ends
-                int fl = 0;
-                if (merged) {
-                    const float uthr_lo_p = a.utol32 * admax * kProvDn;
-#pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) continue;  // padding: never a candidate
-                        float lo_h, lo_l;
-                        bracket(xs[i], dreg[k], __ldg(a.bnd + i), a.bound_err, a.dtol_hi, a.dtol_lo, uthr_max,
-                                uthr_lo_p, lo_h, lo_l, uh, ul, fl);
-                        my_lh = fminf(my_lh, lo_h);
-                        my_ll = fminf(my_ll, lo_l);
-                    }
-                    uh = warp_min_f32(uh);
-                    ul = warp_min_f32(ul);
-                }
-#pragma unroll
-                for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                // Each thread timed its own wait: OR every lane's outcome so that
-                // the whole block leaves (or stays) together.
-                const bool warp_failed = __any_sync(0xffffffffu, failed);
-                if (lane == 0) {
-                    rs->sum1[warp] = ss;
-                    rs->flag1[warp] = warp_failed ? 1 : 0;
-                    if (merged) rs->min2[warp] = make_float2(uh, ul);
-                }
-                __syncthreads();
-                ss = 0.0f;
-                int f1 = 0;
-#pragma unroll
-                for (int w = 0; w < NW; ++w) {
-                    ss += rs->sum1[w];
-                    f1 |= rs->flag1[w];
-                }
-                if (merged) {
-                    uh = INFINITY;
-                    ul = INFINITY;
-#pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float2 v = rs->min2[w];
-                        uh = fminf(uh, v.x);
-                        ul = fminf(ul, v.y);
-                    }
-                }
-                if (f1) {
+                if (r < 0 || r >= a.W) {  // never read outside the warmup matrix (uniform over the CTA)
                     failed = true;
                     break;
                 }
-                const float norm32 = sqrtf(ss);
-
-                // Prefetch the next step's warmup column while this one is tested.
-                if (s + 1 < (a.step0 + a.T)) {
-                    const int rn =
-                        (s + 1 - tbase < kTbl)
-                            ? (int)tbl[s + 1 - tbase].idx
-                            : (int)warmup_index(step_draw(a.seed, ACHR_CHAIN_ID, (uint32_t)(s + 1), 0u), (uint32_t)a.W);
-                    if (rn != buf_col && rn >= 0 && rn < a.W) {
-                        if (tid == 0) {
-                            fence_proxy_async_smem();
-                            mbar_arrive_expect_tx(bar, column_bytes(a));
-                            tma_load_1d(ws, a.warmup + (size_t)rn * (size_t)a.ldw, column_bytes(a), bar);
-                        }
-                        inflight = true;
-                        buf_col = rn;
+                if (buf_col != r) {
+                    const double2 *col = reinterpret_cast<const double2 *>(a.warmup + (size_t)r * (size_t)a.ldw);
+#pragma unroll
+                    for (int k = 0; k < KP; ++k) {
+                        const int q = tid + k * BD;
+                        double2 v = make_double2(0.0, 0.0);
+                        if (q < npair) v = ld_column(col + q);
+                        dreg[2 * k] = v.x;
+                        dreg[2 * k + 1] = v.y;
                     }
                 }
+                buf_col = -1;  // from here on dreg is the direction
+
+                // Phase A: d = w_r - A / (W + t)  (reference ACHRCuda.cu:260-264);
+                // in hit-and-run mode the column is the direction itself.
+                // Phase B1 (merged): the brackets need ||d|| only for the
+                // candidacy test |d_i| > u_tol ||d||, so they are formed in the
+                // same pass, where they fill the FP64 pipe's latency, with a
+                // threshold interval checked once the block has the norm: above
+                // by uthr_max, below by a hundredth of the last attempt's (0
+                // before the first).  A coordinate certain under both is
+                // classified; any other keeps its lower ends and is settled
+                // exactly in phase B2.
+                float ss = 0.0f;
+                Minima mn;
+                {
+                    const double ninv = -te->inv;
+                    const float t_hi = fmaxf(a.uthr_max, kDCert);
+#pragma unroll
+                    for (int k = 0; k < KP; ++k) {
+                        const int q = tid + k * BD;
+                        if (ACHR_PAD_SLOT(k)) continue;  // padding: d stays 0, never a candidate
+                        if (q == odd) dreg[2 * k + 1] = 0.0;
+                        if (!hr) {
+                            const double2 A2 = As2[q];
+                            dreg[2 * k] = fma(A2.x, ninv, dreg[2 * k]);
+                            dreg[2 * k + 1] = fma(A2.y, ninv, dreg[2 * k + 1]);
+                        }
+                        const float4 b = __ldg(bnd2 + q);
+                        ACHR_X32(k, x0, x1)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const float d32 = d_to_f32(dreg[2 * k + c]);
+                            ss = fmaf(d32, d32, ss);
+                            if (merged) mn.add(bracket(c ? x1 : x0, d32, c ? b.z : b.x, c ? b.w : b.y, e0, t_hi, t_lo));
+                        }
+                    }
+                }
+                float uh = warp_min_f32(mn.uh), ul = warp_min_f32(mn.ul);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                if (NW > 1) {
+                    if (lane == 0) {
+                        rs->sum1[warp] = ss;
+                        rs->uh[warp] = uh;
+                        rs->ul[warp] = ul;
+                    }
+                    cta_sync<BD>();
+                    if (tid == 0) rsb[(it + 1) & 1u].clear();  // read last before this barrier
+                    ss = slots_sum<NW>(rs->sum1);
+                    uh = slots_min<NW>(rs->uh);
+                    ul = slots_min<NW>(rs->ul);
+                }
+                const float norm32 = sqrt_approx(ss);
                 if (!(norm32 > 0.0f) || !(norm32 < INFINITY)) {
                     if (tid == 0) ++cnt[CNT_REJECTED];
                     continue;
@@ -791,161 +929,166 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 // Phase B1: FP32 brackets (reference ratio test ACHRCuda.cu:266-281)
                 const float uthr = a.utol32 * norm32;
                 const float uthr_hi = uthr * kNormUp, uthr_lo = uthr * kNormDn;
-                if (merged && uthr_hi <= uthr_max) {
-                    fl = 0;  // the merged brackets stand; their flags are not used
-                } else {
-                    // separate pass (merged: ||d|| exceeded the bound the merged brackets assumed)
-                    if (merged) __syncthreads();  // min2 of this attempt may still be read
-                    uh = INFINITY;
-                    ul = INFINITY;
-                    my_lh = INFINITY;
-                    my_ll = INFINITY;
-                    fl = 0;
+                const bool stands = merged && uthr_hi <= a.uthr_max && t_lo <= uthr_lo;
+                t_lo = 0.01f * uthr_lo;
+                if (!stands) {
+                    // separate pass (merged: ||d|| left the interval the merged brackets assumed)
+                    if (merged) cta_sync<BD>();  // uh and ul of this attempt may still be read
+                    mn = Minima();
                     if (!a.exact_ratio) {
+                        const float t_hi = fmaxf(uthr_hi, kDCert);
 #pragma unroll
-                        for (int k = 0; k < EPT; ++k) {
-                            const int i = tid + k * BD;
+                        for (int k = 0; k < KP; ++k) {
                             if (ACHR_PAD_SLOT(k)) continue;
-                            float lo_h, lo_l;
-                            bracket(xs[i], dreg[k], __ldg(a.bnd + i), a.bound_err, a.dtol_hi, a.dtol_lo, uthr_hi,
-                                    uthr_lo, lo_h, lo_l, uh, ul, fl);
-                            my_lh = fminf(my_lh, lo_h);  // NaN (not a candidate) is ignored, -inf (undecided) wins
-                            my_ll = fminf(my_ll, lo_l);
-                        }
-                    } else {
-                        fl = 2 | 4;
-                        my_lh = my_ll = -INFINITY;
-                    }
-                    uh = warp_min_f32(uh);
-                    ul = warp_min_f32(ul);
-                    fl = (int)__reduce_or_sync(0xffffffffu, (unsigned)fl);
-                    if (lane == 0) {
-                        rs->min2[warp] = make_float2(uh, ul);
-                        rs->flag2[warp] = fl;
-                    }
-                    __syncthreads();
-                    uh = INFINITY;
-                    ul = INFINITY;
-                    fl = 0;
+                            const float4 b = __ldg(bnd2 + tid + k * BD);
+                            ACHR_X32(k, x0, x1)
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float2 v = rs->min2[w];
-                        uh = fminf(uh, v.x);
-                        ul = fminf(ul, v.y);
-                        fl |= rs->flag2[w];
+                            for (int c = 0; c < 2; ++c) {
+                                mn.add(bracket(c ? x1 : x0, d_to_f32(dreg[2 * k + c]), c ? b.z : b.x,
+                                               c ? b.w : b.y, e0, t_hi, uthr_lo));
+                            }
+                        }
+                    }
+                    uh = warp_min_f32(mn.uh);
+                    ul = warp_min_f32(mn.ul);
+                    if (NW > 1) {
+                        if (lane == 0) {
+                            rs->uh[warp] = uh;
+                            rs->ul[warp] = ul;
+                        }
+                        cta_sync<BD>();
+                        uh = slots_min<NW>(rs->uh);
+                        ul = slots_min<NW>(rs->ul);
                     }
                 }
 
                 // FP64 norm, only when some candidacy test sits inside the FP32
-                // norm's margin (or every candidate is evaluated in FP64).  With
-                // merged brackets that is known only in phase B2, which then
-                // asks for it and runs once more.
-                double thr64 = 0.0;
-                bool have_norm64 = false;
-                double norm64 = 0.0;
-                unsigned long long kh, kl;
+                // norm's margin (found in phase B2, which then runs once more)
+                // or every candidate is evaluated in FP64.
+                RatioTest t;
+                t.uh = uh;
+                t.ul = ul;
+                t.uthr_hi = uthr_hi;
+                t.uthr_lo = uthr_lo;
+                t.e0 = e0;
+                t.have_norm64 = false;
+                t.thr64 = 0.0;
+                bool want_norm64 = a.exact_ratio != 0;
                 int anyv;
-                for (int b2 = 0;; ++b2) {
-                    if ((fl & 4) && !have_norm64) {
+                for (;;) {
+                    if (want_norm64) {
                         double s64 = fp64_zero_here();
 #pragma unroll
                         for (int k = 0; k < EPT; ++k) s64 = fma(dreg[k], dreg[k], s64);
 #pragma unroll
                         for (int o = 16; o; o >>= 1) s64 += __shfl_xor_sync(0xffffffffu, s64, o);
                         if (lane == 0) rs->sum5[warp] = s64;
-                        __syncthreads();
+                        cta_sync<BD>();
                         s64 = 0.0;
 #pragma unroll
                         for (int w = 0; w < NW; ++w) s64 += rs->sum5[w];
-                        norm64 = sqrt(s64);
-                        have_norm64 = true;
-                        thr64 = a.u_tol * norm64;
+                        t.have_norm64 = true;
+                        t.thr64 = a.u_tol * sqrt(s64);
                     }
 
                     // Phase B2: FP64 evaluation of every coordinate whose bracket can
-                    // hold a minimum, or whose candidacy the brackets left open.
-                    kh = kInfBits;
-                    kl = kInfBits;
-                    anyv = 0;
-                    int nex = 0, need64 = 0;
-                    unsigned mh = 0, ml = 0, mam = 0;  // bit k: contender for max / min step, undecided
-                    // Only a thread whose own bracket lower ends reach the block minima
-                    // can hold a contender; the others skip the second pass.
-                    const bool mine = my_lh <= uh || my_ll <= ul;
-                    if (!a.exact_ratio && mine) {
+                    // hold a minimum.  Only a thread whose own smallest lower ends
+                    // reach the block minima can hold one.
+                    t.kh = t.kl = kInfBits;
+                    t.found = 0;
+                    const bool mine = mn.lh <= uh || mn.ll <= ul;
+                    if (EPT <= 8 || a.exact_ratio) {
+                        // Each thread its own: a few elements (or, exact_ratio, all of
+                        // them), both sides of different lanes at once.
+                        unsigned mh = 0, ml = 0;  // bit k: contender for max / min step
+                        if (a.exact_ratio) {
+                            mh = ml = (EPT >= 32) ? 0xFFFFFFFFu : ((1u << EPT) - 1u);
+                        } else if (EPT <= 8 && mine) {
 #pragma unroll
-                        for (int k = 0; k < EPT; ++k) {
-                            const int i = tid + k * BD;
-                            if (ACHR_PAD_SLOT(k)) continue;
-                            float lo_h, lo_l, uh2 = INFINITY, ul2 = INFINITY;  // minima already known
-                            int fl2 = 0;
-                            bracket(xs[i], dreg[k], __ldg(a.bnd + i), a.bound_err, a.dtol_hi, a.dtol_lo, uthr_hi,
-                                    uthr_lo, lo_h, lo_l, uh2, ul2, fl2);
-                            mh |= (lo_h <= uh ? 1u : 0u) << k;
-                            ml |= (lo_l <= ul ? 1u : 0u) << k;
-                            mam |= (lo_h == -INFINITY ? 1u : 0u) << k;
-                        }
-                    } else if (a.exact_ratio) {
-                        mh = ml = mam = (EPT >= 32) ? 0xFFFFFFFFu : ((1u << EPT) - 1u);
-                    }
-                    for (unsigned m = mh | ml; m; m &= m - 1) {
-                        const int k = __ffs(m) - 1;
-                        const unsigned bit = 1u << k;
-                        const int i = tid + k * BD;
-                        ++nex;
-                        const double xi = xs[i], dk = pick(dreg, k);
-                        const double2 lu = ld_lbub(a.lbub + i);
-                        const double Dp = lu.y - xi, Dm = xi - lu.x;
-                        bool valid = true;
-                        if (mam & bit) {  // undecided: full FP64 candidacy test
-                            bool u_pass;
-                            if (have_norm64) {
-                                u_pass = abs_bits(dk) > (unsigned long long)__double_as_longlong(thr64);
-                            } else {
-                                const float ad32 = fabsf(f64_to_f32_rz(dk));
-                                // inside the FP32 norm's margin: settled with the FP64 norm
-                                if (!(ad32 > uthr_hi) && !(ad32 * kAdUp < uthr_lo)) need64 = 1;
-                                u_pass = ad32 > uthr_hi;
+                            for (int k = 0; k < KP; ++k) {
+                                if (ACHR_PAD_SLOT(k)) continue;
+                                const float4 b = __ldg(bnd2 + tid + k * BD);
+                                ACHR_X32(k, x0, x1)
+#pragma unroll
+                                for (int c = 0; c < 2; ++c) {
+                                    const Bracket B = bracket(c ? x1 : x0, d_to_f32(dreg[2 * k + c]), c ? b.z : b.x,
+                                                              c ? b.w : b.y, e0, 0.0f, uthr_lo);
+                                    mh |= (B.live && B.lo_h <= uh ? 1u : 0u) << (2 * k + c);
+                                    ml |= (B.live && B.lo_l <= ul ? 1u : 0u) << (2 * k + c);
+                                }
                             }
-                            valid = Dp > a.d_tol && Dm > a.d_tol && u_pass;
                         }
-                        if (valid) {
-                            const double ad = abs_int(dk);
-                            const bool pos = positive_int(dk);
-                            if (mh & bit) kh = umin(kh, (unsigned long long)__double_as_longlong((pos ? Dp : Dm) / ad));
-                            if (ml & bit) kl = umin(kl, (unsigned long long)__double_as_longlong((pos ? Dm : Dp) / ad));
-                            anyv = 1;
+                        if (mh | ml) atomicAdd(exact_count, __popc(mh | ml));
+                        while (mh | ml) {
+                            const int k = __ffs(mh | ml) - 1;
+                            const unsigned bit = 1u << k;
+                            const int i = 2 * (tid + (k >> 1) * BD) + (k & 1);
+                            const bool side_h = (mh & bit) != 0;
+                            if (side_h) mh &= ~bit;
+                            else ml &= ~bit;
+                            evaluate(a, t, xs[i], pick(dreg, k), i, __ldg(a.bnd + i), side_h);
                         }
-                    }
-                    if (nex) atomicAdd(exact_count, nex);
-                    kh = warp_min_u64(kh);
-                    kl = warp_min_u64(kl);
-                    anyv = (int)__reduce_or_sync(0xffffffffu, (unsigned)(anyv | (need64 << 1)));
-                    if (lane == 0) {
-                        rs->min3[warp] = make_ulonglong2(kh, kl);
-                        rs->flag3[warp] = anyv;
-                    }
-                    __syncthreads();
-                    kh = kInfBits;
-                    kl = kInfBits;
-                    anyv = 0;
+                    } else {
+                        // A thread's elements one per lane: the warp passes them their d
+                        // (a thread forming its own EPT brackets again held up the chain
+                        // for a thousand clocks a step).
+                        for (unsigned m = __ballot_sync(0xffffffffu, mine); m; m &= m - 1) {
+                            const int src = __ffs(m) - 1;
+                            double dk = 0.0;
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const ulonglong2 v = rs->min3[w];
-                        kh = umin(kh, v.x);
-                        kl = umin(kl, v.y);
-                        anyv |= rs->flag3[w];
+                            for (int k = 0; k < EPT; ++k) {
+                                const double v = __shfl_sync(0xffffffffu, dreg[k], src);
+                                dk = lane == k ? v : dk;
+                            }
+                            const int i = 2 * (warp * 32 + src + (lane >> 1) * BD) + (lane & 1);
+                            bool h = false, l = false;
+                            double xi = 0.0;
+                            float2 b = make_float2(0.0f, 0.0f);
+                            if (lane < EPT) {
+                                xi = xs[i];
+                                b = __ldg(a.bnd + i);
+                                const Bracket B = bracket(x_to_f32(xi), d_to_f32(dk), b.x, b.y, e0, 0.0f, uthr_lo);
+                                h = B.live && B.lo_h <= uh;
+                                l = B.live && B.lo_l <= ul;
+                            }
+                            if (h || l) atomicAdd(exact_count, 1);
+                            while (h || l) {  // one coordinate is rarely a contender for both
+                                evaluate(a, t, xi, dk, i, b, h);
+                                if (h) h = false;
+                                else l = false;
+                            }
+                            __syncwarp();
+                        }
                     }
-                    if (!(anyv & 2) || have_norm64) break;
-                    fl |= 4;  // a contender's candidacy needs the FP64 norm: evaluate again with it
+                    if (NW > 1) {  // a contender or two per step: they meet in shared memory
+                        if (t.found) {
+                            atomicMin(&rs->kh, t.kh);
+                            atomicMin(&rs->kl, t.kl);
+                            atomicOr(&rs->flags, (unsigned)t.found);
+                        }
+                        cta_sync<BD>();
+                        t.kh = rs->kh;
+                        t.kl = rs->kl;
+                        anyv = (int)rs->flags;
+                    } else {
+                        __syncwarp();
+                        t.kh = warp_min_u64(t.kh);
+                        t.kl = warp_min_u64(t.kl);
+                        anyv = (int)__reduce_or_sync(0xffffffffu, (unsigned)t.found);
+                    }
+                    if (!(anyv & 2) || t.have_norm64) break;
+                    // a contender's candidacy needs the FP64 norm: evaluate again with it
+                    want_norm64 = true;
+                    cta_sync<BD>();
+                    if (tid == 0) rs->clear();  // (the norm's barrier follows)
                 }
                 anyv &= 1;
                 if (!anyv) {  // no candidate: rejection (see ACHRCuda.cu:283-288)
                     if (tid == 0) ++cnt[CNT_REJECTED];
                     continue;
                 }
-                const double qh = __longlong_as_double((long long)kh);
-                const double ql = __longlong_as_double((long long)kl);
+                const double qh = __longlong_as_double((long long)t.kh);
+                const double ql = __longlong_as_double((long long)t.kl);
 
                 // Rejection test |min| < tol && |max| < tol (ACHRCuda.cu:316-319),
                 // min = -ql ||d||, max = qh ||d||; FP32 unless inside the margin.
@@ -967,9 +1110,9 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                         for (int k = 0; k < EPT; ++k) s64 = fma(dreg[k], dreg[k], s64);
 #pragma unroll
                         for (int o = 16; o; o >>= 1) s64 += __shfl_xor_sync(0xffffffffu, s64, o);
-                        __syncthreads();  // slot sum5 may hold this attempt's earlier norm
+                        cta_sync<BD>();  // slot sum5 may hold this attempt's earlier norm
                         if (lane == 0) rs->sum5[warp] = s64;
-                        __syncthreads();
+                        cta_sync<BD>();
                         s64 = 0.0;
 #pragma unroll
                         for (int w = 0; w < NW; ++w) s64 += rs->sum5[w];
@@ -981,132 +1124,146 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                     if (tid == 0) ++cnt[CNT_REJECTED];
                     continue;
                 }
-                // t / ||d|| with t = U (max - min) + min (reference ACHRCuda.cu:314)
-                const double sstep = fma(te->U, qh + ql, -ql);
+                // t / ||d|| with t = U (max - min) + min (reference ACHRCuda.cu:314).
+                // One warp computes it: its two FP64 instructions in each of 12 warps
+                // would hold the pipe for 465 clocks, the extra barrier costs 60.
+                double sstep;
+                if (NW > 1) {
+                    if (warp == 0) {
+                        const double v = fma(te->U, qh + ql, -ql);
+                        if (lane == 0) rs->step = v;
+                    }
+                    cta_sync<BD>();
+                    sstep = rs->step;
+                } else {
+                    sstep = fma(te->U, qh + ql, -ql);
+                }
 
                 // Phase C: x = prev + t u (ACHRCuda.cu:242-249), residual check every
                 // check_period steps (:325-344), clip + centre (:193-206, :347-350).
                 const bool check = chk == 0;
                 chk = (chk + 1 == a.check_period) ? 0 : chk + 1;
-                if (!check && hr) {  // hit-and-run: no centre to update
-                    unsigned edge = 0;
-#pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) continue;
-                        const double xn = fma(sstep, dreg[k], xs[i]);
-                        xs[i] = xn;
-                        if (!surely_inside(f64_to_f32_rz(xn), __ldg(a.bnd + i), a.bound_err)) edge |= 1u << k;
-                    }
-                    for (; edge; edge &= edge - 1) {
-                        const int i = tid + (__ffs(edge) - 1) * BD;
-                        xs[i] = clip_exact(xs[i], ld_lbub(a.lbub + i));
-                    }
-                } else if (!check) {
+                // The next step's column, requested as dreg's pairs come free (the
+                // table's last step leaves it to the next step's refill).
+                const int nxt = (s + 1 < a.step0 + a.T && s + 1 - tbase < kTbl) ? (int)tbl[s + 1 - tbase].idx : -1;
+                const bool pre = nxt >= 0 && nxt < a.W;
+                const double2 *ncol =
+                    reinterpret_cast<const double2 *>(a.warmup + (size_t)(pre ? nxt : 0) * (size_t)a.ldw);
+                if (!check) {
                     unsigned edge = 0;  // bit k: not provably inside the box, clip exactly below
 #pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) continue;
-                        const double xn = fma(sstep, dreg[k], xs[i]);
-                        xs[i] = xn;
-                        if (surely_inside(f64_to_f32_rz(xn), __ldg(a.bnd + i), a.bound_err)) As[i] += xn;
-                        else edge |= 1u << k;
+                    for (int k = 0; k < KP; ++k) {
+                        const int q = tid + k * BD;
+                        if (!ACHR_PAD_SLOT(k)) {
+                            const float4 b = __ldg(bnd2 + q);
+                            double2 x2 = xs2[q];
+                            x2.x = fma(sstep, dreg[2 * k], x2.x);
+                            x2.y = fma(sstep, dreg[2 * k + 1], x2.y);
+                            xs2[q] = x2;
+                            const float x0 = x_to_f32(x2.x), x1 = x_to_f32(x2.y);
+                            if (KX) {
+                                xf[KX ? 2 * k : 0] = x0;
+                                xf[KX ? 2 * k + 1 : 1] = x1;
+                            }
+                            const bool in0 = surely_inside(x0, b.x, b.y, a.bound_err);
+                            const bool in1 = surely_inside(x1, b.z, b.w, a.bound_err);
+                            edge |= (in0 ? 0u : 1u << (2 * k)) | (in1 ? 0u : 2u << (2 * k));
+                            if (!hr) {  // hit-and-run: no centre to update
+                                double2 A2 = As2[q];
+                                if (in0) A2.x += x2.x;
+                                if (in1) A2.y += x2.y;
+                                As2[q] = A2;
+                            }
+                        }
+                        if (pre && q < npair) {
+                            const double2 v = ld_column(ncol + q);
+                            dreg[2 * k] = v.x;
+                            dreg[2 * k + 1] = v.y;
+                        }
                     }
-                    for (; edge; edge &= edge - 1) {
-                        const int i = tid + (__ffs(edge) - 1) * BD;
-                        const double xc = clip_exact(xs[i], ld_lbub(a.lbub + i));
-                        xs[i] = xc;
-                        As[i] += xc;
-                    }
-                } else if (SEG) {
-                    // Segmented sampling: the check ends this launch for the chain.
+                    if (pre) buf_col = nxt;
+                    if (edge) {
+                        for (; edge; edge &= edge - 1) {
+                            const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
+                            const double xc = clip_exact(xs[i], exact_bounds(a, i));
+                            xs[i] = xc;
+                            if (!hr) As[i] += xc;
+                        }
+                        if (KX) {
 #pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
+                            for (int k = 0; k < KP; ++k) {
+                                const double2 x2 = xs2[tid + k * BD];
+                                xf[KX ? 2 * k : 0] = x_to_f32(x2.x);
+                                xf[KX ? 2 * k + 1 : 1] = x_to_f32(x2.y);
+                            }
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < KP; ++k) {
+                        const int q = tid + k * BD;
                         if (ACHR_PAD_SLOT(k)) continue;
-                        xs[i] = fma(sstep, dreg[k], xs[i]);
+                        double2 x2 = xs2[q];
+                        x2.x = fma(sstep, dreg[2 * k], x2.x);
+                        x2.y = fma(sstep, dreg[2 * k + 1], x2.y);
+                        xs2[q] = x2;
                     }
-                    if (inflight) {  // (the launch ends here, so nothing was prefetched; kept for safety)
-                        if (!mbar_wait_bounded(bar, phase)) failed = true;
-                        phase ^= 1u;
-                        inflight = false;
-                    }
-                    __syncthreads();  // every x update visible; the staging buffer is free
+                    cta_sync<BD>();  // every x update visible
                     if (tid == 0) ++cnt[CNT_CHECKS];
-                    double *rr = ws;  // S x, m doubles (m <= BD * EPT for segmented launches)
-                    unsigned long long mx = residual_rows<BD>(a, xs, rr, tid);
-                    mx = warp_max_u64(mx);
-                    if (lane == 0) rs->max4[warp] = mx;
-                    __syncthreads();
-                    mx = 0;
+                    if (SEG) {
+                        // Segmented sampling: the check ends this launch for the chain.  S x goes
+                        // out as it is summed (FP64 and BF16 split, device row order); the passes
+                        // read it only for a chain flagged below.
+                        unsigned long long mx = residual_rows<BD>(a, xs, p, tid);
+                        mx = warp_max_u64(mx);
+                        if (lane == 0) rs->max4[warp] = mx;
+                        cta_sync<BD>();
+                        mx = 0;
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) mx = umax(mx, rs->max4[w]);
-                    const bool reproject = mx > (unsigned long long)__double_as_longlong(a.residual_tol);
-                    if (reproject) {
-                        if (tid == 0) {
+                        for (int w = 0; w < NW; ++w) mx = umax(mx, rs->max4[w]);
+                        const bool reproject = mx > (unsigned long long)__double_as_longlong(a.residual_tol);
+                        if (reproject && tid == 0) {
                             ++cnt[CNT_REPROJ];
                             if (*a.seg_any == 0ull) atomicOr(a.seg_any, 1ull);
                         }
-                        unsigned short *rh = a.seg_Rh + (size_t)p * (size_t)a.kpad;
-                        unsigned short *rl = a.seg_Rl + (size_t)p * (size_t)a.kpad;
-                        double *rd = a.seg_rd + (size_t)p * (size_t)a.ld_r;
-                        for (int q = tid; q < a.m; q += BD) {
-                            // (no FP64 operation: the FP32 image for the split is a truncation by
-                            // integer operations, and the FP64 value is stored as it is)
-                            unsigned short h, l;
-                            split_bf16_bits(f64_to_f32_rz(rr[q]), h, l);
-                            rh[q] = h;  // device row order, as the batched passes read them
-                            rl[q] = l;
-                            rd[q] = rr[q];
-                        }
-                    }
 #pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (i < a.n) {
-                            a.seg_x[(size_t)p * (size_t)a.ld_seg + (size_t)i] = xs[i];
-                            a.seg_A[(size_t)p * (size_t)a.ld_seg + (size_t)i] = As[i];
+                        for (int k = 0; k < EPT; ++k) {
+                            const int i = tid + k * BD;
+                            if (i < a.n) {
+                                a.seg_x[(size_t)p * (size_t)a.ld_seg + (size_t)i] = xs[i];
+                                a.seg_A[(size_t)p * (size_t)a.ld_seg + (size_t)i] = As[i];
+                            }
                         }
+                        if (tid == 0) {
+                            a.seg_flags[p] =
+                                SEG_STARTED | SEG_ACCEPTED | SEG_PENDING | (reproject ? SEG_REPROJ : 0u);
+                            ++cnt[CNT_ACCEPTED];
+                        }
+                        any_accepted = true;
+                        seg_pending = true;
+                        ++it;
+                        break;
                     }
-                    if (tid == 0) {
-                        a.seg_flags[p] =
-                            SEG_STARTED | SEG_ACCEPTED | SEG_PENDING | (reproject ? SEG_REPROJ : 0u);
-                        ++cnt[CNT_ACCEPTED];
-                    }
-                    __syncthreads();  // the residual rows in ws are read before the next chain's column lands
-                    any_accepted = true;
-                    seg_pending = true;
-                    break;
-                } else {
-#pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) continue;
-                        xs[i] = fma(sstep, dreg[k], xs[i]);
-                    }
-                    __syncthreads();
-                    if (tid == 0) ++cnt[CNT_CHECKS];
                     unsigned long long mx = residual_max_bits<BD>(a, xs, tid);
                     mx = warp_max_u64(mx);
                     if (lane == 0) rs->max4[warp] = mx;
-                    __syncthreads();
+                    cta_sync<BD>();
                     mx = 0;
 #pragma unroll
                     for (int w = 0; w < NW; ++w) mx = umax(mx, rs->max4[w]);
                     if (mx > (unsigned long long)__double_as_longlong(a.residual_tol)) {
                         // x <- N (N^T x) in FP64 (reference reprojectPoint(2), ACHRCuda.cu:208-230).
-                        // The scratch is ws: let the prefetched column land, use the
-                        // buffer, then fetch the column again.
+                        // The scratch is As: the accumulator waits in the direction's registers.
                         if (tid == 0) ++cnt[CNT_REPROJ];
-                        if (inflight) {
-                            if (!mbar_wait_bounded(bar, phase)) failed = true;
-                            phase ^= 1u;
-                            inflight = false;
+#pragma unroll
+                        for (int k = 0; k < KP; ++k) {
+                            const double2 A2 = As2[tid + k * BD];
+                            dreg[2 * k] = A2.x;
+                            dreg[2 * k + 1] = A2.y;
                         }
-                        if (__syncthreads_or(failed ? 1 : 0)) failed = true;  // block-uniform from here
+                        cta_sync<BD>();
                         if (a.pinv32) {
-                            residual_form_reproject<BD>(a, xs, reinterpret_cast<float2 *>(ws), zs, tid);
+                            residual_form_reproject<BD>(a, xs, reinterpret_cast<float2 *>(As), zs, tid);
                         } else {
                             const int n = a.n;
                             for (int j = warp; j < a.d; j += NW) {
@@ -1117,7 +1274,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                                 for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                                 if (lane == 0) ys[j] = acc;
                             }
-                            __syncthreads();
+                            cta_sync<BD>();
                             for (int i = tid; i < n; i += BD) {
                                 double acc = 0.0;
                                 for (int j = 0; j < a.d; ++j)
@@ -1125,47 +1282,67 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                                 xs[i] = acc;
                             }
                         }
-                        __syncthreads();
-                        if (buf_col >= 0) {
-                            if (tid == 0) {
-                                fence_proxy_async_smem();
-                                mbar_arrive_expect_tx(bar, column_bytes(a));
-                                tma_load_1d(ws, a.warmup + (size_t)buf_col * (size_t)a.ldw, column_bytes(a), bar);
-                            }
-                            inflight = true;
-                        }
+                        cta_sync<BD>();
+#pragma unroll
+                        for (int k = 0; k < KP; ++k)
+                            As2[tid + k * BD] = make_double2(dreg[2 * k], dreg[2 * k + 1]);
                     }
                     unsigned edge = 0;
 #pragma unroll
-                    for (int k = 0; k < EPT; ++k) {
-                        const int i = tid + k * BD;
-                        if (ACHR_PAD_SLOT(k)) continue;
-                        const double xv = xs[i];
-                        if (surely_inside(f64_to_f32_rz(xv), __ldg(a.bnd + i), a.bound_err)) {
-                            if (!hr) As[i] += xv;
+                    for (int k = 0; k < KP; ++k) {
+                        const int q = tid + k * BD;
+                        if (!ACHR_PAD_SLOT(k)) {
+                            const float4 b = __ldg(bnd2 + q);
+                            const double2 x2 = xs2[q];
+                            const float x0 = x_to_f32(x2.x), x1 = x_to_f32(x2.y);
+                            if (KX) {
+                                xf[KX ? 2 * k : 0] = x0;
+                                xf[KX ? 2 * k + 1 : 1] = x1;
+                            }
+                            const bool in0 = surely_inside(x0, b.x, b.y, a.bound_err);
+                            const bool in1 = surely_inside(x1, b.z, b.w, a.bound_err);
+                            edge |= (in0 ? 0u : 1u << (2 * k)) | (in1 ? 0u : 2u << (2 * k));
+                            if (!hr) {
+                                double2 A2 = As2[q];
+                                if (in0) A2.x += x2.x;
+                                if (in1) A2.y += x2.y;
+                                As2[q] = A2;
+                            }
+                        }
+                        if (pre && q < npair) {
+                            const double2 v = ld_column(ncol + q);
+                            dreg[2 * k] = v.x;
+                            dreg[2 * k + 1] = v.y;
                         } else {
-                            edge |= 1u << k;
+                            dreg[2 * k] = dreg[2 * k + 1] = 0.0;
                         }
                     }
-                    for (; edge; edge &= edge - 1) {
-                        const int i = tid + (__ffs(edge) - 1) * BD;
-                        const double xc = clip_exact(xs[i], ld_lbub(a.lbub + i));
-                        xs[i] = xc;
-                        if (!hr) As[i] += xc;
+                    if (pre) buf_col = nxt;
+                    if (edge) {
+                        for (; edge; edge &= edge - 1) {
+                            const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
+                            const double xc = clip_exact(xs[i], exact_bounds(a, i));
+                            xs[i] = xc;
+                            if (!hr) As[i] += xc;
+                        }
+                        if (KX) {
+#pragma unroll
+                            for (int k = 0; k < KP; ++k) {
+                                const double2 x2 = xs2[tid + k * BD];
+                                xf[KX ? 2 * k : 0] = x_to_f32(x2.x);
+                                xf[KX ? 2 * k + 1 : 1] = x_to_f32(x2.y);
+                            }
+                        }
                     }
                 }
                 if (tid == 0) ++cnt[CNT_ACCEPTED];
                 any_accepted = true;
+                ++it;  // the next attempt takes the other slots
                 break;
             }
         }
-        if (inflight) {
-            if (!mbar_wait_bounded(bar, phase)) failed = true;
-            phase ^= 1u;
-            inflight = false;
-        }
         if (stuck && !was_stuck && tid == 0) ++cnt[CNT_STUCK];
-        if (__syncthreads_or(failed ? 1 : 0)) {
+        if (cta_any<BD>(failed)) {
             failed = true;
             break;
         }
@@ -1183,27 +1360,30 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 a.seg_flags[p] = SEG_STARTED | (any_accepted ? SEG_ACCEPTED : 0u) | (stuck ? SEG_STUCK : 0u);
         }
         if (SEG && (seg_pending || !a.seg_final)) {
-            __syncthreads();
+            cta_sync<BD>();
             continue;  // the point is emitted by the run's last launch
         }
 
         // Emitted point: residual / bound diagnostics and, on request, the final
         // feasibility projection (project, clip, re-check).
         if (any_accepted) {
-            RedSlots *rs = rsb;
+            RedSlots<NW> *rs = rsb;
             const int n = a.n;
             unsigned long long res = 0;
             for (int pass = 0; pass < 2; ++pass) {
                 unsigned long long mx = residual_max_bits<BD>(a, xs, tid);
                 mx = warp_max_u64(mx);
-                __syncthreads();
+                cta_sync<BD>();
                 if (lane == 0) rs->max4[warp] = mx;
-                __syncthreads();
+                cta_sync<BD>();
                 res = 0;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) res = umax(res, rs->max4[w]);
                 if (pass == 1 || !a.final_project || __longlong_as_double((long long)res) <= a.feasibility_tol) break;
                 if (tid == 0) ++cnt[CNT_FINAL_PROJ];
+#pragma unroll
+                for (int k = 0; k < EPT; ++k) dreg[k] = As[tid + k * BD];
+                cta_sync<BD>();
                 for (int j = warp; j < a.d; j += NW) {
                     const double *Nj = a.N + (size_t)j * (size_t)n;
                     double acc = 0.0;
@@ -1212,13 +1392,15 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                     if (lane == 0) ys[j] = acc;
                 }
-                __syncthreads();
+                cta_sync<BD>();
                 for (int i = tid; i < n; i += BD) {
                     double acc = 0.0;
                     for (int j = 0; j < a.d; ++j) acc = fma(__ldg(a.N + (size_t)j * (size_t)n + i), ys[j], acc);
                     xs[i] = clip_exact(acc, ld_lbub(a.lbub + i));
                 }
-                __syncthreads();
+                cta_sync<BD>();
+#pragma unroll
+                for (int k = 0; k < EPT; ++k) As[tid + k * BD] = dreg[k];
             }
             double viol = 0.0;
             for (int i = tid; i < n; i += BD) {
@@ -1228,9 +1410,9 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
             }
             unsigned long long vb = (unsigned long long)__double_as_longlong(viol);
             vb = warp_max_u64(vb);
-            __syncthreads();
+            cta_sync<BD>();
             if (lane == 0) rs->max4[warp] = vb;
-            __syncthreads();
+            cta_sync<BD>();
             vb = 0;
 #pragma unroll
             for (int w = 0; w < NW; ++w) vb = umax(vb, rs->max4[w]);
@@ -1242,12 +1424,13 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
         for (int i = tid; i < a.n; i += BD) a.out[(size_t)i * (size_t)a.ld_out + (size_t)p] = any_accepted ? xs[i] : 0.0;
         if (a.A_out)
             for (int i = tid; i < a.n; i += BD) a.A_out[(size_t)i * (size_t)a.ld_state + (size_t)p] = As[i];
-        __syncthreads();
+        cta_sync<BD>();
     }
 #undef ACHR_CHAIN_ID
 #undef ACHR_PAD_SLOT
+#undef ACHR_X32
 
-    __syncthreads();
+    cta_sync<BD>();
     if (tid == 0) {
         unsigned long long *c = a.counters;
         const int slots[6] = {CNT_ACCEPTED, CNT_REJECTED, CNT_CHECKS, CNT_REPROJ, CNT_STUCK, CNT_FINAL_PROJ};
@@ -1261,26 +1444,19 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     return failed;
 }
 
-// The staging barriers of a CTA (header of the dynamic shared memory).
-template <int NP>
-__device__ __forceinline__ void chain_init_barriers(unsigned char *smem_raw) {
-    uint64_t *bar, *never;
-    chain_barriers<NP>(smem_raw, bar, never);
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        mbar_init(never, 1);
-        fence_mbar_init();
-    }
+// The `never` barrier of a CTA (tail of the dynamic shared memory).
+template <int BD, int EPT>
+__device__ __forceinline__ void chain_init_barrier(unsigned char *smem_raw) {
+    if (threadIdx.x == 0) mbar_init(chain_never<BD, EPT>(smem_raw), 1);
     __syncthreads();
 }
 
 // One model: CTA b takes chains b, b + grid, ...
 template <int BD, int EPT, bool SEG>
-__global__ void __launch_bounds__(BD, (BD <= 384 ? 2 : 1)) achr_chain_kernel(const ChainArgs a) {
+__global__ void __launch_bounds__(BD, (chain_min_ctas<BD, EPT>())) achr_chain_kernel(const ChainArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    chain_init_barriers<BD * EPT>(smem_raw);
-    unsigned phase = 0;
-    chain_run<BD, EPT, SEG>(a, blockIdx.x, gridDim.x, a.P, smem_raw, phase);
+    chain_init_barrier<BD, EPT>(smem_raw);
+    chain_run<BD, EPT, SEG>(a, blockIdx.x, gridDim.x, a.P, smem_raw);
 }
 
 // Many models of one configuration in one persistent launch: each CTA takes
@@ -1291,13 +1467,12 @@ __global__ void __launch_bounds__(BD, (BD <= 384 ? 2 : 1)) achr_chain_kernel(con
 // model's last chain is done, its finish time (globaltimer, ns) goes to
 // done_ns[model].
 template <int BD, int EPT>
-__global__ void __launch_bounds__(BD, (BD <= 384 ? 2 : 1)) achr_chain_queue_kernel(const ChainQueue q) {
+__global__ void __launch_bounds__(BD, (chain_min_ctas<BD, EPT>())) achr_chain_queue_kernel(const ChainQueue q) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ ChainArgs sa;
     __shared__ int4 cur;
     static_assert(sizeof(ChainArgs) % sizeof(int) == 0, "ChainArgs is copied as 32-bit words");
-    chain_init_barriers<BD * EPT>(smem_raw);
-    unsigned phase = 0;
+    chain_init_barrier<BD, EPT>(smem_raw);
     int model = -1;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1314,7 +1489,7 @@ __global__ void __launch_bounds__(BD, (BD <= 384 ? 2 : 1)) achr_chain_queue_kern
             model = item.x;
         }
         __syncthreads();
-        const bool failed = chain_run<BD, EPT, false>(sa, item.y, 1, item.z, smem_raw, phase);
+        const bool failed = chain_run<BD, EPT, false>(sa, item.y, 1, item.z, smem_raw);
         if (threadIdx.x == 0) {
             const int n = item.z - item.y;
             if (atomicAdd(q.chains_done + item.x, n) + n == sa.P) q.done_ns[item.x] = global_ns();
@@ -1331,12 +1506,12 @@ template <int BD, int EPT, bool SEG>
 cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int max_ctas, int *per_sm_out) {
     auto *const KFN = achr_chain_kernel<BD, EPT, SEG>;
     ChainArgs a = a_in;
-    const size_t base = chain_smem_bytes_cfg(BD * EPT, a.d, BD);
+    const size_t base = chain_smem_bytes_cfg<BD, EPT>();
     // The residual-form reprojection keeps z (m floats) in shared memory and
-    // the residual in the staging buffer; it is used only when both fit
+    // the residual in the accumulator's place; it is used only when z fits
     // without costing a resident CTA per SM.
     const size_t zbytes = ((size_t)a.m * sizeof(float) + 15) & ~(size_t)15;
-    // (its residual occupies the column buffer below the buffer's zero padding: m <= ldw)
+    // (its residual takes the accumulator's NP doubles while that waits in registers: m <= ldw <= NP)
     if (a.pinv32 && a.m > a.ldw) a.pinv32 = nullptr;
     size_t smem = base + (a.pinv32 ? zbytes : 0);
     cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1375,7 +1550,7 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
 template <int BD, int EPT>
 cudaError_t launch_queue_cfg(const ChainQueue &q, cudaStream_t stream, int grid, int *per_sm_out) {
     auto *const KFN = achr_chain_queue_kernel<BD, EPT>;
-    const size_t smem = chain_smem_bytes_cfg(BD * EPT, 0, BD) + q.extra_smem;
+    const size_t smem = chain_smem_bytes_cfg<BD, EPT>() + q.extra_smem;
     cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

@@ -22,18 +22,23 @@ struct Cfg {
     bool dflt;
 };
 
-// Ordered by padded length; the default for each length comes first.
-// 320 x 12 and 384 x 10 (3840 elements) put 20 or 24 warps on an SM with two
-// chains each, against 16 for 256 x 16, at the cost of fewer registers per
-// thread; 384 x 10 is the default up to 3840 reactions (2.04e7 against 1.95e7
-// chain-steps/s for 256 x 16 on a 2766 x 3742 model).  512 x 12 and 512 x 15
-// cut the padding of 4097-7680 reactions (a 7440-reaction model pads to 7680,
-// not 8192: 3 % of the FP64 work on padding instead of 10 %).
+// Ordered by padded length; the default for each length comes first.  The
+// kernel is bound by the FP64 pipe once enough chains share an SM to fill each
+// other's latency, so a default has few warps per chain (each repeats the
+// reductions) where shared memory still holds four chains or more, and more
+// warps where it holds two.  Measured, SM clocks per chain-step at full
+// residency (the previous kernel's in brackets): n = 95, 32 x 4: 400 [689];
+// n = 1060, 64 x 20: 3550 [7760], 256 x 8: 4920; n = 2500, 128 x 20: 6900,
+// 320 x 12: 8680; n = 3000, 128 x 24: 8690, 320 x 12: 9080; n = 3742, 320 x 12:
+// 10190 [13960 with 384 x 10], 384 x 10: 10350, 256 x 16: 10940; n = 7440, 384 x
+// 20: 26500 [31020 with 512 x 15], 512 x 16: 26600.  The others serve an explicit
+// threads_per_chain and the autotuner.
 const Cfg kLadder[] = {
-    {32, 4, true},    {64, 4, true},    {32, 8, false},   {128, 4, true},  {64, 8, false},
-    {128, 8, true},   {256, 4, false},  {256, 8, true},   {128, 16, false}, {512, 4, false},
-    {320, 12, false}, {384, 10, true},  {256, 16, true},  {512, 8, false},  {128, 32, false},
-    {512, 12, true},  {512, 15, true},  {512, 16, true},  {512, 32, true},
+    {32, 4, true},    {64, 4, false},   {32, 8, true},    {64, 6, true},    {128, 4, false},  {64, 8, true},
+    {64, 12, true},   {64, 16, true},   {128, 8, false},  {256, 4, false},  {64, 20, true},   {128, 12, true},
+    {128, 16, true},  {256, 8, false},  {512, 4, false},  {128, 20, true},  {128, 24, true},  {320, 12, true},
+    {384, 10, false}, {256, 16, true},  {512, 8, false},  {128, 32, false}, {256, 18, true},  {256, 20, true},
+    {256, 24, true},  {512, 12, false}, {256, 26, true},  {384, 20, true},  {512, 16, true},  {512, 32, true},
 };
 
 const Cfg *find_cfg(int n, int threads_per_chain) {
@@ -76,13 +81,6 @@ int chain_candidates(int n, int max_np, int *bds, int cap) {
     return k;
 }
 
-size_t chain_smem_bytes(int n, int d, int ldw, int block) {
-    (void)ldw;
-    (void)d;
-    const int np = chain_padded_length(n, block);
-    return sizeof(double) * 3 * (size_t)np + 24 * 64 + 2 * 1792 + 128;
-}
-
 bool chain_config(int n, int threads_per_chain, int *bd, int *ept) {
     const Cfg *c = find_cfg(n, threads_per_chain);
     if (!c) return false;
@@ -92,9 +90,8 @@ bool chain_config(int n, int threads_per_chain, int *bd, int *ept) {
 }
 
 cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_t stream, int grid, int *per_sm) {
-    if (bd <= 128) return launch_chain_queue_small(bd, ept, q, stream, grid, per_sm);
-    if (bd == 320 || bd == 384 || (bd == 512 && (ept == 12 || ept == 15)))
-        return launch_chain_queue_mid(bd, ept, q, stream, grid, per_sm);
+    if (bd <= 64) return launch_chain_queue_small(bd, ept, q, stream, grid, per_sm);
+    if (bd <= 128) return launch_chain_queue_mid(bd, ept, q, stream, grid, per_sm);
     return launch_chain_queue_large(bd, ept, q, stream, grid, per_sm);
 }
 
@@ -103,9 +100,8 @@ cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_
     const Cfg *c = find_cfg(a.n, threads_per_chain);
     if (!c || c->bd * c->ept > a.np) return cudaErrorInvalidValue;
     if (a.P <= 0 && !per_sm) return cudaSuccess;
-    if (c->bd <= 128) return launch_chain_cfg_small(c->bd, c->ept, a, stream, max_ctas, per_sm);
-    if (c->bd == 320 || c->bd == 384 || (c->bd == 512 && (c->ept == 12 || c->ept == 15)))
-        return launch_chain_cfg_mid(c->bd, c->ept, a, stream, max_ctas, per_sm);
+    if (c->bd <= 64) return launch_chain_cfg_small(c->bd, c->ept, a, stream, max_ctas, per_sm);
+    if (c->bd <= 128) return launch_chain_cfg_mid(c->bd, c->ept, a, stream, max_ctas, per_sm);
     return launch_chain_cfg_large(c->bd, c->ept, a, stream, max_ctas, per_sm);
 }
 

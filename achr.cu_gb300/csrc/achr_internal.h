@@ -41,6 +41,7 @@ struct ChainArgs {
     const double *A0;           // np: (W + centre_offset) * c0, the centre accumulator at step 0
     const double2 *lbub;        // np: (lb, ub) in FP64; padding (0, 0)
     const float2 *bnd;          // np: (lb, ub) rounded to FP32, infinite bounds as -+3e38; padding (-1, 1)
+    int bound_exact;            // 1: every bound is finite and exact in FP32, so bnd holds the bounds themselves
     float bound_err;            // max |lb - float(lb)|, |ub - float(ub)| over finite bounds, rounded up
     float dtol_hi, dtol_lo;     // FP32 brackets of d_tol (1 +- 2^-20)
     float utol32, mmt32;        // u_tol and max_min_tol in FP32
@@ -139,6 +140,13 @@ inline float f32_down(double v) {
     return f;
 }
 
+// Whether a finite bound equals its FP32 image as a normal number or zero (the
+// chain kernel widens the image with integer operations, which drop subnormals).
+inline bool f32_exact_bound(double v) {
+    const float f = (float)v;
+    return (double)f == v && (v == 0.0 || std::fabs(v) >= 1.1754943508222875e-38);
+}
+
 // Upper bound of the FP32 candidacy threshold u_tol ||d|| (times its margin)
 // for the ratio-test brackets formed before the block norm is known, from a
 // bound on ||d||; without a finite bound the brackets keep their own pass.
@@ -173,7 +181,6 @@ int chain_padded_length(int n, int threads_per_chain);
 int chain_alloc_length(int n);
 // Threads-per-chain values worth timing for n (padded length within max_np).
 int chain_candidates(int n, int max_np, int *bds, int cap);
-size_t chain_smem_bytes(int n, int d, int ldw, int block);
 
 // Tensor-core GEMM (achr_tc_gemm.cu): C (M x N, FP32, row-major, ldc) =
 // A0 B0^T (nsplit 1) or A0 B0^T + A0 B1^T + A1 B0^T (nsplit 3); operands BF16

@@ -109,11 +109,11 @@ typedef struct {
     double u_tol;             /* 1e-9 (ACHRCuda.cu:508) */
     double d_tol;             /* 1e-14 (ACHRCuda.cu:512) */
     double feasibility_tol;   /* 1e-8: ||S v||_inf bound for emitted points in FEASIBLE mode */
-    int32_t wait_limit_ns;    /* bound on the chain kernel's wait for a staged warmup column; on expiry
-                                 the launch stops, drains its copy and returns ACHR_ERR_TIMEOUT
-                                 (0: the default of 2 s).  A negative value -L is a test of that
-                                 path: the wait is on a barrier nothing completes and runs out after
-                                 L ns every time. */
+    int32_t wait_limit_ns;    /* limit of the chain kernel's bounded wait (0: the default of 2 s).  Warmup
+                                 columns are read with ordinary loads, so only the failure-detection
+                                 test waits: a negative value -L makes each CTA wait on a barrier nothing
+                                 completes, which runs out after L ns every time; the launch then stops
+                                 and the call returns ACHR_ERR_TIMEOUT. */
     int32_t bracket_pass;     /* FP32 ratio-test brackets (ACHRCuda.cu:266-281): 0: formed in the same pass
                                  as the direction, before its norm is known, with the candidacy threshold
                                  bounded through the box (or the longest hit-and-run direction); a step
