@@ -46,6 +46,7 @@
 #include <cmath>
 
 #include "achr_div.cuh"
+#include "achr_float.cuh"
 #include "achr_internal.h"
 #include "achr_rng.cuh"
 
@@ -67,19 +68,6 @@ constexpr float kDCert = 1.5777218104420236e-30f;      // 2^-99: no smaller |d| 
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bounded mbarrier wait: 2 s
 constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 
-// FP64 -> FP32 rounding toward zero with integer operations only.
-// |v - f| <= 2^-23 |f| + 2^-126; tiny values flush to signed zero, overflow
-// and inf map to inf.
-__device__ __forceinline__ float f64_to_f32_rz(double v) {
-    const unsigned hi = (unsigned)__double2hiint(v);
-    const unsigned lo = (unsigned)__double2loint(v);
-    const int fe = (int)((hi >> 20) & 0x7FFu) - 896;  // re-bias 1023 -> 127
-    unsigned mag = ((unsigned)fe << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-    mag = (fe <= 0) ? 0u : mag;
-    mag = (fe >= 255) ? 0x7F800000u : mag;
-    return __uint_as_float((hi & 0x80000000u) | mag);
-}
-
 // The same for the hot loops, in six integer operations: the magnitude is
 // clamped to [2^LO_EXP, 2^128 (1 - 2^-20)) in its FP64 form (three spare low
 // bits of a clamped value are below the error bound), then the exponent is
@@ -97,24 +85,6 @@ __device__ __forceinline__ float f64_to_f32_clamped(double v) {
 // x: clamped at 2^-126 (kTiny covers it); d: clamped at kDMin.
 __device__ __forceinline__ float x_to_f32(double v) { return f64_to_f32_clamped<-126>(v); }
 __device__ __forceinline__ float d_to_f32(double v) { return f64_to_f32_clamped<-100>(v); }
-
-// Order-preserving integer key of a double (sign-magnitude -> two's
-// complement; -0 and +0 share key 0).  a < b  <=>  key(a) < key(b) for non-NaN.
-__device__ __forceinline__ long long order_key(double v) {
-    const long long b = __double_as_longlong(v);
-    const long long mag = b & 0x7FFFFFFFFFFFFFFFll;
-    return b < 0 ? -mag : mag;
-}
-
-// Exact clip of x to [lb, ub] (reference correctBounds, ACHRCuda.cu:198-202):
-// x itself when inside, else the bound, compared through integer keys.
-__device__ __forceinline__ double clip_exact(double x, double2 lu) {
-    const long long kx = order_key(x);
-    double r = x;
-    if (kx < order_key(lu.x)) r = lu.x;
-    if (kx > order_key(lu.y)) r = lu.y;
-    return r;
-}
 
 // |v| and its bit pattern through integer operations (fabs on a double can be
 // issued to the FP64 pipe).
@@ -448,32 +418,10 @@ __device__ __forceinline__ double fp64_zero_here() {
     return z;
 }
 
-// FP32 -> FP64 with integer operations only (exact for normal values; zero and
-// subnormal values give a signed zero).
-__device__ __forceinline__ double f32_to_f64_exact(float f) {
-    const unsigned u = __float_as_uint(f);
-    const unsigned e = (u >> 23) & 0xFFu;
-    const unsigned long long s = (unsigned long long)(u & 0x80000000u) << 32;
-    if (e == 0) return __longlong_as_double((long long)s);
-    return __longlong_as_double(
-        (long long)(s | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(u & 0x7FFFFFu) << 29)));
-}
-
 __device__ __forceinline__ double2 exact_bounds(const ChainArgs &a, int i) {
     if (!a.bound_exact) return ld_lbub(a.lbub + i);
     const float2 b = __ldg(a.bnd + i);
     return make_double2(f32_to_f64_exact(b.x), f32_to_f64_exact(b.y));
-}
-
-// BF16 bits of f rounded to nearest even (hi) and of the remainder f - hi (lo),
-// for finite f; FP32 and integer operations only.
-__device__ __forceinline__ void split_bf16_bits(float f, unsigned short &hi, unsigned short &lo) {
-    const unsigned u = __float_as_uint(f);
-    const unsigned hu = (u + 0x7FFFu + ((u >> 16) & 1u)) & 0xFFFF0000u;
-    hi = (unsigned short)(hu >> 16);
-    const unsigned r = __float_as_uint(f - __uint_as_float(hu));
-    const unsigned ru = (r + 0x7FFFu + ((r >> 16) & 1u)) & 0xFFFF0000u;
-    lo = (unsigned short)(ru >> 16);
 }
 
 // The same row sums as residual_max_bits (same rows, same order of terms, so

@@ -47,7 +47,9 @@ struct ReprojState {
     double lam_max = 0.0, lam_min = 0.0;
     DevBuf<__nv_bfloat16> Bh, Bl;  // m x kpad row-major: (S S^T)^+ split into hi + lo
     DevBuf<int> rp, ci, cp, ri;    // CSR and CSC of S (original row order)
-    DevBuf<double> rv, cv;
+    DevBuf<double> rv;
+    DevBuf<float> ch, cl;          // CSC values in FP32 hi + lo
+    bool exact32 = false;          // every lo part is zero
     DevBuf<__nv_bfloat16> Rh, Rl;  // chunk x kpad: residuals of a chunk of chains, hi + lo
     DevBuf<float> Z;               // m x chunk: B r for the chunk
     int chunk_cap = 0;

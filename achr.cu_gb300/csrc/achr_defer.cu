@@ -56,6 +56,7 @@
 #include <vector>
 
 #include "achr_ctx.h"
+#include "achr_float.cuh"
 
 extern "C" void achr_io_set_error(const char *msg);
 
@@ -126,43 +127,6 @@ achr_status set_err(achr_status st, const std::string &msg) {
         cudaError_t e_ = (expr);                                                                               \
         if (e_ != cudaSuccess) return set_err(ACHR_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
-
-// Error-free transformations on FP32 (IEEE round-to-nearest; nvcc neither
-// reassociates these nor contracts them beyond the explicit fmaf).
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-__device__ __forceinline__ void fast_two_sum(float a, float b, float &s, float &e) {  // |a| >= |b| or a = 0
-    s = __fadd_rn(a, b);
-    e = __fsub_rn(b, __fsub_rn(s, a));
-}
-__device__ __forceinline__ void two_prod(float a, float b, float &p, float &e) {
-    p = __fmul_rn(a, b);
-    e = fmaf(a, b, -p);
-}
-
-// FP64 -> (hi, lo) FP32 with integer operations only: hi is v truncated to 24
-// significant bits, lo the rest (up to 29 bits, rounded to 24); |v - hi - lo|
-// <= 2^-48 |v|.  Values below 2^-126 become 0.
-__device__ __forceinline__ void split_f64(double v, float &hi, float &lo) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-    const int e = (int)((b >> 52) & 0x7FF);
-    const int fe = e - 896;  // FP32 biased exponent
-    if (fe <= 0 || fe >= 255) {
-        hi = (fe >= 255) ? __uint_as_float(sign | 0x7F800000u) : __uint_as_float(sign);
-        lo = 0.0f;
-        return;
-    }
-    const unsigned long long mant = b & 0xFFFFFFFFFFFFFull;
-    hi = __uint_as_float(sign | ((unsigned)fe << 23) | (unsigned)(mant >> 29));
-    const unsigned rest = (unsigned)(mant & 0x1FFFFFFFull);  // the low 29 bits: rest * 2^(e - 1075)
-    const float r = __uint2float_rn(rest);
-    const float l = ldexpf(r, e - 1075);
-    lo = sign ? -l : l;
-}
 
 __device__ __forceinline__ void split_store(float r, __nv_bfloat16 *rh, __nv_bfloat16 *rl, int i) {
     const __nv_bfloat16 h = __float2bfloat16_rn(r);

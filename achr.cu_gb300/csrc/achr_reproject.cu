@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "achr_ctx.h"
+#include "achr_float.cuh"
 
 extern "C" void achr_io_set_error(const char *msg);
 
@@ -46,9 +47,12 @@ void reproj_free(ReprojState *r) { delete r; }
 namespace {
 
 constexpr int kRowChunk = 64;   // residual rows per staging tile (one 128-byte BF16 row per chain)
-constexpr int kResWarps = 4;
+constexpr int kResWarps = 8;
 constexpr int kStageStride = 72;  // BF16 entries per chain row of the staging tile (144 B: 16-byte aligned)
 constexpr int kCorrWarps = 8;
+constexpr int kCorrRows = 16;     // reactions per warp of the correction
+constexpr int kLoads = 4;         // nonzeros requested before any is used
+constexpr size_t kResSmem = (size_t)kResWarps * 2 * 32 * kStageStride * sizeof(__nv_bfloat16);
 constexpr int kMaxChunk = 65536;  // chains per GEMM
 
 achr_status set_err(achr_status st, const std::string &msg) {
@@ -70,12 +74,18 @@ __device__ __forceinline__ unsigned long long abs_bits64(double v) {
     return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
 }
 
-// r = S x for 32 chains per block column (lane = chain, so every load of x is
+// r = S x for 32 chains per block row (lane = chain, so every load of x is
 // one coalesced 256-byte row segment) and 64-row chunks per warp.  With SPLIT
 // the residuals go out as BF16 hi/lo rows of R (chain-major, K = metabolite
 // contiguous, the layout the GEMM's TMA maps read), staged through shared
 // memory so every chain row is written as 16-byte pieces.  Always: the
 // largest |r| (as non-negative double bits) goes to *maxbits.
+//
+// Bound by the FP64 pipe: one DFMA per nonzero and chain (5063 x 7440, 16,384
+// chains: 0.98 ms at the pipe's rate) and nothing else on it, the split being
+// integer and FP32 work.  The blocks of one group of chains run together (the
+// row chunks vary fastest), so the group's 1.9 MB of x stay in L2 for the four
+// times its rows are read.
 template <bool SPLIT>
 __global__ void __launch_bounds__(kResWarps * 32)
     residual_kernel(int m, int kpad, int P, const double *__restrict__ X, long long ldx,
@@ -88,32 +98,41 @@ __global__ void __launch_bounds__(kResWarps * 32)
         if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *maxbits = *prev;
         return;
     }
-    __shared__ __align__(16) __nv_bfloat16 stage[SPLIT ? kResWarps : 1][2][32 * kStageStride];
+    extern __shared__ __align__(16) unsigned short stage_raw[];  // [warp][hi, lo][chain][row]
     __shared__ unsigned long long wmax[kResWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p0 = blockIdx.x * 32;
+    unsigned short *const sh = stage_raw + (size_t)warp * 2 * 32 * kStageStride, *const sl = sh + 32 * kStageStride;
+    const int p0 = blockIdx.y * 32;
     const int p = p0 + lane;
     const bool live = p < P;
-    const double *xp = X + (live ? p : 0);
+    const double *xp = X + (live ? p : P - 1);
     unsigned long long mx = 0;
     const int nchunks = kpad / kRowChunk;
-    for (int c = blockIdx.y * kResWarps + warp; c < nchunks; c += gridDim.y * kResWarps) {
+    for (int c = blockIdx.x * kResWarps + warp; c < nchunks; c += gridDim.x * kResWarps) {
         for (int r = 0; r < kRowChunk; ++r) {
             const int i = c * kRowChunk + r;
             double acc = 0.0;
             if (i < m) {
                 const int q1 = __ldg(rp + i + 1);
-                for (int q = __ldg(rp + i); q < q1; ++q) {
-                    const double xv = live ? xp[(long long)__ldg(ci + q) * ldx] : 0.0;
-                    acc = fma(__ldg(rv + q), xv, acc);
+                for (int q = __ldg(rp + i); q < q1; q += kLoads) {
+                    double v[kLoads], x[kLoads];
+#pragma unroll
+                    for (int u = 0; u < kLoads; ++u) {  // past the row: its last entry again, not used
+                        const int qq = min(q + u, q1 - 1);
+                        v[u] = __ldg(rv + qq);
+                        x[u] = xp[(long long)__ldg(ci + qq) * ldx];
+                    }
+#pragma unroll
+                    for (int u = 0; u < kLoads; ++u)
+                        if (q + u < q1) acc = fma(v[u], x[u], acc);
                 }
             }
-            mx = max(mx, abs_bits64(acc));
+            if (live) mx = max(mx, abs_bits64(acc));
             if (SPLIT) {
-                const __nv_bfloat16 hi = __double2bfloat16(acc);
-                const __nv_bfloat16 lo = __double2bfloat16(acc - (double)__bfloat162float(hi));
-                stage[SPLIT ? warp : 0][0][lane * kStageStride + r] = hi;
-                stage[SPLIT ? warp : 0][1][lane * kStageStride + r] = lo;
+                unsigned short h, l;
+                split_bf16_bits(f64_to_f32_near(acc), h, l);
+                sh[lane * kStageStride + r] = h;
+                sl[lane * kStageStride + r] = l;
             }
         }
         if (SPLIT) {
@@ -124,9 +143,9 @@ __global__ void __launch_bounds__(kResWarps * 32)
                 if (pp < P) {
                     const size_t off = (size_t)pp * (size_t)kpad + (size_t)c * kRowChunk + (size_t)part * 8;
                     *reinterpret_cast<uint4 *>(Rh + off) =
-                        *reinterpret_cast<const uint4 *>(&stage[SPLIT ? warp : 0][0][row * kStageStride + part * 8]);
+                        *reinterpret_cast<const uint4 *>(&sh[row * kStageStride + part * 8]);
                     *reinterpret_cast<uint4 *>(Rl + off) =
-                        *reinterpret_cast<const uint4 *>(&stage[SPLIT ? warp : 0][1][row * kStageStride + part * 8]);
+                        *reinterpret_cast<const uint4 *>(&sl[row * kStageStride + part * 8]);
                 }
             }
             __syncwarp();
@@ -142,28 +161,55 @@ __global__ void __launch_bounds__(kResWarps * 32)
     }
 }
 
-// x_j <- clip(x_j - sum_i S_ij z_i, lb_j, ub_j) for 32 chains per block column
+// x_j <- clip(x_j - sum_i S_ij z_i, lb_j, ub_j) for 32 chains per block row
 // (lane = chain: loads of z and x are coalesced rows); the centre accumulator
-// moves with the point.
+// moves with the point.  The sum is formed in double-float on the FP32 pipes
+// (error-free products and sums, about 48 bits: far below z's own FP32
+// rounding), so the FP64 pipe does only dh + dl, x - d and the accumulator's
+// two additions; the clip compares integers.  Summed and converted in FP64 it
+// was the larger half of a round (3.4 ms of 6.6 at 5063 x 7440, 16,384 chains).
+// The blocks of one group of chains run together, so the group's z stays in L2.
+template <bool EXACT32>
 __global__ void __launch_bounds__(kCorrWarps * 32)
     correct_kernel(int n, int P, double *__restrict__ X, long long ldx, double *__restrict__ Acc, long long lda,
-                   const int *__restrict__ cp, const int *__restrict__ ri, const double *__restrict__ cv,
-                   const float *__restrict__ Z, long long ldz, const double2 *__restrict__ lbub,
-                   const unsigned long long *gate, unsigned long long tol_bits) {
+                   const int *__restrict__ cp, const int *__restrict__ ri, const float *__restrict__ ch,
+                   const float *__restrict__ cl, const float *__restrict__ Z, long long ldz,
+                   const double2 *__restrict__ lbub, const unsigned long long *gate, unsigned long long tol_bits) {
     if (*gate <= tol_bits) return;  // this chunk's residual is already within tolerance
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p = blockIdx.x * 32 + lane;
+    const int p = blockIdx.y * 32 + lane;
     if (p >= P) return;
-    for (int j = blockIdx.y * kCorrWarps + warp; j < n; j += gridDim.y * kCorrWarps) {
-        double dl = 0.0;
+    const float *zp = Z + p;
+    for (int j = blockIdx.x * kCorrWarps + warp; j < n; j += gridDim.x * kCorrWarps) {
+        float ah = 0.0f, al = 0.0f;
         const int q1 = __ldg(cp + j + 1);
-        for (int q = __ldg(cp + j); q < q1; ++q)
-            dl = fma(__ldg(cv + q), (double)__ldg(Z + (long long)__ldg(ri + q) * ldz + p), dl);
+        for (int q = __ldg(cp + j); q < q1; q += kLoads) {
+            float vh[kLoads], vl[kLoads], z[kLoads];
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u) {
+                const int qq = min(q + u, q1 - 1);
+                vh[u] = __ldg(ch + qq);
+                if (!EXACT32) vl[u] = __ldg(cl + qq);
+                z[u] = __ldg(zp + (long long)__ldg(ri + qq) * ldz);
+            }
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u)
+                if (q + u < q1) {
+                    float ph, pe, s, e;
+                    two_prod(vh[u], z[u], ph, pe);
+                    if (!EXACT32) pe = fmaf(vl[u], z[u], pe);
+                    two_sum(ah, ph, s, e);
+                    ah = s;
+                    al = __fadd_rn(al, __fadd_rn(e, pe));
+                }
+        }
         double *xp = X + (long long)j * ldx + p;
         const double xo = *xp;
-        const double2 lu = lbub[j];
-        double xn = xo - dl;
-        xn = xn < lu.x ? lu.x : (xn > lu.y ? lu.y : xn);
+        double d;
+        if (fabsf(ah) + fabsf(al) < INFINITY) d = f32_to_f64_exact(ah) + f32_to_f64_exact(al);
+        else d = (double)ah + (double)al;  // (infinite or NaN: keep it so)
+        const double xc = xo - d;
+        const double xn = abs_bits64(xc) > 0x7FF0000000000000ull ? xc : clip_exact(xc, lbub[j]);
         *xp = xn;
         if (Acc) Acc[(long long)j * lda + p] += xn - xo;
     }
@@ -227,7 +273,15 @@ achr_status build_reproj(achr_ctx *ctx, ReprojState &R, bool want_pinv32 = false
     REPROJ_TRY(R.rv.upload(rv.data(), rv.size()));
     REPROJ_TRY(R.cp.upload(cp.data(), cp.size()));
     REPROJ_TRY(R.ri.upload(ri.data(), ri.size()));
-    REPROJ_TRY(R.cv.upload(cv.data(), cv.size()));
+    std::vector<float> ch(cv.size()), cl(cv.size());
+    R.exact32 = true;
+    for (size_t q = 0; q < cv.size(); ++q) {
+        ch[q] = (float)cv[q];
+        cl[q] = (float)(cv[q] - (double)ch[q]);
+        R.exact32 = R.exact32 && cl[q] == 0.0f;
+    }
+    REPROJ_TRY(R.ch.upload(ch.data(), ch.size()));
+    REPROJ_TRY(R.cl.upload(cl.data(), cl.size()));
 
     // B = (S S^T)^+ from the eigen-decomposition of S S^T, eigenvalues below
     // m * lambda_max * 2.2204e-16 dropped (the reference's null-space cutoff
@@ -352,7 +406,7 @@ double bits_to_double(unsigned long long b) {
 
 dim3 residual_grid(int P, int kpad) {
     const int nchunks = kpad / kRowChunk;
-    return dim3((unsigned)((P + 31) / 32), (unsigned)((nchunks + kResWarps - 1) / kResWarps));
+    return dim3((unsigned)((nchunks + kResWarps - 1) / kResWarps), (unsigned)((P + 31) / 32));
 }
 
 }  // namespace
@@ -409,6 +463,7 @@ achr_status achr_reproject_batch(achr_ctx *ctx, int32_t n_points, double *d_poin
     st = ensure_chunk(R, chunk);
     if (st != ACHR_OK) return st;
     const int nchunks = (n_points + chunk - 1) / chunk;
+    REPROJ_TRY(cudaFuncSetAttribute(residual_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
     const size_t nflags = 8 + (size_t)max_rounds * nchunks;
     if (R.flags.count < nflags) REPROJ_TRY(R.flags.alloc(nflags));
     cudaStream_t s = (cudaStream_t)stream_v;
@@ -445,7 +500,7 @@ achr_status achr_reproject_batch(achr_ctx *ctx, int32_t n_points, double *d_poin
             double *X = d_points + c0;
             unsigned long long *slot = R.flags.p + 8 + (size_t)r * nchunks + c;
             const unsigned long long *prev = r > 0 ? slot - nchunks : nullptr;
-            residual_kernel<true><<<residual_grid(pc, R.kpad), kResWarps * 32, 0, s>>>(
+            residual_kernel<true><<<residual_grid(pc, R.kpad), kResWarps * 32, kResSmem, s>>>(
                 R.m, R.kpad, pc, X, ld, R.rp.p, R.ci.p, R.rv.p, R.Rh.p, R.Rl.p, slot, prev, tol_bits);
             REPROJ_TRY(cudaGetLastError());
             TcGemm g{R.m, pc, R.kpad, 3, R.Bh.p, R.Bl.p, (long long)R.kpad, R.Rh.p, R.Rl.p, (long long)R.kpad,
@@ -464,18 +519,22 @@ achr_status achr_reproject_batch(achr_ctx *ctx, int32_t n_points, double *d_poin
                 gemm_ev.emplace_back(g0, g1);
             }
             chunk_flops[(size_t)c] = tc_gemm_flops(g);
-            const int ny = std::max(1, std::min((R.n + kCorrWarps * 16 - 1) / (kCorrWarps * 16), 65535));
-            correct_kernel<<<dim3((unsigned)((pc + 31) / 32), (unsigned)ny), kCorrWarps * 32, 0, s>>>(
-                R.n, pc, X, ld, d_centre_acc ? d_centre_acc + c0 : nullptr, ld, R.cp.p, R.ri.p, R.cv.p, R.Z.p,
+            const dim3 cgrid((unsigned)((R.n + kCorrWarps * kCorrRows - 1) / (kCorrWarps * kCorrRows)),
+                             (unsigned)((pc + 31) / 32));
+            (R.exact32 ? correct_kernel<true> : correct_kernel<false>)<<<cgrid, kCorrWarps * 32, 0, s>>>(
+                R.n, pc, X, ld, d_centre_acc ? d_centre_acc + c0 : nullptr, ld, R.cp.p, R.ri.p, R.ch.p, R.cl.p, R.Z.p,
                 (long long)pc, ctx->lbub.p, slot, tol_bits);
             REPROJ_TRY(cudaGetLastError());
         }
     }
     if (stats) {
-        residual_kernel<false><<<residual_grid(n_points, R.kpad), kResWarps * 32, 0, s>>>(
-            R.m, R.kpad, n_points, d_points, ld, R.rp.p, R.ci.p, R.rv.p, nullptr, nullptr, R.flags.p + 1, nullptr,
-            0ull);
-        REPROJ_TRY(cudaGetLastError());
+        for (int c0 = 0; c0 < n_points; c0 += chunk) {
+            const int pc = std::min(chunk, n_points - c0);
+            residual_kernel<false><<<residual_grid(pc, R.kpad), kResWarps * 32, 0, s>>>(
+                R.m, R.kpad, pc, d_points + c0, ld, R.rp.p, R.ci.p, R.rv.p, nullptr, nullptr, R.flags.p + 1, nullptr,
+                0ull);
+            REPROJ_TRY(cudaGetLastError());
+        }
         REPROJ_TRY(cudaEventRecord(t1, s));
     }
     std::vector<unsigned long long> h(nflags, 0);
