@@ -177,9 +177,11 @@ achr_status validate_options(const achr_options &o) {
 // n * sigma_0 * 2.2204e-16; the basis is every eigenvector whose eigenvalue
 // magnitude is below the cutoff (ACHRCuda.cu:459-489).  If no value falls
 // below the cutoff the reference keeps istart = 0 and uses all n columns.
+// row (or NULL) receives the other eigenpairs; its vectors stay in V_out.
 achr_status null_space_sts(int n, int m, const std::vector<double> &denseS, std::vector<double> &N, int &d,
-                           double &kappa) {
-    DevBuf<double> dS, dStS, dW, work;
+                           double &kappa, achr::RowSpace *row = nullptr, DevBuf<double> *V_out = nullptr) {
+    DevBuf<double> dS, own, dW, work;
+    DevBuf<double> &dStS = V_out ? *V_out : own;
     DevBuf<int> info;
     ACHR_CUDA_TRY(dS.upload(denseS.data(), (size_t)m * n));
     ACHR_CUDA_TRY(dStS.alloc((size_t)n * n));
@@ -224,6 +226,11 @@ achr_status null_space_sts(int n, int m, const std::vector<double> &denseS, std:
     }
     // condition number of S S^T on its range (the same non-zero spectrum as S^T S)
     kappa = lkept > 0.0 ? smax / lkept : 1.0;
+    // (eigenvalues ascend, so the row space is the trailing block of columns)
+    if (row && (cols.empty() || cols.back() == (int)cols.size() - 1)) {
+        row->V = dStS.p + cols.size() * (size_t)n;
+        row->lam.assign(lam.begin() + (std::ptrdiff_t)cols.size(), lam.end());
+    }
     if (cols.empty())
         for (int i = 0; i < n; ++i) cols.push_back(i);
     d = (int)cols.size();
@@ -426,7 +433,10 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     if (!ctx) return fail(ACHR_ERR_NOMEM, "context allocation failed");
     struct Guard {
         achr_ctx *&c;
-        ~Guard() { delete c; }
+        ~Guard() {
+            if (c) achr::reproj_free(c->reproj);
+            delete c;
+        }
     };
     achr_ctx *owned = ctx;
     Guard guard{owned};
@@ -582,6 +592,8 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
             denseS[(size_t)ctx->h_colidx[q] * m + r] = ctx->h_val[q];
     std::vector<double> Nh;
     int d = 0;
+    achr::RowSpace row_space;  // from the null space's eigen-decomposition, for the reprojection operator
+    DevBuf<double> eigenvectors;
     if (m == 0) {
         // No constraints: the reference's rule keeps every column (identity basis).
         d = n;
@@ -603,17 +615,19 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
         ctx->kappa_sst = INFINITY;  // the deferred projector (built from S alone) would not match this basis
     } else {
         st = (opt.null_space == ACHR_NULL_SVD_S) ? null_space_svd_s(n, m, denseS, Nh, d, ctx->kappa_sst)
-                                                 : null_space_sts(n, m, denseS, Nh, d, ctx->kappa_sst);
+                                                 : null_space_sts(n, m, denseS, Nh, d, ctx->kappa_sst, &row_space,
+                                                                  &eigenvectors);
         if (st != ACHR_OK) return st;
     }
     st = upload_null_space(ctx, Nh.data(), d);
     if (st != ACHR_OK) return st;
+    const achr::RowSpace *rows = row_space.V ? &row_space : nullptr;
     // Large models reproject a chain through (S S^T)^+ on the residual (about
     // m^2 FP32 operations) instead of N (N^T x) (4 n d FP64 operations).
     const bool want_residual_form =
         opt.reproject_form == 2 || (opt.reproject_form == 0 && (double)n * (double)d >= 4.0e6);
     if (want_residual_form && m > 0 && m <= std::min(np, 8192)) {
-        st = achr::build_pinv32(ctx);
+        st = achr::build_operator(ctx, true, rows);
         if (st != ACHR_OK) return st;
     }
 
@@ -623,6 +637,13 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     ACHR_CUDA_TRY(ctx->A0.alloc(np));
     st = prepare_warmup_and_centre(ctx);
     if (st != ACHR_OK) return st;
+    // Sampling on these warmup points will need the reprojection operator: build it
+    // while the eigenvectors are here (on first use it takes a decomposition of its own,
+    // which for a small model is milliseconds).
+    if (rows && achr::defer_selected(ctx) && (double)n * (double)d >= 1.0e4) {
+        st = achr::build_operator(ctx, false, rows);
+        if (st != ACHR_OK) return st;
+    }
 
     owned = nullptr;  // release from the guard
     *out = ctx;
@@ -673,7 +694,7 @@ achr_status achr_sample_device(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
     }
     // Reprojections either inside the chain kernel, or deferred to a batched
     // tensor-core pass between segmented launches (achr_defer.cu).
-    const bool deferred = achr::defer_selected(ctx) && n_points > 0 && n_steps > 0;
+    const bool deferred = achr::defer_chosen(ctx, a, s);
     if (ctx->opt.reproject_form == 3 && !deferred && n_points > 0 && n_steps > 0 && ctx->opt.check_period > 0 &&
         ctx->m > 0) {
         if (e0) cudaEventDestroy(e0);
@@ -850,7 +871,7 @@ achr_status achr_sample_resume(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
         ACHR_CUDA_TRY(cudaEventCreate(&e1));
         ACHR_CUDA_TRY(cudaEventRecord(e0, s));
     }
-    const bool deferred = achr::defer_selected(ctx) && n_points > 0 && n_steps > 0;
+    const bool deferred = achr::defer_chosen(ctx, a, s);
     cudaError_t e = cudaSuccess;
     achr_status dst = ACHR_OK;
     if (deferred) dst = achr::defer_sample(ctx, a, ctx->opt.threads_per_chain, s, stats != nullptr);

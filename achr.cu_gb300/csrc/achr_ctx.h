@@ -64,9 +64,15 @@ void defer_free(DeferState *d);  // achr_defer.cu
 
 struct achr_ctx;
 namespace achr {
-// (S S^T)^+ in FP32, rows and columns in the device row order, into ctx->pinv32
-// (achr_reproject.cu; builds the batched-reprojection operator on the way).
-achr_status build_pinv32(achr_ctx *ctx);
+// Eigenvectors of S^T S with eigenvalues above the null-space cutoff (device, n x lam.size(),
+// column-major) and those eigenvalues.
+struct RowSpace {
+    const double *V = nullptr;
+    std::vector<double> lam;
+};
+// The batched-reprojection operator and, with want_pinv32, (S S^T)^+ in FP32 in the device row order
+// (ctx->pinv32), from the row space if it is given (achr_reproject.cu).
+achr_status build_operator(achr_ctx *ctx, bool want_pinv32, const RowSpace *eig);
 // The batched-reprojection operator of the context, built on first use.
 achr_status ensure_reproj(achr_ctx *ctx);
 // Segmented sampling with the per-chain reprojections deferred to a batched
@@ -77,8 +83,11 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a, int threads_per_chai
 // After the stream of a timed defer_sample has completed: device time of its
 // chain-kernel launches and of its batched passes, and the chains per sweep.
 achr_status defer_times(achr_ctx *ctx, double *chain_ms, double *pass_ms, double *chains_per_sweep);
-// Whether sampling with these options takes the deferred path.
+// Whether sampling with these options may take the deferred path, and whether a
+// run of n_points chains described by `a` on `stream` does (deferred sampling's
+// buffers are then ready, or will be built by defer_sample).
 bool defer_selected(const achr_ctx *ctx);
+bool defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream);
 }  // namespace achr
 
 struct achr_ctx {

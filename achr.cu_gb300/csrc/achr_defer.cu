@@ -735,8 +735,7 @@ bool defer_selected(const achr_ctx *ctx) {
     const achr_options &o = ctx->opt;
     if (o.check_period <= 0 || ctx->m <= 0) return false;
     const int np = chain_padded_length(ctx->n, o.threads_per_chain);
-    // S x is staged in the chain kernel's column buffer, below its zero padding (the padding
-    // beyond the column's ldw entries must stay zero: padded reactions read it as their w)
+    // (the chain kernel's padding stays zero: m <= ldw keeps every per-row block below it)
     if (np == 0 || ctx->m > ctx->ldw) return false;
     // Each BF16-split pass multiplies the remaining error by roughly 1.5e-6 times the
     // condition number of S S^T (measured: 1.9e-3 at 1265); beyond 2e4 the passes
@@ -744,20 +743,60 @@ bool defer_selected(const achr_ctx *ctx) {
     if (ctx->kappa_sst > kDeferMaxKappa) return false;
     if (o.reproject_form == 3) return true;
     if (o.reproject_form != 0 || ctx->n_dirs > 0) return false;
-    return ctx->warmup_residual > o.residual_tol / 8.0 && (double)ctx->n * (double)ctx->d >= 2.5e5;
+    return ctx->warmup_residual > o.residual_tol / 8.0;
+}
+
+// Reprojecting P chains in the chain kernel takes P 4 n d FP64 operations at every
+// check, deferring it about 0.1 ms of launches and passes, so the line lies at a
+// work of P n d.  Measured per 50 steps (five checks), in the kernel / deferred:
+//   n = 95, d = 20:    P = 1000 0.23 / 0.64 ms, 5000 0.75 / 1.18
+//   n = 200, d = 43:   P = 1000 0.49 / 0.82,    5000 1.85 / 1.58   (P n d = 8.6e6, 4.3e7)
+//   n = 400, d = 84:   P = 1000 1.08 / 0.87,    5000 5.19 / 2.23   (3.4e7, 1.7e8)
+//   n = 1060, d = 159: P = 1000 3.92 / 1.61,    5000 19.9 / 5.62
+// Models of n d >= 2.5e5 are always deferred.
+constexpr double kDeferWork = 2.0e7, kDeferModel = 2.5e5;
+
+namespace {
+
+int segments_of(const ChainArgs &a) { return (a.step0 + a.T) / a.check_period - a.step0 / a.check_period + 3; }
+
+// Operator, buffers and one gate word per launch and pass ([seg * (kMaxPasses + 1) + pass]) of a run.
+achr_status prepare(achr_ctx *ctx, const ChainArgs &a) {
+    const achr_status st = ensure_reproj(ctx);
+    return st != ACHR_OK ? st : ensure_defer(ctx, std::min(a.P, kDeferChunk), segments_of(a) * (kMaxPasses + 1));
+}
+
+}  // namespace
+
+bool defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream) {
+    if (a.P <= 0 || a.T <= 0 || !defer_selected(ctx)) return false;
+    const double nd = (double)ctx->n * (double)ctx->d;
+    if (ctx->opt.reproject_form == 3 || nd >= kDeferModel) return true;
+    if ((double)a.P * nd < kDeferWork) return false;
+    // A model that could as well reproject in the kernel does so where the buffers
+    // cannot be had: their memory is short, or the stream is being captured (a
+    // capture allows no allocation).
+    const DeferState *D = ctx->defer;
+    if (D && ctx->reproj && D->cap >= std::min(a.P, kDeferChunk) && D->any_cap >= segments_of(a) * (kMaxPasses + 1))
+        return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (prepare(ctx, a) == ACHR_OK) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_chain, cudaStream_t s, bool timed) {
-    achr_status st = ensure_reproj(ctx);
-    if (st != ACHR_OK) return st;
     // Steps [S0, E) of every chain (S0 > 0: chains resumed from a_in.x_in / A_in).
     const int P = a_in.P, S0 = a_in.step0, E = a_in.step0 + a_in.T, k = a_in.check_period;
     if (P <= 0) return ACHR_OK;
-    const int cap = std::min(P, kDeferChunk);
-    const int segments = E / k - S0 / k + 3;
-    // one gate word per launch and pass: [seg * (kMaxPasses + 1) + pass]
-    st = ensure_defer(ctx, cap, segments * (kMaxPasses + 1));
+    const achr_status st = prepare(ctx, a_in);
     if (st != ACHR_OK) return st;
+    const int cap = std::min(P, kDeferChunk);
+    const int segments = segments_of(a_in);
     DeferState &D = *ctx->defer;
     const ReprojState &R = *ctx->reproj;
     D.ev_used = 0;

@@ -83,8 +83,9 @@ typedef struct {
     int32_t reproject_form;   /* per-chain reprojection x <- N (N^T x) (ACHRCuda.cu:208-230) computed as
                                  0: chosen by the inputs: deferred (3) when the warmup points carry a
                                     residual max|S w| > residual_tol / 8 (a %f-rounded CSV: nearly every
-                                    check then reprojects), n_rxns x null_dim >= 2.5e5 and form 3's
-                                    conditions hold; otherwise in the chain kernel, as 2 when
+                                    check then reprojects), n_rxns x null_dim >= 2.5e5 or chains x
+                                    n_rxns x null_dim >= 2e7, and form 3's conditions hold; otherwise
+                                    in the chain kernel, as 2 when
                                     n_rxns x null_dim >= 4e6, else as 1,
                                  1: N (N^T x) in FP64 in the chain kernel,
                                  2: x - S^T (S S^T)^+ S x in the chain kernel, the pseudo-inverse product
