@@ -129,5 +129,6 @@ struct achr_ctx {
     // reactions that are fixed across all warmup points also held fixed
     // (n x d_act, column-major); built on first use by the preconditioner.
     achr::DevBuf<double> Nact;
+    achr::DevBuf<__nv_bfloat16> NactH, NactL;  // the same, transposed and split (d_act x n rounded up to 64)
     int d_act = -1, n_frozen = 0;
 };

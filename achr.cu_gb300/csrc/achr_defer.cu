@@ -190,9 +190,10 @@ __device__ __forceinline__ float over_warps(const float *r) {
 }
 
 
-// Shared-memory floats per chain of the pass kernels (multiples of 4, so every
-// chain's block starts on a 16-byte boundary): z (ldz floats) and d, as a
-// double-float pair in the first pass, in FP32 in the later ones.
+// Shared-memory floats per chain of the pass kernels (multiples of 4): z (ldz
+// floats) and d, as a double-float pair in the first pass, in FP32 in the later
+// ones.  The chains of a CTA are interleaved (entry i of every chain side by
+// side), so one 8- or 16-byte gather serves all of them.
 __host__ __device__ inline size_t pass1_floats(long long ldz, long long ld) {
     return ((size_t)ldz + 2 * (size_t)ld + 3) & ~(size_t)3;
 }
@@ -200,36 +201,65 @@ __host__ __device__ inline size_t pass_floats(long long ldz, long long ld) {
     return ((size_t)ldz + (size_t)ld + 3) & ~(size_t)3;
 }
 
-// The kernels below are bound by latency, not by bandwidth or arithmetic: each
-// sparse slot is a global load of its index and value followed by a shared-
-// memory gather, and each per-chain vector moves between global and shared
-// memory.  So every loop issues a batch of independent loads before it uses
-// any of them: kSlots slots of a sparse line, and two elements per thread of
+// C consecutive floats (aligned to their size, at most 16 bytes at a time).
+template <int C>
+__device__ __forceinline__ void load_vec(const float *p, float (&v)[C]) {
+    if constexpr (C == 1) {
+        v[0] = *p;
+    } else if constexpr (C == 2) {
+        const float2 x = *reinterpret_cast<const float2 *>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+    } else {
+#pragma unroll
+        for (int c = 0; c < C; c += 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(p + c);
+            v[c] = x.x;
+            v[c + 1] = x.y;
+            v[c + 2] = x.z;
+            v[c + 3] = x.w;
+        }
+    }
+}
+template <int C>
+__device__ __forceinline__ void store_vec(float *p, const float (&v)[C]) {
+    if constexpr (C == 1) {
+        *p = v[0];
+    } else if constexpr (C == 2) {
+        *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < C; c += 4) *reinterpret_cast<float4 *>(p + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+    }
+}
+
+// The kernels below are bound by shared-memory gathers and by latency, not by
+// bandwidth or arithmetic: each sparse slot is a global load of its index and
+// value followed by a gather at random banks, and each per-chain vector moves
+// between global and shared memory.  Interleaving the chains makes one gather
+// of two or four, and every loop issues a batch of independent loads before it
+// uses any of them: kSlots slots of a sparse line, four elements per thread of
 // every resident chain's vectors.
 constexpr int kSlots = 8;
+constexpr int kVecLoads = 4;
 
-// z rows of the CTA's live chains into shared memory (float4 copies).
+// z rows of the CTA's live chains into shared memory.
 template <int CPB>
-__device__ __forceinline__ void stage_z(const PassArgs &a, int p0, const int *live, float *sm, size_t per) {
-    const int q4 = (int)(a.ldz >> 2);
-    for (int i0 = 0; i0 < q4; i0 += 2 * kPassThreads) {
-        float4 v[CPB][2];
+__device__ __forceinline__ void stage_z(const PassArgs &a, int p0, const int *live, float *zs) {
+    for (int i0 = threadIdx.x; i0 < (int)a.ldz; i0 += kVecLoads * kPassThreads) {
+        float v[kVecLoads][CPB];
 #pragma unroll
-        for (int c = 0; c < CPB; ++c)
+        for (int u = 0; u < kVecLoads; ++u)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int i = i0 + u * kPassThreads + (int)threadIdx.x;
-                v[c][u] = (live[c] && i < q4)
-                              ? __ldg(reinterpret_cast<const float4 *>(a.Z + (size_t)(p0 + c) * (size_t)a.ldz) + i)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < CPB; ++c) {
+                const int i = i0 + u * kPassThreads;
+                v[u][c] = (live[c] && i < (int)a.ldz) ? __ldg(a.Z + (size_t)(p0 + c) * (size_t)a.ldz + (size_t)i) : 0.0f;
             }
 #pragma unroll
-        for (int c = 0; c < CPB; ++c)
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int i = i0 + u * kPassThreads + (int)threadIdx.x;
-                if (live[c] && i < q4) reinterpret_cast<float4 *>(sm + c * per)[i] = v[c][u];
-            }
+        for (int u = 0; u < kVecLoads; ++u) {
+            const int i = i0 + u * kPassThreads;
+            if (i < (int)a.ldz) store_vec<CPB>(zs + (size_t)i * CPB, v[u]);
+        }
     }
 }
 
@@ -259,8 +289,8 @@ __global__ void __launch_bounds__(kPassThreads, MINB) defer_pass1_kernel(const P
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float redm[2 * CPB][kPassWarps];
     __shared__ int live[CPB];
-    const size_t per = pass1_floats(a.ldz, a.ld);
-    float *const sm = reinterpret_cast<float *>(smem_raw);
+    float *const zs = reinterpret_cast<float *>(smem_raw);   // [row][chain]
+    float *const ds = zs + (size_t)a.ldz * CPB;               // [reaction][chain][hi, lo]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (*a.this_gate == 0ull) return;  // no chain's check fired (the GEMM did not run either)
     if (blockIdx.x == 0 && tid == 0) atomicAdd(a.counters + CNT_GEMMS, 1ull);
@@ -274,7 +304,7 @@ __global__ void __launch_bounds__(kPassThreads, MINB) defer_pass1_kernel(const P
             __syncthreads();
             continue;
         }
-        stage_z<CPB>(a, p0, live, sm, per);
+        stage_z<CPB>(a, p0, live, zs);
         __syncthreads();
         // d = S^T z, one line (column of S) per lane
         for (int g = warp; g < a.cols.groups; g += kPassWarps) {
@@ -291,12 +321,13 @@ __global__ void __launch_bounds__(kPassThreads, MINB) defer_pass1_kernel(const P
 #pragma unroll
                 for (int u = 0; u < kSlots; ++u) {
                     if (t0 + u >= len) break;  // (len is the warp's: a uniform branch)
+                    float z[CPB];
+                    load_vec<CPB>(zs + (size_t)ii[u] * CPB, z);
 #pragma unroll
                     for (int c = 0; c < CPB; ++c) {
-                        const float z = sm[c * per + ii[u]];
                         float ph, pe, s, e;
-                        two_prod(hh[u], z, ph, pe);
-                        if (!EXACT32) pe = fmaf(ll[u], z, pe);
+                        two_prod(hh[u], z[c], ph, pe);
+                        if (!EXACT32) pe = fmaf(ll[u], z[c], pe);
                         two_sum(ah[c], ph, s, e);
                         ah[c] = s;
                         al[c] = __fadd_rn(al[c], __fadd_rn(e, pe));
@@ -304,26 +335,23 @@ __global__ void __launch_bounds__(kPassThreads, MINB) defer_pass1_kernel(const P
                 }
             }
             if (j >= 0) {
+                float hl[2 * CPB];
 #pragma unroll
-                for (int c = 0; c < CPB; ++c) {
-                    float h, l;
-                    fast_two_sum(ah[c], al[c], h, l);
-                    float *dh = sm + c * per + a.ldz;
-                    dh[j] = h;
-                    dh[a.ld + j] = l;
-                }
+                for (int c = 0; c < CPB; ++c) fast_two_sum(ah[c], al[c], hl[2 * c], hl[2 * c + 1]);
+                store_vec<2 * CPB>(ds + (size_t)j * 2 * CPB, hl);
             }
         }
         __syncthreads();
         // d leaves shared memory in reaction order (the lines above run in column-length order)
+        for (int j = tid; j < a.n; j += kPassThreads) {
+            float hl[2 * CPB];
+            load_vec<2 * CPB>(ds + (size_t)j * 2 * CPB, hl);
 #pragma unroll
-        for (int c = 0; c < CPB; ++c) {
-            if (!live[c]) continue;
-            const float *dh = sm + c * per + a.ldz;
-            float *gh = a.dxh + (size_t)(p0 + c) * (size_t)a.ld, *gl = a.dxl + (size_t)(p0 + c) * (size_t)a.ld;
-            for (int j = tid; j < a.n; j += kPassThreads) {
-                gh[j] = dh[j];
-                gl[j] = dh[a.ld + j];
+            for (int c = 0; c < CPB; ++c) {
+                if (!live[c]) continue;
+                const size_t o = (size_t)(p0 + c) * (size_t)a.ld + (size_t)j;
+                a.dxh[o] = hl[2 * c];
+                a.dxl[o] = hl[2 * c + 1];
             }
         }
         // r = r0 - S d, one line (row of S, device order: line q is row q) per lane
@@ -356,10 +384,11 @@ __global__ void __launch_bounds__(kPassThreads, MINB) defer_pass1_kernel(const P
 #pragma unroll
                 for (int u = 0; u < kSlots; ++u) {
                     if (t0 + u >= len) break;
+                    float x[2 * CPB];
+                    load_vec<2 * CPB>(ds + (size_t)ii[u] * 2 * CPB, x);
 #pragma unroll
                     for (int c = 0; c < CPB; ++c) {
-                        const float *dh = sm + c * per + a.ldz;
-                        const float xh = dh[ii[u]], xl = dh[a.ld + ii[u]];
+                        const float xh = x[2 * c], xl = x[2 * c + 1];
                         float ph, pe, s, e;
                         two_prod(hh[u], xh, ph, pe);
                         pe = fmaf(hh[u], xl, pe);
@@ -417,8 +446,8 @@ __global__ void __launch_bounds__(kPassThreads, 2) defer_pass_kernel(const PassA
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float redm[CPB][kPassWarps];
     __shared__ int live[CPB];
-    const size_t per = pass_floats(a.ldz, a.ld);
-    float *const sm = reinterpret_cast<float *>(smem_raw);
+    float *const zs = reinterpret_cast<float *>(smem_raw);   // [row][chain]
+    float *const ds = zs + (size_t)a.ldz * CPB;               // [reaction][chain]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (*a.this_gate == 0ull) return;  // no chain needed this pass (its GEMM did not run either)
     if (blockIdx.x == 0 && tid == 0) atomicAdd(a.counters + CNT_GEMMS, 1ull);
@@ -432,7 +461,7 @@ __global__ void __launch_bounds__(kPassThreads, 2) defer_pass_kernel(const PassA
             __syncthreads();
             continue;
         }
-        stage_z<CPB>(a, p0, live, sm, per);
+        stage_z<CPB>(a, p0, live, zs);
         __syncthreads();
         for (int g = warp; g < a.cols.groups; g += kPassWarps) {
             const int base = __ldg(a.cols.off + g);
@@ -448,14 +477,13 @@ __global__ void __launch_bounds__(kPassThreads, 2) defer_pass_kernel(const PassA
 #pragma unroll
                 for (int u = 0; u < kSlots; ++u) {
                     if (t0 + u >= len) break;
+                    float z[CPB];
+                    load_vec<CPB>(zs + (size_t)ii[u] * CPB, z);
 #pragma unroll
-                    for (int c = 0; c < CPB; ++c) d[c] = fmaf(hh[u], sm[c * per + ii[u]], d[c]);
+                    for (int c = 0; c < CPB; ++c) d[c] = fmaf(hh[u], z[c], d[c]);
                 }
             }
-            if (j >= 0) {
-#pragma unroll
-                for (int c = 0; c < CPB; ++c) sm[c * per + a.ldz + j] = d[c];
-            }
+            if (j >= 0) store_vec<CPB>(ds + (size_t)j * CPB, d);
         }
         __syncthreads();
         // dx += d in reaction order (the lines above run in column-length order)
@@ -472,17 +500,21 @@ __global__ void __launch_bounds__(kPassThreads, 2) defer_pass_kernel(const PassA
                     l[c][u] = on ? a.dxl[o] : 0.0f;
                 }
 #pragma unroll
-            for (int c = 0; c < CPB; ++c)
+            for (int u = 0; u < 2; ++u) {
+                const int j = j0 + u * kPassThreads + tid;
+                if (j >= a.n) continue;
+                float d[CPB];
+                load_vec<CPB>(ds + (size_t)j * CPB, d);
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int j = j0 + u * kPassThreads + tid;
-                    if (!(live[c] && j < a.n)) continue;
+                for (int c = 0; c < CPB; ++c) {
+                    if (!live[c]) continue;
                     const size_t o = (size_t)(p0 + c) * (size_t)a.ld + (size_t)j;
                     float s, e;
-                    two_sum(h[c][u], sm[c * per + a.ldz + j], s, e);
+                    two_sum(h[c][u], d[c], s, e);
                     a.dxh[o] = s;
                     a.dxl[o] = __fadd_rn(l[c][u], e);
                 }
+            }
         }
         float mx[CPB];
 #pragma unroll
@@ -505,8 +537,10 @@ __global__ void __launch_bounds__(kPassThreads, 2) defer_pass_kernel(const PassA
 #pragma unroll
                 for (int u = 0; u < kSlots; ++u) {
                     if (t0 + u >= len) break;
+                    float x[CPB];
+                    load_vec<CPB>(ds + (size_t)ii[u] * CPB, x);
 #pragma unroll
-                    for (int c = 0; c < CPB; ++c) acc[c] = fmaf(hh[u], sm[c * per + a.ldz + ii[u]], acc[c]);
+                    for (int c = 0; c < CPB; ++c) acc[c] = fmaf(hh[u], x[c], acc[c]);
                 }
             }
             if (i >= 0) {

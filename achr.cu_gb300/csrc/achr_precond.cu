@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "achr_ctx.h"
+#include "achr_float.cuh"
 #include "achr_pool.h"
 #include "achr_rng.cuh"
 #include "achr_sgemm.cuh"
@@ -247,24 +248,36 @@ __global__ void split_nt_kernel(int n, int d, int kpad, const double *__restrict
 }
 
 // (x - mu) for 32 chains x 64 reactions per warp, transposed through shared
-// memory into chain-major BF16 hi/lo rows (K = reaction contiguous).
-constexpr int kSplitWarps = 4, kSplitStride = 72;
+// memory into chain-major BF16 hi/lo rows (K = reaction contiguous).  One FP64
+// operation per value (x - mu); with the split's conversions there as well the
+// kernel was bound by that pipe (2766 x 3742, 16,384 chains: 0.64 ms, now 0.17,
+// of which the bytes take 0.11).  Eight values of a warp's column are in flight.
+constexpr int kSplitWarps = 4, kSplitStride = 72, kSplitLoads = 8;
 __global__ void __launch_bounds__(kSplitWarps * 32)
     split_points_kernel(int n, int kpad, int P, const double *__restrict__ X, long long ldx,
                         const double *__restrict__ mu, __nv_bfloat16 *__restrict__ Xh, __nv_bfloat16 *__restrict__ Xl) {
-    __shared__ __align__(16) __nv_bfloat16 stage[kSplitWarps][2][32 * kSplitStride];
+    __shared__ __align__(16) unsigned short stage[kSplitWarps][2][32 * kSplitStride];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p0 = blockIdx.x * 32, p = p0 + lane;
-    const bool live = p < P;
+    const double *xp = X + (p < P ? p : P - 1);
     const int nchunks = kpad / 64;
     for (int c = blockIdx.y * kSplitWarps + warp; c < nchunks; c += gridDim.y * kSplitWarps) {
-        for (int r = 0; r < 64; ++r) {
-            const int i = c * 64 + r;
-            double v = 0.0;
-            if (live && i < n) v = X[(long long)i * ldx + p] - (mu ? mu[i] : 0.0);
-            const __nv_bfloat16 hi = __double2bfloat16(v);
-            stage[warp][0][lane * kSplitStride + r] = hi;
-            stage[warp][1][lane * kSplitStride + r] = __double2bfloat16(v - (double)__bfloat162float(hi));
+        for (int r = 0; r < 64; r += kSplitLoads) {
+            double x[kSplitLoads], m[kSplitLoads];
+#pragma unroll
+            for (int u = 0; u < kSplitLoads; ++u) {
+                const int i = c * 64 + r + u, ii = min(i, n - 1);
+                x[u] = __ldg(xp + (long long)ii * ldx);
+                m[u] = mu ? __ldg(mu + ii) : 0.0;
+                if (i >= n) x[u] = m[u] = 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kSplitLoads; ++u) {
+                unsigned short h, l;
+                split_bf16_bits(f64_to_f32_near(mu ? x[u] - m[u] : x[u]), h, l);
+                stage[warp][0][lane * kSplitStride + r + u] = h;
+                stage[warp][1][lane * kSplitStride + r + u] = l;
+            }
         }
         __syncwarp();
         for (int t = lane; t < 32 * 8; t += 32) {
@@ -711,29 +724,39 @@ achr_status achr_null_coords(achr_ctx *ctx, int32_t n_points, const double *d_po
     if (n_points == 0 || ctx->d_act == 0) return ACHR_OK;
     const int n = ctx->n, d = ctx->d_act, kpad = (n + 63) / 64 * 64;
     cudaStream_t st = (cudaStream_t)stream;
-    DevBuf<__nv_bfloat16> Nh, Nl, Xh, Xl;
-    DevBuf<unsigned long long> err;
-    PC_TRY(Nh.alloc((size_t)d * kpad));
-    PC_TRY(Nl.alloc((size_t)d * kpad));
-    PC_TRY(err.alloc(1));
-    PC_TRY(cudaMemsetAsync(err.p, 0, sizeof(unsigned long long), st));
-    split_nt_kernel<<<blocks_for((long long)d * kpad), 256, 0, st>>>(n, d, kpad, ctx->Nact.p, Nh.p, Nl.p);
-    PC_TRY(cudaGetLastError());
-    const int chunk = std::min(n_points, 65536);
-    PC_TRY(Xh.alloc((size_t)chunk * kpad));
-    PC_TRY(Xl.alloc((size_t)chunk * kpad));
+    // The basis split for the tensor cores, laid out once per context.
+    if (!ctx->NactL.p) {
+        const size_t cnt = (size_t)d * (size_t)kpad;
+        PC_TRY(ctx->NactH.alloc(cnt));
+        DevBuf<__nv_bfloat16> lo;
+        PC_TRY(lo.alloc(cnt));
+        split_nt_kernel<<<blocks_for((long long)cnt), 256, 0, st>>>(n, d, kpad, ctx->Nact.p, ctx->NactH.p, lo.p);
+        PC_TRY(cudaGetLastError());
+        PC_TRY(cudaStreamSynchronize(st));  // later calls may come on other streams
+        std::swap(ctx->NactL.p, lo.p);
+        std::swap(ctx->NactL.count, lo.count);
+    }
+    // A workspace for one block of chains (124 MB at 3742 reactions) from the pool.
+    const int chunk = std::min(n_points, 8192);
+    const size_t xcnt = (size_t)chunk * (size_t)kpad;
+    PoolBuf buf(st);
+    PC_TRY(buf.alloc(256 + 2 * xcnt * sizeof(__nv_bfloat16)));
+    unsigned long long *err = reinterpret_cast<unsigned long long *>(buf.p);
+    __nv_bfloat16 *Xh = reinterpret_cast<__nv_bfloat16 *>(buf.p + 256), *Xl = Xh + xcnt;
+    PC_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned long long), st));
     for (int c0 = 0; c0 < n_points; c0 += chunk) {
         const int pc = std::min(chunk, n_points - c0);
         const int nchunks = kpad / 64;
         dim3 grid((unsigned)((pc + 31) / 32), (unsigned)((nchunks + kSplitWarps - 1) / kSplitWarps));
-        split_points_kernel<<<grid, kSplitWarps * 32, 0, st>>>(n, kpad, pc, d_points + c0, ld, d_mu, Xh.p, Xl.p);
+        split_points_kernel<<<grid, kSplitWarps * 32, 0, st>>>(n, kpad, pc, d_points + c0, ld, d_mu, Xh, Xl);
         PC_TRY(cudaGetLastError());
-        TcGemm g{d, pc, kpad, 3, Nh.p, Nl.p, (long long)kpad, Xh.p, Xl.p, (long long)kpad, d_Y + c0, (long long)ldy};
+        TcGemm g{d, pc, kpad, 3, ctx->NactH.p, ctx->NactL.p, (long long)kpad, Xh, Xl, (long long)kpad, d_Y + c0,
+                 (long long)ldy};
         if (const char *why = tc_gemm_check(g)) return pc_err(ACHR_ERR_INVALID, why);
-        PC_TRY(launch_tc_gemm(g, err.p, st));
+        PC_TRY(launch_tc_gemm(g, err, st));
     }
     unsigned long long h = 0;
-    PC_TRY(cudaMemcpyAsync(&h, err.p, sizeof h, cudaMemcpyDeviceToHost, st));
+    PC_TRY(cudaMemcpyAsync(&h, err, sizeof h, cudaMemcpyDeviceToHost, st));
     PC_TRY(cudaStreamSynchronize(st));
     if (h) return pc_err(ACHR_ERR_TIMEOUT, "a tensor-core pipeline wait expired");
     return ACHR_OK;

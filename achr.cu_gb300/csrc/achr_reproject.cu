@@ -37,6 +37,7 @@
 
 #include "achr_ctx.h"
 #include "achr_float.cuh"
+#include "achr_pool.h"
 
 extern "C" void achr_io_set_error(const char *msg);
 
@@ -479,12 +480,13 @@ achr_status achr_gemm_bf16(int32_t M, int32_t N, int32_t K, int32_t nsplit, cons
                            void *stream) {
     achr::TcGemm g{M, N, K, nsplit, A0, A1, (long long)lda, B0, B1, (long long)ldb, C, (long long)ldc};
     if (const char *why = achr::tc_gemm_check(g)) return achr::set_err(ACHR_ERR_INVALID, why);
-    achr::DevBuf<unsigned long long> err;
-    REPROJ_TRY(err.alloc(1));
-    REPROJ_TRY(cudaMemsetAsync(err.p, 0, sizeof(unsigned long long), (cudaStream_t)stream));
-    REPROJ_TRY(achr::launch_tc_gemm(g, err.p, (cudaStream_t)stream));
+    achr::PoolBuf buf((cudaStream_t)stream);
+    REPROJ_TRY(buf.alloc(sizeof(unsigned long long)));
+    unsigned long long *err = reinterpret_cast<unsigned long long *>(buf.p);
+    REPROJ_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned long long), (cudaStream_t)stream));
+    REPROJ_TRY(achr::launch_tc_gemm(g, err, (cudaStream_t)stream));
     unsigned long long h = 0;
-    REPROJ_TRY(cudaMemcpyAsync(&h, err.p, sizeof h, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    REPROJ_TRY(cudaMemcpyAsync(&h, err, sizeof h, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     REPROJ_TRY(cudaStreamSynchronize((cudaStream_t)stream));
     if (h) return achr::set_err(ACHR_ERR_TIMEOUT, "a tensor-core pipeline wait expired");
     return ACHR_OK;
