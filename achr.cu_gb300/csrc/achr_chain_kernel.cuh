@@ -445,6 +445,48 @@ __device__ __forceinline__ unsigned long long residual_rows(const ChainArgs &a, 
     return mx;
 }
 
+// ys = N^T x (reference reprojectPoint, ACHRCuda.cu:208-218), eight columns of N
+// per warp at a time: their loads are in flight together, and their sums over
+// the lanes are formed together, each step halving the columns a lane carries
+// (nine FP64 additions for eight columns; one column at a time they were 40,
+// which at 95 reactions and 24 columns was 120 of a reprojection's 264 FP64
+// instructions).
+template <int BD>
+__device__ __forceinline__ void null_coordinates(const ChainArgs &a, const double *xs, double *ys, int tid) {
+    constexpr int NW = BD / 32;
+    const int lane = tid & 31, warp = tid >> 5, n = a.n;
+#pragma unroll 1
+    for (int j0 = 8 * warp; j0 < a.d; j0 += 8 * NW) {
+        const double *Nj = a.N + (size_t)j0 * (size_t)n;
+        const int cols = min(8, a.d - j0);
+        double acc[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] = 0.0;
+        for (int i = lane; i < n; i += 32) {
+            const double x = xs[i];
+            double v[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = __ldg(Nj + (size_t)min(c, cols - 1) * (size_t)n + i);
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (c < cols) acc[c] = fma(v[c], x, acc[c]);  // (uniform)
+        }
+#pragma unroll
+        for (int half = 4, o = 16; half; half >>= 1, o >>= 1) {
+            const bool upper = lane & o;  // carries the upper half of the columns on
+#pragma unroll
+            for (int c = 0; c < half; ++c) {
+                const double keep = upper ? acc[c + half] : acc[c], send = upper ? acc[c] : acc[c + half];
+                acc[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+        const int c = ((lane & 16) ? 4 : 0) + ((lane & 8) ? 2 : 0) + ((lane & 4) ? 1 : 0);
+        if (!(lane & 3) && c < cols) ys[j0 + c] = acc[0];
+    }
+}
+
 // x <- x - S^T z, z = (S S^T)^+ S x: the reference's N (N^T x) written through
 // the residual (equal in exact arithmetic).  S x is summed in FP64 over the
 // same rows as the check and kept as FP32 hi + lo pairs in rr (m entries
@@ -1214,14 +1256,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             residual_form_reproject<BD>(a, xs, reinterpret_cast<float2 *>(As), zs, tid);
                         } else {
                             const int n = a.n;
-                            for (int j = warp; j < a.d; j += NW) {
-                                const double *Nj = a.N + (size_t)j * (size_t)n;
-                                double acc = 0.0;
-                                for (int i = lane; i < n; i += 32) acc = fma(__ldg(Nj + i), xs[i], acc);
-#pragma unroll
-                                for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                                if (lane == 0) ys[j] = acc;
-                            }
+                            null_coordinates<BD>(a, xs, ys, tid);
                             cta_sync<BD>();
                             for (int i = tid; i < n; i += BD) {
                                 double acc = 0.0;
@@ -1332,14 +1367,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
 #pragma unroll
                 for (int k = 0; k < EPT; ++k) dreg[k] = As[tid + k * BD];
                 cta_sync<BD>();
-                for (int j = warp; j < a.d; j += NW) {
-                    const double *Nj = a.N + (size_t)j * (size_t)n;
-                    double acc = 0.0;
-                    for (int i = lane; i < n; i += 32) acc = fma(__ldg(Nj + i), xs[i], acc);
-#pragma unroll
-                    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                    if (lane == 0) ys[j] = acc;
-                }
+                null_coordinates<BD>(a, xs, ys, tid);
                 cta_sync<BD>();
                 for (int i = tid; i < n; i += BD) {
                     double acc = 0.0;
