@@ -477,7 +477,8 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     // Per-reaction arrays are padded to the kernel's block size x elements per
     // thread; padding entries are fixed at 0 (lb = ub = 0) and never move.
     const int np_cfg = achr::chain_padded_length(n, opt.threads_per_chain);
-    if (np_cfg == 0) return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for n_rxns with this threads_per_chain");
+    if (np_cfg == 0 || !achr::chain_takes_threads(n, opt.threads_per_chain))
+        return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for n_rxns with this threads_per_chain");
     const int np = std::max(np_cfg, achr::chain_alloc_length(n));  // room for every autotuning candidate
     ctx->np = np;
     // Padding reactions have lb = ub = 0 in FP64 and the FP32 box (-1, 1), so
@@ -1008,7 +1009,7 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
         if (!c || n_points[k] < 0 || (n_points[k] > 0 && (!d_points_out[k] || ld_out[k] < n_points[k])))
             return fail(ACHR_ERR_INVALID, "bad batch entry " + std::to_string(k));
         int bd = 0, ept = 0;
-        if (!achr::chain_config(c->n, c->opt.threads_per_chain, &bd, &ept) || bd * ept > c->np)
+        if (!achr::chain_config(c->n, c->opt.threads_per_chain, std::max(c->m, c->d), &bd, &ept) || bd * ept > c->np)
             return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for batch entry " + std::to_string(k));
         cfg_key[(size_t)k] = bd * 100 + ept;
         // disjoint chain ids: model k uses ids off .. off + P_k - 1

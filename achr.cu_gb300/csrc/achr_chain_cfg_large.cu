@@ -12,6 +12,7 @@ cudaError_t launch_chain_cfg_large(int bd, int ept, const ChainArgs &a, cudaStre
         case 256 * 100 + 20: return launch_cfg<256, 20>(a, s, max_ctas, per_sm);
         case 256 * 100 + 24: return launch_cfg<256, 24>(a, s, max_ctas, per_sm);
         case 256 * 100 + 26: return launch_cfg<256, 26>(a, s, max_ctas, per_sm);
+        case 256 * 100 + 30: return launch_cfg<256, 30>(a, s, max_ctas, per_sm);
         case 320 * 100 + 12: return launch_cfg<320, 12>(a, s, max_ctas, per_sm);
         case 384 * 100 + 10: return launch_cfg<384, 10>(a, s, max_ctas, per_sm);
         case 384 * 100 + 20: return launch_cfg<384, 20>(a, s, max_ctas, per_sm);
@@ -33,6 +34,7 @@ cudaError_t launch_chain_queue_large(int bd, int ept, const ChainQueue &q, cudaS
         case 256 * 100 + 20: return launch_queue_cfg<256, 20>(q, s, grid, per_sm);
         case 256 * 100 + 24: return launch_queue_cfg<256, 24>(q, s, grid, per_sm);
         case 256 * 100 + 26: return launch_queue_cfg<256, 26>(q, s, grid, per_sm);
+        case 256 * 100 + 30: return launch_queue_cfg<256, 30>(q, s, grid, per_sm);
         case 320 * 100 + 12: return launch_queue_cfg<320, 12>(q, s, grid, per_sm);
         case 384 * 100 + 10: return launch_queue_cfg<384, 10>(q, s, grid, per_sm);
         case 384 * 100 + 20: return launch_queue_cfg<384, 20>(q, s, grid, per_sm);

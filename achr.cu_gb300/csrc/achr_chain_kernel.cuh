@@ -595,7 +595,7 @@ __device__ __forceinline__ void evaluate(const ChainArgs &a, RatioTest &t, doubl
 
 constexpr int kTbl = 64;  // steps per refill of the step table
 
-// Shared memory of one CTA: xs, As (NP doubles each; a reprojection parks the
+// Shared memory of one CTA: xs, As (NP doubles each, see chain_kept_pairs; a reprojection parks the
 // accumulator in registers and uses As as its scratch), the step table, two
 // reduction slots, then eight statistics counters, the exact-evaluation count
 // (two ints), the `never` barrier and the two worst-case words.
@@ -603,9 +603,23 @@ template <int BD>
 __host__ __device__ constexpr size_t chain_tail_bytes() {
     return sizeof(StepEntry) * kTbl + 2 * sizeof(RedSlots<BD / 32>) + 128;
 }
+// Pairs of the accumulator a thread keeps in registers instead, the last ones:
+// where two vectors in shared memory are just too long for two chains per SM
+// (256 x 30), three pairs less make room for the second (7440 reactions, SM
+// clocks per chain-step: 23090; one chain per SM, 384 x 20: 26500).
+template <int BD, int EPT>
+__host__ __device__ constexpr int chain_kept_pairs() {
+    return BD == 256 && EPT == 30 ? 3 : 0;
+}
+// Doubles of the accumulator in shared memory: also the reprojection's scratch,
+// which holds the d null-space coordinates or the m residuals.
+template <int BD, int EPT>
+__host__ __device__ constexpr int chain_acc_doubles() {
+    return BD * (EPT - 2 * chain_kept_pairs<BD, EPT>());
+}
 template <int BD, int EPT>
 __host__ __device__ constexpr size_t chain_smem_bytes_cfg() {
-    return sizeof(double) * 2 * (size_t)(BD * EPT) + chain_tail_bytes<BD>();
+    return sizeof(double) * (size_t)(BD * EPT + chain_acc_doubles<BD, EPT>()) + chain_tail_bytes<BD>();
 }
 
 // Resident CTAs per SM a configuration is compiled for, with `regs` registers
@@ -635,8 +649,7 @@ constexpr int chain_min_ctas() {
 
 template <int BD, int EPT>
 __device__ __forceinline__ uint64_t *chain_never(unsigned char *smem_raw) {
-    return reinterpret_cast<uint64_t *>(smem_raw + sizeof(double) * 2 * (size_t)(BD * EPT) + sizeof(StepEntry) * kTbl +
-                                        2 * sizeof(RedSlots<BD / 32>) + 72);
+    return reinterpret_cast<uint64_t *>(smem_raw + chain_smem_bytes_cfg<BD, EPT>() - 128 + 72);
 }
 
 // Entries e = tid, tid + BD, ... < kTbl of the step table for steps s + e below
@@ -679,6 +692,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     static_assert(EPT % 2 == 0, "threads own pairs of reactions");
     constexpr int NP = BD * EPT, KP = EPT / 2;
     constexpr int NW = BD / 32;
+    constexpr int KA = KP - chain_kept_pairs<BD, EPT>();  // pairs of the accumulator in shared memory
     constexpr bool KX = chain_keeps_x32<BD, EPT>();
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -686,7 +700,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     double *As = xs + NP;
     double2 *xs2 = reinterpret_cast<double2 *>(xs), *As2 = reinterpret_cast<double2 *>(As);
     double *ys = As;  // reprojection scratch (the accumulator waits in registers)
-    StepEntry *tbl = reinterpret_cast<StepEntry *>(As + NP);
+    StepEntry *tbl = reinterpret_cast<StepEntry *>(As + chain_acc_doubles<BD, EPT>());
     RedSlots<NW> *rsb = reinterpret_cast<RedSlots<NW> *>(tbl + kTbl);
     unsigned long long *cnt = reinterpret_cast<unsigned long long *>(rsb + 2);  // CTA statistics, CNT_* slots
     int *exact_count = reinterpret_cast<int *>(cnt + 8);
@@ -714,6 +728,27 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     // operations on it would change nothing.
     const bool tail_live = warp * 32 + (KP - 1) * BD < npair;
 #define ACHR_PAD_SLOT(k) ((k) == KP - 1 && !tail_live)
+// Pair k of the accumulator (k a constant of an unrolled loop).
+#define ACHR_ACC_GET(k) ((k) < KA ? As2[tid + (k) * BD] : make_double2(at[(k) < KA ? 0 : 2 * ((k) - KA)], at[(k) < KA ? 0 : 2 * ((k) - KA) + 1]))
+#define ACHR_ACC_SET(k, v)                              \
+    do {                                                \
+        if ((k) < KA) {                                 \
+            As2[tid + (k) * BD] = (v);                  \
+        } else {                                        \
+            at[(k) < KA ? 0 : 2 * ((k) - KA)] = (v).x;     \
+            at[(k) < KA ? 0 : 2 * ((k) - KA) + 1] = (v).y; \
+        }                                               \
+    } while (0)
+// Adds v to coordinate i, the thread's k-th of the accumulator (k not a constant).
+#define ACHR_ACC_ADD(k, i, v)                                               \
+    do {                                                                    \
+        if (KA == KP || (k) < 2 * KA) {                                     \
+            As[i] += (v);                                                   \
+        } else {                                                            \
+            _Pragma("unroll") for (int t_ = 0; t_ < 2 * (KP - KA); ++t_)    \
+                if ((k) - 2 * KA == t_) at[t_] += (v);                      \
+        }                                                                   \
+    } while (0)
     const float e0 = (kTiny + a.bound_err + a.dtol_hi) * 1.01f;
     const float4 *bnd2 = reinterpret_cast<const float4 *>(a.bnd);  // (lb, ub, lb, ub) of a pair
     unsigned it = 0;
@@ -729,29 +764,36 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
 #define ACHR_CHAIN_ID (a.chain_offset + (unsigned long long)p)
         // Segmented sampling: the chain's state bits from the earlier launches.
         const unsigned sflags = SEG ? a.seg_flags[p] : 0u;
+        double at[KA < KP ? 2 * (KP - KA) : 1];  // the accumulator's last pairs (KA < KP)
+        // Point and accumulator: of an earlier launch, of the chain's state after
+        // step0 steps (resume), or the centre and its sum.
+        const double *x_src = a.c0, *A_src = a.A0;
+        long long stride = 1;
+        int stored = NP;
         if (sflags & SEG_STARTED) {
+            x_src = a.seg_x + (size_t)p * (size_t)a.ld_seg;
+            A_src = a.seg_A + (size_t)p * (size_t)a.ld_seg;
+            stored = a.n;
+        } else if (a.x_in) {
+            x_src = a.x_in + p;
+            A_src = a.A_in + p;
+            stride = a.ld_state;
+            stored = a.n;
+        }
 #pragma unroll
-            for (int k = 0; k < EPT; ++k) {
-                const int i = tid + k * BD;
-                const bool real = i < a.n;
-                xs[i] = real ? a.seg_x[(size_t)p * (size_t)a.ld_seg + (size_t)i] : 0.0;
-                As[i] = real ? a.seg_A[(size_t)p * (size_t)a.ld_seg + (size_t)i] : 0.0;
+        for (int k = 0; k < KP; ++k) {
+            const int i = 2 * (tid + k * BD);
+            double2 x2 = make_double2(0.0, 0.0), A2 = x2;
+            if (i < stored) {
+                x2.x = x_src[(long long)i * stride];
+                A2.x = A_src[(long long)i * stride];
             }
-        } else if (a.x_in) {  // resume: the chain's point and centre accumulator after step0 steps
-#pragma unroll
-            for (int k = 0; k < EPT; ++k) {
-                const int i = tid + k * BD;
-                const bool real = i < a.n;
-                xs[i] = real ? a.x_in[(size_t)i * (size_t)a.ld_state + (size_t)p] : 0.0;
-                As[i] = real ? a.A_in[(size_t)i * (size_t)a.ld_state + (size_t)p] : 0.0;
+            if (i + 1 < stored) {
+                x2.y = x_src[(long long)(i + 1) * stride];
+                A2.y = A_src[(long long)(i + 1) * stride];
             }
-        } else {
-#pragma unroll
-            for (int k = 0; k < EPT; ++k) {
-                const int i = tid + k * BD;
-                xs[i] = a.c0[i];
-                As[i] = a.A0[i];
-            }
+            xs2[tid + k * BD] = x2;
+            ACHR_ACC_SET(k, A2);
         }
         int buf_col = -1;  // the warmup column dreg holds (-1: none)
         bool any_accepted = a.x_in != nullptr || (sflags & SEG_ACCEPTED), stuck = false;
@@ -762,6 +804,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
             // The batched passes' correction of this chain, x <- x - S^T z summed over
             // the passes, held as a double-float pair: two FP64 subtractions per
             // reaction (the FP32 -> FP64 conversions are integer operations).
+            cta_sync<BD>();  // this loop is per element, the others per pair
 #pragma unroll
             for (int k = 0; k < EPT; ++k) {
                 const int i = tid + k * BD;
@@ -771,7 +814,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 }
             }
         }
-        cta_sync<BD>();  // the loops above are per element, the step's per pair
+        cta_sync<BD>();
         double dreg[EPT];  // the next step's column, then the step's direction
         float xf[KX ? EPT : 2];  // FP32 image of the point (KX; else formed where it is used)
         if (sflags & SEG_PENDING) {
@@ -786,7 +829,10 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 const double xv = xs[i];
                 const float2 b = __ldg(a.bnd + i);
                 if (surely_inside(x_to_f32(xv), b.x, b.y, a.bound_err)) {
-                    if (!hr) As[i] += xv;
+                    if (!hr) {
+                        if ((k >> 1) < KA) As[i] += xv;
+                        else at[(k >> 1) < KA ? 0 : k - 2 * KA] += xv;
+                    }
                 } else {
                     edge |= 1u << k;
                 }
@@ -795,7 +841,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
                 const double xc = clip_exact(xs[i], exact_bounds(a, i));
                 xs[i] = xc;
-                if (!hr) As[i] += xc;
+                if (!hr) ACHR_ACC_ADD(k, i, xc);
             }
         }
 // Pair k of the point's image.
@@ -879,9 +925,14 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                     for (int k = 0; k < KP; ++k) {
                         const int q = tid + k * BD;
                         if (ACHR_PAD_SLOT(k)) continue;  // padding: d stays 0, never a candidate
+                        // Long directions: one pair at a time.  Left to itself the compiler forms many
+                        // pairs together and spills for it (SM clocks per chain-step without and
+                        // with: n = 2500 6935, 6786; 5000 15320, 14672; 6500 19130, 17800; 7440
+                        // 25010, 23090); short ones gain nothing.
+                        if (EPT >= 16) __syncwarp();
                         if (q == odd) dreg[2 * k + 1] = 0.0;
                         if (!hr) {
-                            const double2 A2 = As2[q];
+                            const double2 A2 = ACHR_ACC_GET(k);
                             dreg[2 * k] = fma(A2.x, ninv, dreg[2 * k]);
                             dreg[2 * k + 1] = fma(A2.y, ninv, dreg[2 * k + 1]);
                         }
@@ -1159,10 +1210,10 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             const bool in1 = surely_inside(x1, b.z, b.w, a.bound_err);
                             edge |= (in0 ? 0u : 1u << (2 * k)) | (in1 ? 0u : 2u << (2 * k));
                             if (!hr) {  // hit-and-run: no centre to update
-                                double2 A2 = As2[q];
+                                double2 A2 = ACHR_ACC_GET(k);
                                 if (in0) A2.x += x2.x;
                                 if (in1) A2.y += x2.y;
-                                As2[q] = A2;
+                                ACHR_ACC_SET(k, A2);
                             }
                         }
                         if (pre && q < npair) {
@@ -1177,7 +1228,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
                             const double xc = clip_exact(xs[i], exact_bounds(a, i));
                             xs[i] = xc;
-                            if (!hr) As[i] += xc;
+                            if (!hr) ACHR_ACC_ADD(k, i, xc);
                         }
                         if (KX) {
 #pragma unroll
@@ -1217,11 +1268,17 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             if (*a.seg_any == 0ull) atomicOr(a.seg_any, 1ull);
                         }
 #pragma unroll
-                        for (int k = 0; k < EPT; ++k) {
-                            const int i = tid + k * BD;
+                        for (int k = 0; k < KP; ++k) {
+                            const int i = 2 * (tid + k * BD);
+                            const size_t o = (size_t)p * (size_t)a.ld_seg + (size_t)i;
+                            const double2 A2 = ACHR_ACC_GET(k), x2 = xs2[tid + k * BD];
                             if (i < a.n) {
-                                a.seg_x[(size_t)p * (size_t)a.ld_seg + (size_t)i] = xs[i];
-                                a.seg_A[(size_t)p * (size_t)a.ld_seg + (size_t)i] = As[i];
+                                a.seg_x[o] = x2.x;
+                                a.seg_A[o] = A2.x;
+                            }
+                            if (i + 1 < a.n) {
+                                a.seg_x[o + 1] = x2.y;
+                                a.seg_A[o + 1] = A2.y;
                             }
                         }
                         if (tid == 0) {
@@ -1246,7 +1303,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                         // The scratch is As: the accumulator waits in the direction's registers.
                         if (tid == 0) ++cnt[CNT_REPROJ];
 #pragma unroll
-                        for (int k = 0; k < KP; ++k) {
+                        for (int k = 0; k < KA; ++k) {
                             const double2 A2 = As2[tid + k * BD];
                             dreg[2 * k] = A2.x;
                             dreg[2 * k + 1] = A2.y;
@@ -1267,7 +1324,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                         }
                         cta_sync<BD>();
 #pragma unroll
-                        for (int k = 0; k < KP; ++k)
+                        for (int k = 0; k < KA; ++k)
                             As2[tid + k * BD] = make_double2(dreg[2 * k], dreg[2 * k + 1]);
                     }
                     unsigned edge = 0;
@@ -1286,10 +1343,10 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             const bool in1 = surely_inside(x1, b.z, b.w, a.bound_err);
                             edge |= (in0 ? 0u : 1u << (2 * k)) | (in1 ? 0u : 2u << (2 * k));
                             if (!hr) {
-                                double2 A2 = As2[q];
+                                double2 A2 = ACHR_ACC_GET(k);
                                 if (in0) A2.x += x2.x;
                                 if (in1) A2.y += x2.y;
-                                As2[q] = A2;
+                                ACHR_ACC_SET(k, A2);
                             }
                         }
                         if (pre && q < npair) {
@@ -1306,7 +1363,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                             const int k = __ffs(edge) - 1, i = 2 * (tid + (k >> 1) * BD) + (k & 1);
                             const double xc = clip_exact(xs[i], exact_bounds(a, i));
                             xs[i] = xc;
-                            if (!hr) As[i] += xc;
+                            if (!hr) ACHR_ACC_ADD(k, i, xc);
                         }
                         if (KX) {
 #pragma unroll
@@ -1332,11 +1389,17 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
         if (SEG && !seg_pending && !a.seg_final) {
             // A segmented launch that is not the run's last: keep the state for the next one.
 #pragma unroll
-            for (int k = 0; k < EPT; ++k) {
-                const int i = tid + k * BD;
+            for (int k = 0; k < KP; ++k) {
+                const int i = 2 * (tid + k * BD);
+                const size_t o = (size_t)p * (size_t)a.ld_seg + (size_t)i;
+                const double2 A2 = ACHR_ACC_GET(k), x2 = xs2[tid + k * BD];
                 if (i < a.n) {
-                    a.seg_x[(size_t)p * (size_t)a.ld_seg + (size_t)i] = xs[i];
-                    a.seg_A[(size_t)p * (size_t)a.ld_seg + (size_t)i] = As[i];
+                    a.seg_x[o] = x2.x;
+                    a.seg_A[o] = A2.x;
+                }
+                if (i + 1 < a.n) {
+                    a.seg_x[o + 1] = x2.y;
+                    a.seg_A[o + 1] = A2.y;
                 }
             }
             if (tid == 0)
@@ -1365,7 +1428,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 if (pass == 1 || !a.final_project || __longlong_as_double((long long)res) <= a.feasibility_tol) break;
                 if (tid == 0) ++cnt[CNT_FINAL_PROJ];
 #pragma unroll
-                for (int k = 0; k < EPT; ++k) dreg[k] = As[tid + k * BD];
+                for (int k = 0; k < 2 * KA; ++k) dreg[k] = As[tid + k * BD];
                 cta_sync<BD>();
                 null_coordinates<BD>(a, xs, ys, tid);
                 cta_sync<BD>();
@@ -1376,7 +1439,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                 }
                 cta_sync<BD>();
 #pragma unroll
-                for (int k = 0; k < EPT; ++k) As[tid + k * BD] = dreg[k];
+                for (int k = 0; k < 2 * KA; ++k) As[tid + k * BD] = dreg[k];
             }
             double viol = 0.0;
             for (int i = tid; i < n; i += BD) {
@@ -1398,12 +1461,22 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
             }
         }
         for (int i = tid; i < a.n; i += BD) a.out[(size_t)i * (size_t)a.ld_out + (size_t)p] = any_accepted ? xs[i] : 0.0;
-        if (a.A_out)
-            for (int i = tid; i < a.n; i += BD) a.A_out[(size_t)i * (size_t)a.ld_state + (size_t)p] = As[i];
+        if (a.A_out) {
+#pragma unroll
+            for (int k = 0; k < KP; ++k) {
+                const int i = 2 * (tid + k * BD);
+                const double2 A2 = ACHR_ACC_GET(k);
+                if (i < a.n) a.A_out[(size_t)i * (size_t)a.ld_state + (size_t)p] = A2.x;
+                if (i + 1 < a.n) a.A_out[(size_t)(i + 1) * (size_t)a.ld_state + (size_t)p] = A2.y;
+            }
+        }
         cta_sync<BD>();
     }
 #undef ACHR_CHAIN_ID
 #undef ACHR_PAD_SLOT
+#undef ACHR_ACC_GET
+#undef ACHR_ACC_SET
+#undef ACHR_ACC_ADD
 #undef ACHR_X32
 
     cta_sync<BD>();
@@ -1487,7 +1560,7 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
     // the residual in the accumulator's place; it is used only when z fits
     // without costing a resident CTA per SM.
     const size_t zbytes = ((size_t)a.m * sizeof(float) + 15) & ~(size_t)15;
-    // (its residual takes the accumulator's NP doubles while that waits in registers: m <= ldw <= NP)
+    // (its residual takes the accumulator's place while that waits in registers: m <= ldw <= NP)
     if (a.pinv32 && a.m > a.ldw) a.pinv32 = nullptr;
     size_t smem = base + (a.pinv32 ? zbytes : 0);
     cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -28,22 +28,27 @@ struct Cfg {
 // reductions) where shared memory still holds four chains or more, and more
 // warps where it holds two.  Measured, SM clocks per chain-step at full
 // residency (the previous kernel's in brackets): n = 95, 32 x 4: 400 [689];
-// n = 1060, 64 x 20: 3550 [7760], 256 x 8: 4920; n = 2500, 128 x 20: 6900,
+// n = 1060, 64 x 20: 3550 [7760], 256 x 8: 4920; n = 2500, 128 x 20: 6790,
 // 320 x 12: 8680; n = 3000, 128 x 24: 8690, 320 x 12: 9080; n = 3742, 320 x 12:
-// 10190 [13960 with 384 x 10], 384 x 10: 10350, 256 x 16: 10940; n = 7440, 384 x
-// 20: 26500 [31020 with 512 x 15], 512 x 16: 26600.  The others serve an explicit
+// 10190 [13960 with 384 x 10], 384 x 10: 10350, 256 x 16: 10940; n = 7440, 256 x
+// 30: 23090, 384 x 20: 26500 [31020 with 512 x 15], 512 x 16: 26600.  The others serve an explicit
 // threads_per_chain and the autotuner.
 const Cfg kLadder[] = {
     {32, 4, true},    {64, 4, false},   {32, 8, true},    {64, 6, true},    {128, 4, false},  {64, 8, true},
     {64, 12, true},   {64, 16, true},   {128, 8, false},  {256, 4, false},  {64, 20, true},   {128, 12, true},
     {128, 16, true},  {256, 8, false},  {512, 4, false},  {128, 20, true},  {128, 24, true},  {320, 12, true},
     {384, 10, false}, {256, 16, true},  {512, 8, false},  {128, 32, false}, {256, 18, true},  {256, 20, true},
-    {256, 24, true},  {512, 12, false}, {256, 26, true},  {384, 20, true},  {512, 16, true},  {512, 32, true},
+    {256, 24, true},  {512, 12, false}, {256, 26, true},  {256, 30, true},  {384, 20, true},  {512, 16, true},  {512, 32, true},
 };
 
-const Cfg *find_cfg(int n, int threads_per_chain) {
+// 256 x 30 keeps 6 x 256 of the accumulator's doubles in registers, and the rest
+// is too little scratch for a reprojection onto more than 6144 coordinates.
+constexpr int kScratch256x30 = 256 * (30 - 6);
+
+const Cfg *find_cfg(int n, int threads_per_chain, int scratch = 0) {
     for (const Cfg &c : kLadder) {
         if (c.bd * c.ept < n) continue;
+        if (c.bd == 256 && c.ept == 30 && scratch > kScratch256x30) continue;
         if (threads_per_chain == 0 ? c.dflt : c.bd == threads_per_chain) return &c;
     }
     return nullptr;
@@ -81,8 +86,18 @@ int chain_candidates(int n, int max_np, int *bds, int cap) {
     return k;
 }
 
-bool chain_config(int n, int threads_per_chain, int *bd, int *ept) {
-    const Cfg *c = find_cfg(n, threads_per_chain);
+bool chain_takes_threads(int n, int threads_per_chain) {
+    const int most = threads_per_chain == 32    ? 256
+                     : threads_per_chain == 64  ? 512
+                     : threads_per_chain == 320 ? 3840
+                     : threads_per_chain == 384 ? 3840
+                     : threads_per_chain <= 256 ? 4096
+                                                : 16384;
+    return threads_per_chain == 0 || n <= most;
+}
+
+bool chain_config(int n, int threads_per_chain, int scratch, int *bd, int *ept) {
+    const Cfg *c = find_cfg(n, threads_per_chain, scratch);
     if (!c) return false;
     *bd = c->bd;
     *ept = c->ept;
@@ -97,7 +112,7 @@ cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_
 
 cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_t stream, int max_ctas,
                           int *per_sm) {
-    const Cfg *c = find_cfg(a.n, threads_per_chain);
+    const Cfg *c = find_cfg(a.n, threads_per_chain, a.m > a.d ? a.m : a.d);
     if (!c || c->bd * c->ept > a.np) return cudaErrorInvalidValue;
     if (a.P <= 0 && !per_sm) return cudaSuccess;
     if (c->bd <= 64) return launch_chain_cfg_small(c->bd, c->ept, a, stream, max_ctas, per_sm);

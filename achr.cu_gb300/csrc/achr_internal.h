@@ -172,7 +172,11 @@ cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_
 // reactions (threads_per_chain = 0: default); 0 if no configuration fits.
 int chain_block_size(int n, int threads_per_chain);
 // Configuration (threads, elements per thread) the model of n reactions runs with.
-bool chain_config(int n, int threads_per_chain, int *bd, int *ept);
+// for a reprojection scratch of `scratch` doubles (the larger of m and d).
+bool chain_config(int n, int threads_per_chain, int scratch, int *bd, int *ept);
+// Whether a caller may ask for this many threads per chain at n reactions (the
+// defaults and the autotuner also use longer configurations of a thread count).
+bool chain_takes_threads(int n, int threads_per_chain);
 // Persistent work-queue launch of the configuration (bd, ept); see ChainQueue.
 cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_t stream, int grid, int *per_sm);
 int chain_padded_length(int n, int threads_per_chain);

@@ -229,7 +229,8 @@ extern "C" achr_status achr_sample_noalloc(const achr_device_model *m, const ach
                     "achr_sample_noalloc reprojects as N (N^T x) in FP64; the residual and deferred forms "
                     "(reproject_form 2 and 3) need a pseudo-inverse of S S^T and buffers that only a context builds");
     const int np = achr::chain_padded_length(n, opt.threads_per_chain);
-    if (np == 0 || np > kMaxRxns) return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for this size");
+    if (np == 0 || np > kMaxRxns || !achr::chain_takes_threads(n, opt.threads_per_chain))
+        return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for this size");
     const int prep_blocks = (np + kPrepThreads - 1) / kPrepThreads;
 
     int dev = 0, sms = 0;
