@@ -3,7 +3,7 @@
 // A configuration is (threads per chain BD, elements per thread EPT); its
 // padded length BD * EPT must hold the model's n reactions.  For each padded
 // length there is a default configuration (used when threads_per_chain = 0)
-// and alternatives that the autotuner may pick.
+// and alternatives: for launches of few chains, and for the autotuner.
 #include "achr_internal.h"
 
 namespace achr {
@@ -45,6 +45,8 @@ const Cfg kLadder[] = {
 // is too little scratch for a reprojection onto more than 6144 coordinates.
 constexpr int kScratch256x30 = 256 * (30 - 6);
 
+constexpr int kFewWarps = 16;  // warps per SM up to which a launch counts as one of few chains
+
 const Cfg *find_cfg(int n, int threads_per_chain, int scratch = 0) {
     for (const Cfg &c : kLadder) {
         if (c.bd * c.ept < n) continue;
@@ -52,6 +54,28 @@ const Cfg *find_cfg(int n, int threads_per_chain, int scratch = 0) {
         if (threads_per_chain == 0 ? c.dflt : c.bd == threads_per_chain) return &c;
     }
     return nullptr;
+}
+
+// The default for P chains on `sms` SMs.  A launch of few chains per SM is bound
+// by a chain's own latency, which more warps shorten, up to about 16 warps on an
+// SM; after that the FP64 pipe is the bound, where more warps only repeat the
+// reductions.  The results do not depend on it.  Measured, SM clocks per
+// chain-step, default and the one taken, at 1, 2, 4 and 8 chains per SM: n = 95
+// (32 -> 64 threads) 5358 4607, 2707 2321, 1362 1246, 736 739; n = 250 (32 ->
+// 128, from 8 per SM 64) 7839 5367, 3930 2847, 1980 1650, 1107 1060; n = 500 (64
+// -> 256, 256, 128) 8425 5712, 4255 3400, 2378 2094; n = 1060 (64 -> 256, 256,
+// 128) 16027 8972, 8004 5664, 4649 3895.
+const Cfg *find_cfg_for(const ChainArgs &a, int sms) {
+    const int scratch = a.m > a.d ? a.m : a.d;
+    const Cfg *best = find_cfg(a.n, 0, scratch);
+    if (!best) return nullptr;
+    const int per_sm = (a.P + sms - 1) / sms, np0 = best->bd * best->ept;
+    for (int bd : {64, 128, 256, 512}) {
+        const Cfg *c = find_cfg(a.n, bd, scratch);
+        const int np = c ? c->bd * c->ept : 0;
+        if (c && bd > best->bd && np <= a.np && np <= 2 * np0 && (long long)per_sm * (bd / 32) <= kFewWarps) best = c;
+    }
+    return best;
 }
 
 }  // namespace
@@ -113,6 +137,13 @@ cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_
 cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_t stream, int max_ctas,
                           int *per_sm) {
     const Cfg *c = find_cfg(a.n, threads_per_chain, a.m > a.d ? a.m : a.d);
+    if (threads_per_chain == 0 && a.P > 0) {
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        c = find_cfg_for(a, sms);
+    }
     if (!c || c->bd * c->ept > a.np) return cudaErrorInvalidValue;
     if (a.P <= 0 && !per_sm) return cudaSuccess;
     if (c->bd <= 64) return launch_chain_cfg_small(c->bd, c->ept, a, stream, max_ctas, per_sm);
