@@ -302,9 +302,11 @@ cudaError_t gemm(cudaStream_t st, int M, int N, int K, const float *A, long long
 // summed over k in order.  A column at a time in one CTA (a barrier per column,
 // the matrix in L2) this took 4.9 ms at r = 256.  Here the factorisation works
 // on panels of 32 columns in shared memory (in L2 above kCholSmemMax), X is
-// formed by a CTA per 32 columns, and Minv is a product: 0.27 ms.
+// formed by a CTA per 32 columns, and Minv is a product: 0.18 ms (114 + 49 + 13 us).
 constexpr int kNB = 32;
-constexpr int kCholSmemMax = 320;  // rows of the factor that fit shared memory (packed lower triangle)
+constexpr int kCholSmemMax = 304;  // rows of the factor that fit shared memory (packed lower triangle, and a panel)
+constexpr int kNextBlock = (kNB / 4) * (kNB / 4 + 1) / 2;  // 4 x 4 elements of a diagonal block's triangle
+constexpr int kInverseMax = 1024;  // rows the inverse's shared-memory layouts allow
 
 // Element (i, j), j <= i, of the factor while it is formed: packed rows in shared memory, or the r x r
 // matrix in global memory.
@@ -318,82 +320,50 @@ struct LowerDense {
     __device__ __forceinline__ float &at(int i, int j) const { return p[(long long)i * r + j]; }
 };
 
+// The panel's rows below its diagonal block once more, transposed (column k at panel + k * ld): the
+// trailing update then reads four rows with one 16-byte load.  Row by row from the packed triangle
+// it read single words with bank conflicts.  r = 256: 159 us before; 144 with this; 138 with the divisions
+// below as three operations; 114 with the diagonal block's shuffles free of branches.
+__host__ __device__ inline int chol_panel_ld(int r) { return r <= kNB ? 4 : (r - kNB + 3) / 4 * 4; }
+inline size_t chol_panel_bytes(int r) { return sizeof(float) * (size_t)kNB * chol_panel_ld(r); }
+
+// v / d from inv = 1 / d, both rounded to nearest: the quotient's remainder is exact, and one
+// correction rounds it correctly (Markstein, IBM J. Res. Dev. 34, 1990) for a normal quotient.  The
+// divisions below follow one another; this one is three dependent operations and no branch.
+__device__ __forceinline__ float div_by(float v, float d, float inv) {
+    const float q = v * inv;
+    return fmaf(fmaf(-q, d, v), inv, q);
+}
+
+// diag: the diagonal block, transposed; dinv: 1 / its diagonal.
 template <class Low>
-__device__ __forceinline__ void chol_panels(int r, const Low L, int *bad, float (*diag)[kNB + 1]) {
+__device__ __forceinline__ void chol_panels(int r, const Low L, int *bad, float (*diag)[kNB + 4], float *dinv,
+                                            float *panel) {
+    const int ldp = chol_panel_ld(r);
     const int tid = threadIdx.x, nt = blockDim.x;
+    __syncthreads();
     for (int c0 = 0; c0 < r; c0 += kNB) {
+        // Triangle from row c0 on, less the previous panel's part: 4 x 4 elements per thread and turn.
+        // Warp 0 takes the diagonal block (the first 36 of them) and factors it, a chain of 32 square
+        // roots and divisions, while the others update the rest.
         const int nb = min(kNB, r - c0);
-        __syncthreads();
-        if (tid < 32) {  // the diagonal block: lane i holds row i
-            float row[kNB];
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) row[j] = tid < nb && j <= tid ? L.at(c0 + tid, c0 + j) : 0.0f;
-#pragma unroll
-            for (int k = 0; k < kNB; ++k) {
-                float d = __shfl_sync(0xffffffffu, row[k], k);
-                if (k < nb) {
-                    if (!(d > 0.0f)) {
-                        if (tid == 0) *bad = 1;
-                        d = 1.0f;
-                    }
-                    const float piv = sqrtf(d);
-                    row[k] = tid == k ? piv : row[k] / piv;
-                }
-#pragma unroll
-                for (int j = k + 1; j < kNB; ++j) {
-                    const float ljk = __shfl_sync(0xffffffffu, row[k], j);
-                    if (k < nb) row[j] = fmaf(-row[k], ljk, row[j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) {
-                diag[tid][j] = row[j];
-                if (tid < nb && j <= tid) L.at(c0 + tid, c0 + j) = row[j];
-            }
-        }
-        __syncthreads();
-        // rows below: a thread per row, its 32 elements in registers
-        for (int i = c0 + nb + tid; i < r; i += nt) {
-            float v[kNB];
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) v[j] = L.at(i, c0 + j);
-#pragma unroll
-            for (int k = 0; k < kNB; ++k) {
-                asm volatile("" ::: "memory");  // this column's 32 loads only (all 496 would not fit the registers)
-                v[k] = v[k] / diag[k][k];
-#pragma unroll
-                for (int j = k + 1; j < kNB; ++j) v[j] = fmaf(-v[k], diag[j][k], v[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) L.at(i, c0 + j) = v[j];
-        }
-        __syncthreads();
-        // trailing triangle: 4 x 4 elements per thread and turn
-        const int t0 = c0 + nb, nq = (r - t0 + 3) / 4;
-        for (int t = tid; t < nq * (nq + 1) / 2; t += nt) {
+        const int nq = c0 ? (r - c0 + 3) / 4 : 0, all = nq * (nq + 1) / 2, first = min(kNextBlock, all);
+        for (int t = tid < 32 ? tid : first + tid - 32; t < (tid < 32 ? first : all); t += tid < 32 ? 32 : nt - 32) {
             int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
             while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
             while (bi * (bi + 1) / 2 > t) --bi;
-            const int i0 = t0 + 4 * bi, j0 = t0 + 4 * (t - bi * (bi + 1) / 2);
+            const int i0 = c0 + 4 * bi, j0 = c0 + 4 * (t - bi * (bi + 1) / 2);
             float acc[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = i0 + i < r && j0 + j <= i0 + i ? L.at(i0 + i, j0 + j) : 0.0f;
-            const float *pa[4], *pb[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                pa[q] = &L.at(min(i0 + q, r - 1), c0);
-                pb[q] = &L.at(min(j0 + q, r - 1), c0);
-            }
-#pragma unroll 4
+            const float *pi = panel + i0 - c0, *pj = panel + j0 - c0;
+#pragma unroll 8
             for (int k = 0; k < kNB; ++k) {
-                float a[4], b[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    a[q] = pa[q][k];
-                    b[q] = pb[q][k];
-                }
+                const float4 a4 = *reinterpret_cast<const float4 *>(pi + k * ldp);
+                const float4 b4 = *reinterpret_cast<const float4 *>(pj + k * ldp);
+                const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -405,8 +375,55 @@ __device__ __forceinline__ void chol_panels(int r, const Low L, int *bad, float 
                 for (int j = 0; j < 4; ++j)
                     if (i0 + i < r && j0 + j <= i0 + i) L.at(i0 + i, j0 + j) = acc[i][j];
         }
+        if (tid < 32) {  // lane i holds row i of the block
+            __syncwarp();
+            float row[kNB];
+            bool failed = false;
+#pragma unroll
+            for (int j = 0; j < kNB; ++j) row[j] = tid < nb && j <= tid ? L.at(c0 + tid, c0 + j) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < kNB; ++k) {
+                float d = __shfl_sync(0xffffffffu, row[k], k);
+                const bool ok = d > 0.0f;
+                failed |= !ok && k < nb;
+                d = ok ? d : 1.0f;  // (past a ragged block's end: row k is zero and stays so)
+                const float piv = sqrtf(d);
+                row[k] = tid == k ? piv : row[k] / piv;
+                // (no branch around these: their shuffles are in flight together)
+#pragma unroll
+                for (int j = k + 1; j < kNB; ++j)
+                    row[j] = fmaf(-row[k], __shfl_sync(0xffffffffu, row[k], j), row[j]);
+            }
+            if (failed && tid == 0) *bad = 1;
+#pragma unroll
+            for (int j = 0; j < kNB; ++j) {
+                diag[j][tid] = row[j];
+                if (tid < nb && j <= tid) L.at(c0 + tid, c0 + j) = row[j];
+            }
+            __syncwarp();
+            dinv[tid] = 1.0f / diag[tid][tid];
+        }
+        __syncthreads();
+        // rows below: a thread per row, its 32 elements in registers
+        for (int i = c0 + nb + tid; i < r; i += nt) {
+            float v[kNB];
+#pragma unroll
+            for (int j = 0; j < kNB; ++j) v[j] = L.at(i, c0 + j);
+#pragma unroll
+            for (int k = 0; k < kNB; ++k) {
+                asm volatile("" ::: "memory");  // this column's 32 loads only (all 496 would not fit the registers)
+                v[k] = div_by(v[k], diag[k][k], dinv[k]);
+#pragma unroll
+                for (int j = k + 1; j < kNB; ++j) v[j] = fmaf(-v[k], diag[k][j], v[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < kNB; ++j) {
+                L.at(i, c0 + j) = v[j];
+                panel[j * ldp + i - c0 - nb] = v[j];
+            }
+        }
+        __syncthreads();
     }
-    __syncthreads();
 }
 
 // One CTA: Lw = the Cholesky factor of M (lower triangle, r x r) and *logdet of M; a non-positive
@@ -415,8 +432,10 @@ template <bool SMEM>
 __global__ void __launch_bounds__(512)
     chol_kernel(int r, const float *__restrict__ M, float *__restrict__ Lw, float *__restrict__ logdet,
                 int *__restrict__ bad) {
-    extern __shared__ float packed[];
-    __shared__ float diag[kNB][kNB + 1], red[32];
+    extern __shared__ __align__(16) float packed[];
+    __shared__ __align__(16) float diag[kNB][kNB + 4];
+    __shared__ float dinv[kNB], red[32];
+    float *panel = packed + (SMEM ? (r * (r + 1) / 2 + 3) / 4 * 4 : 0);
     const int tid = threadIdx.x, nt = blockDim.x;
     if (SMEM) {
         const LowerPacked L{packed};
@@ -424,7 +443,7 @@ __global__ void __launch_bounds__(512)
             const int i = t / r, j = t % r;
             if (j <= i) L.at(i, j) = M[t];
         }
-        chol_panels(r, L, bad, diag);
+        chol_panels(r, L, bad, diag, dinv, panel);
         for (int t = tid; t < r * r; t += nt) {
             const int i = t / r, j = t % r;
             if (j <= i) Lw[t] = L.at(i, j);
@@ -432,7 +451,7 @@ __global__ void __launch_bounds__(512)
     } else {
         const LowerDense L{Lw, r};
         for (int t = tid; t < r * r; t += nt) Lw[t] = M[t];
-        chol_panels(r, L, bad, diag);
+        chol_panels(r, L, bad, diag, dinv, panel);
     }
     __syncthreads();
     // log det M = 2 sum log L_kk, in the order of 1024 strided sums
@@ -454,53 +473,69 @@ __global__ void __launch_bounds__(512)
 }
 
 // X = L^-1, 32 columns per CTA: rows in blocks of 32, each first with the earlier blocks' part of the
-// sums (a thread per 4 columns of a row), then by forward substitution (a thread per column).
+// sums (a thread per 4 columns of a row), then by forward substitution (a thread per column).  A CTA
+// is one serial chain of blocks, so latency bounds it: its columns of X stay in shared memory, and the next 32 x 32 tile of L is requested before the present one is used
+// (r = 256: 103 us with both read from L2 when needed, 49 now).
+constexpr int kTriLd = kNB + 4;
 __global__ void __launch_bounds__(256) tri_inverse_kernel(int r, const float *__restrict__ Lw, float *__restrict__ X) {
-    __shared__ float Ls[kNB][kNB + 1];
-    __shared__ __align__(16) float Xs[kNB][kNB + 4], S[kNB][kNB + 4];
+    extern __shared__ __align__(16) float packed[];
+    float *const xs = packed;  // rows c0.. of the CTA's columns
+    __shared__ __align__(16) float Ls[kNB][kTriLd], S[kNB][kTriLd];
+    __shared__ float dinv[kNB];
     const int tid = threadIdx.x, c0 = blockIdx.x * kNB;
-    const int row = tid >> 3, cq = 4 * (tid & 7);
-    auto load = [&](float *dst, int ld, const float *src, int i0, int j0) {
-        for (int t = tid; t < kNB * kNB; t += 256) {
-            const int i = t / kNB, j = t % kNB;
-            dst[i * ld + j] = i0 + i < r && j0 + j < r ? src[(long long)(i0 + i) * r + j0 + j] : 0.0f;
+    const int row = tid >> 3, cq = 4 * (tid & 7), lr = tid >> 5, lc = tid & 31;
+    float next[kNB / 8];
+    auto request = [&](int i0, int k0) {
+#pragma unroll
+        for (int u = 0; u < kNB / 8; ++u) {
+            const int i = i0 + lr + 8 * u, k = k0 + lc;
+            next[u] = i < r && k < r ? __ldg(Lw + (long long)i * r + k) : 0.0f;
         }
     };
     for (int t = tid; t < c0 * kNB; t += 256)  // zeros above
         if (c0 + t % kNB < r) X[(long long)(t / kNB) * r + c0 + t % kNB] = 0.0f;
+    request(c0, c0);
     for (int i0 = c0; i0 < r; i0 += kNB) {
         float acc[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[q] = i0 + row == c0 + cq + q ? 1.0f : 0.0f;
-        for (int k0 = c0; k0 < i0; k0 += kNB) {
+        for (int k0 = c0; k0 <= i0; k0 += kNB) {
             __syncthreads();
-            load(&Ls[0][0], kNB + 1, Lw, i0, k0);
-            load(&Xs[0][0], kNB + 4, X, k0, c0);
+#pragma unroll
+            for (int u = 0; u < kNB / 8; ++u) Ls[lr + 8 * u][lc] = next[u];
+            const float *xb = xs + (k0 - c0) * kTriLd;
+            if (k0 < i0) request(i0, k0 + kNB);
+            else request(i0 + kNB, c0);
+            if (k0 == i0) *reinterpret_cast<float4 *>(&S[row][cq]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
             __syncthreads();
-#pragma unroll 8
-            for (int k = 0; k < kNB; ++k) {
-                const float l = Ls[row][k];
-                const float4 x = *reinterpret_cast<const float4 *>(&Xs[k][cq]);
-                acc[0] = fmaf(-l, x.x, acc[0]);
-                acc[1] = fmaf(-l, x.y, acc[1]);
-                acc[2] = fmaf(-l, x.z, acc[2]);
-                acc[3] = fmaf(-l, x.w, acc[3]);
-            }
-        }
-        __syncthreads();
-        load(&Ls[0][0], kNB + 1, Lw, i0, i0);
-        *reinterpret_cast<float4 *>(&S[row][cq]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        __syncthreads();
-        if (tid < kNB) {
-            float x[kNB];
+            if (k0 < i0) {
 #pragma unroll
-            for (int i = 0; i < kNB; ++i) {
-                asm volatile("" ::: "memory");  // (one row's loads at a time)
-                float v = S[i][tid];
+                for (int k = 0; k < kNB; k += 4) {
+                    const float4 l4 = *reinterpret_cast<const float4 *>(&Ls[row][k]);
+                    const float l[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-                for (int k = 0; k < i; ++k) v = fmaf(-Ls[i][k], x[k], v);
-                x[i] = i0 + i < r ? v / Ls[i][i] : 0.0f;
-                if (i0 + i < r && c0 + tid < r) X[(long long)(i0 + i) * r + c0 + tid] = x[i];
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 x = *reinterpret_cast<const float4 *>(xb + (k + u) * kTriLd + cq);
+                        acc[0] = fmaf(-l[u], x.x, acc[0]);
+                        acc[1] = fmaf(-l[u], x.y, acc[1]);
+                        acc[2] = fmaf(-l[u], x.z, acc[2]);
+                        acc[3] = fmaf(-l[u], x.w, acc[3]);
+                    }
+                }
+            } else if (tid < kNB) {
+                dinv[tid] = 1.0f / Ls[tid][tid];
+                __syncwarp();
+                float x[kNB];
+#pragma unroll
+                for (int i = 0; i < kNB; ++i) {
+                    asm volatile("" ::: "memory");  // (one row's loads at a time)
+                    float v = S[i][tid];
+#pragma unroll
+                    for (int k = 0; k < i; ++k) v = fmaf(-Ls[i][k], x[k], v);
+                    x[i] = i0 + i < r ? div_by(v, Ls[i][i], dinv[i]) : 0.0f;
+                    xs[(i0 - c0 + i) * kTriLd + tid] = x[i];
+                    if (i0 + i < r && c0 + tid < r) X[(long long)(i0 + i) * r + c0 + tid] = x[i];
+                }
             }
         }
     }
@@ -510,17 +545,17 @@ __global__ void __launch_bounds__(256) tri_inverse_kernel(int r, const float *__
 inline cudaError_t spd_inverse(cudaStream_t st, int r, const float *M, float *Lw, float *X, float *Minv, float *logdet,
                                int *bad) {
     cudaError_t e;
-    if (r <= kCholSmemMax) {
-        const size_t smem = sizeof(float) * (size_t)r * (r + 1) / 2;
-        if ((e = cudaFuncSetAttribute(chol_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(float) * kCholSmemMax * (kCholSmemMax + 1) / 2))))
-            return e;
-        chol_kernel<true><<<1, 512, smem, st>>>(r, M, Lw, logdet, bad);
-    } else {
-        chol_kernel<false><<<1, 512, 0, st>>>(r, M, Lw, logdet, bad);
-    }
+    if (r > kInverseMax) return cudaErrorInvalidValue;
+    constexpr size_t kSmemMost = 216 * 1024;  // dynamic shared memory asked for at most
+    const size_t tri = r <= kCholSmemMax ? sizeof(float) * (((size_t)r * (r + 1) / 2 + 3) / 4 * 4) : 0;
+    const auto chol = r <= kCholSmemMax ? chol_kernel<true> : chol_kernel<false>;
+    if ((e = cudaFuncSetAttribute(chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost))) return e;
+    chol<<<1, 512, tri + chol_panel_bytes(r), st>>>(r, M, Lw, logdet, bad);
     if ((e = cudaGetLastError())) return e;
-    tri_inverse_kernel<<<(unsigned)((r + kNB - 1) / kNB), 256, 0, st>>>(r, Lw, X);
+    const int blocks = (r + kNB - 1) / kNB;
+    if ((e = cudaFuncSetAttribute(tri_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost)))
+        return e;
+    tri_inverse_kernel<<<(unsigned)blocks, 256, sizeof(float) * (size_t)blocks * kNB * kTriLd, st>>>(r, Lw, X);
     if ((e = cudaGetLastError())) return e;
     return gemm(st, r, r, r, X, r, X, r, nullptr, 1.0f, 0.0f, nullptr, 0, Minv);
 }
