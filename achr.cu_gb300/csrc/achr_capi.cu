@@ -579,7 +579,7 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     ACHR_CUDA_TRY(ctx->counters.alloc(achr::CNT_SLOTS));
 
     // Warmup matrix with an even leading dimension so every column starts on a
-    // 16-byte boundary (a TMA bulk-copy requirement).
+    // 16-byte boundary (read in pairs).
     ctx->ldw = (n + 1) & ~1;
     ACHR_CUDA_TRY(ctx->warmup.alloc((size_t)ctx->ldw * n_warmup));
     ACHR_CUDA_TRY(cudaMemset(ctx->warmup.p, 0, sizeof(double) * (size_t)ctx->ldw * n_warmup));

@@ -719,7 +719,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     }
     cta_sync<BD>();
 
-    const bool hr = a.hit_and_run != 0;  // directions are the staged columns themselves (no centre)
+    const bool hr = a.hit_and_run != 0;  // directions are the columns themselves (no centre)
     const bool merged = a.merged_ab != 0 && !a.exact_ratio;  // ratio-test brackets formed before ||d|| is known
     const int npair = (a.n + 1) >> 1;
     const int odd = (a.n & 1) ? npair - 1 : -1;  // the pair whose second reaction is padding

@@ -80,8 +80,8 @@ struct ChainArgs {
     int hit_and_run;            // 1: `warmup` holds directions; d = column r, no centre (A stays as loaded)
     double residual_tol, max_min_tol, u_tol, d_tol, feasibility_tol;
     unsigned long long *counters;  // CNT_SLOTS entries
-    unsigned long long wait_ns;    // limit of the wait for a staged column (0: the default, 2 s)
-    int wait_never;                // 1: that wait is on a barrier nothing completes (tests the timeout)
+    unsigned long long wait_ns;    // limit of the wait that tests the timeout (0: the default, 2 s)
+    int wait_never;                // 1: wait, before the first chain, on a barrier nothing completes
     // Segmented sampling (achr_defer.cu): the reference's per-chain reprojection
     // is deferred to a batched pass between launches.  A launch runs the steps
     // [step0, step0 + T) of every chain; a check step ends the chain's launch

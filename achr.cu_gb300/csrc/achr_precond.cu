@@ -434,7 +434,7 @@ struct PcWork {
 // both ways round, with the sums of Y V and V V per coordinate.  The chain from
 // M to T = V^T U keeps the order of every sum (nothing split): T is a difference
 // of large terms when U dominates, and carries the rounding of all of them.
-// d = 940, r = 256, B = 4096: 0.61 ms for the whole call (6.34 before: 4.9 the
+// d = 940, r = 256, B = 4096: 0.51 ms for the whole call (6.34 before: 4.9 the
 // inverse of M, 0.9 the products, 0.5 allocations), 0.27 of them the products.
 cudaError_t loss_grad(cudaStream_t st, int d, int r, int B, const float *s, const float *U, const float *Y,
                       long long ldy, PcWork &w, float *gs, float *gU) {
