@@ -945,7 +945,11 @@ achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out) {
     if (!ctx) return fail(ACHR_ERR_INVALID, "ctx is NULL");
     int dev = 0;
     ACHR_CUDA_TRY(cudaGetDevice(&dev));
-    const std::pair<int, int> key(achr::chain_padded_length(ctx->n, 0), dev);
+    // A context that reprojects through the residual in the kernel takes only
+    // configurations that leave it room (the others would fall back to N (N^T x)).
+    ChainArgs probe = chain_args(ctx, 0, 0, 0, 0, nullptr, 0);
+    const bool residual = probe.pinv32 && ctx->opt.check_period > 0;
+    const std::pair<int, int> key(2 * achr::chain_padded_length(ctx->n, 0) + (residual ? 1 : 0), dev);
     int cand[8];
     int nc = 0;
     {
@@ -956,7 +960,16 @@ achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out) {
             nc = 1;
         }
     }
-    if (nc == 0) nc = achr::chain_candidates(ctx->n, ctx->np, cand, 8);
+    if (nc == 0) {
+        nc = achr::chain_candidates(ctx->n, ctx->np, cand, 8);
+        int kept = 0;
+        for (int c = 0; c < nc && residual; ++c) {
+            int per_sm = 0;
+            ACHR_CUDA_TRY(achr::launch_chains(probe, cand[c], nullptr, 0, &per_sm));
+            if (per_sm > 0) cand[kept++] = cand[c];
+        }
+        if (kept > 0) nc = kept;
+    }
     if (nc == 0) return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration to tune");
     int sms = 0;
     ACHR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1009,11 +1022,11 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
         if (!c || n_points[k] < 0 || (n_points[k] > 0 && (!d_points_out[k] || ld_out[k] < n_points[k])))
             return fail(ACHR_ERR_INVALID, "bad batch entry " + std::to_string(k));
         int bd = 0, ept = 0;
-        if (!achr::chain_config(c->n, c->opt.threads_per_chain, std::max(c->m, c->d), &bd, &ept) || bd * ept > c->np)
-            return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for batch entry " + std::to_string(k));
-        cfg_key[(size_t)k] = bd * 100 + ept;
         // disjoint chain ids: model k uses ids off .. off + P_k - 1
         args[(size_t)k] = chain_args(c, seed, off, n_points[k], n_steps, d_points_out[k], ld_out[k]);
+        if (!achr::chain_config(args[(size_t)k], c->opt.threads_per_chain, &bd, &ept) || bd * ept > c->np)
+            return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for batch entry " + std::to_string(k));
+        cfg_key[(size_t)k] = bd * 100 + ept;
         off += (uint64_t)n_points[k];
         // measured by the autotuner (whole-GPU rate), else padded elements x steps
         chain_time[(size_t)k] = c->tuned_rate > 0 ? (double)n_steps / c->tuned_rate
@@ -1062,7 +1075,11 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
             if (e != cudaSuccess || per_sm_z < per_sm) {
                 (void)cudaGetLastError();
                 extra = 0;
-                for (int k : G.models) args[(size_t)k].pinv32 = nullptr;
+                for (int k : G.models) {  // z takes turns beside the residual, or the form is off
+                    ChainArgs &a = args[(size_t)k];
+                    a.z_rows = achr::residual_z_rows(a.m, achr::chain_scratch_doubles(G.bd, G.ept));
+                    if (!a.z_rows) a.pinv32 = nullptr;
+                }
             }
         }
         G.extra = extra;

@@ -496,7 +496,7 @@ __device__ __forceinline__ void null_coordinates(const ChainArgs &a, const doubl
 // the residual's preimage; the update x_j -= sum_i S_ij z_i is FP64 (CSC).
 template <int BD>
 __device__ __forceinline__ void residual_form_reproject(const ChainArgs &a, double *xs, float2 *rr, float *zs,
-                                                        int tid) {
+                                                        int zcap, int tid) {
     constexpr int NW = BD / 32;
     const int lane = tid & 31, warp = tid >> 5;
     const int m = a.m;
@@ -507,24 +507,31 @@ __device__ __forceinline__ void residual_form_reproject(const ChainArgs &a, doub
         }
     });
     __syncthreads();
-    for (int i = warp; i < m; i += NW) {
-        const float *Bi = a.pinv32 + (size_t)i * (size_t)m;
-        float acc = 0.0f;
-        for (int k = lane; k < m; k += 32) {
-            const float b = __ldg(Bi + k);
-            const float2 r = rr[k];
-            acc = fmaf(b, r.x, fmaf(b, r.y, acc));
-        }
+    for (int i0 = 0; i0 < m; i0 += zcap) {  // zcap rows of z at a time
+        const int rows = min(zcap, m - i0);
+        for (int i = i0 + warp; i < i0 + rows; i += NW) {
+            const float *Bi = a.pinv32 + (size_t)i * (size_t)m;
+            float acc = 0.0f;
+            for (int k = lane; k < m; k += 32) {
+                const float b = __ldg(Bi + k);
+                const float2 r = rr[k];
+                acc = fmaf(b, r.x, fmaf(b, r.y, acc));
+            }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) zs[i] = acc;
-    }
-    __syncthreads();
-    for (int j = tid; j < a.n; j += BD) {
-        double dl = 0.0;
-        const int q1 = __ldg(a.csc_ptr + j + 1);
-        for (int q = __ldg(a.csc_ptr + j); q < q1; ++q) dl = fma(__ldg(a.csc_val + q), (double)zs[__ldg(a.csc_row + q)], dl);
-        xs[j] -= dl;
+            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) zs[i - i0] = acc;
+        }
+        __syncthreads();
+        for (int j = tid; j < a.n; j += BD) {
+            double dl = 0.0;
+            const int q1 = __ldg(a.csc_ptr + j + 1);
+            for (int q = __ldg(a.csc_ptr + j); q < q1; ++q) {
+                const int i = __ldg(a.csc_row + q) - i0;
+                if ((unsigned)i < (unsigned)rows) dl = fma(__ldg(a.csc_val + q), (double)zs[i], dl);
+            }
+            xs[j] -= dl;
+        }
+        if (i0 + zcap < m) __syncthreads();  // (read before the next rows take their place)
     }
 }
 
@@ -708,7 +715,8 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
     // largest residual and bound violation of the CTA's emitted points (bits of non-negative doubles)
     unsigned long long *worst = reinterpret_cast<unsigned long long *>(never + 1);
     // (S S^T)^+ r of the residual-form reprojection (m floats), when enabled
-    float *zs = reinterpret_cast<float *>(smem_raw + chain_smem_bytes_cfg<BD, EPT>());
+    float *zs = a.z_rows ? reinterpret_cast<float *>(As) + 2 * a.m
+                         : reinterpret_cast<float *>(smem_raw + chain_smem_bytes_cfg<BD, EPT>());
 
     if (tid == 0) {
         *exact_count = 0;
@@ -1310,7 +1318,8 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
                         }
                         cta_sync<BD>();
                         if (a.pinv32) {
-                            residual_form_reproject<BD>(a, xs, reinterpret_cast<float2 *>(As), zs, tid);
+                            residual_form_reproject<BD>(a, xs, reinterpret_cast<float2 *>(As), zs,
+                                                        a.z_rows ? a.z_rows : a.m, tid);
                         } else {
                             const int n = a.n;
                             null_coordinates<BD>(a, xs, ys, tid);
@@ -1555,13 +1564,17 @@ template <int BD, int EPT, bool SEG>
 cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int max_ctas, int *per_sm_out) {
     auto *const KFN = achr_chain_kernel<BD, EPT, SEG>;
     ChainArgs a = a_in;
+    a.z_rows = 0;
     const size_t base = chain_smem_bytes_cfg<BD, EPT>();
     // The residual-form reprojection keeps z (m floats) in shared memory and
-    // the residual in the accumulator's place; it is used only when z fits
-    // without costing a resident CTA per SM.
+    // the residual in the accumulator's place.  Where z would cost a resident
+    // CTA per SM, it takes turns in what the residual leaves of that place
+    // (5063 x 7440, 256 x 30: three turns of 2162 rows), if those are at most
+    // eight; else the form is not used.
     const size_t zbytes = ((size_t)a.m * sizeof(float) + 15) & ~(size_t)15;
     // (its residual takes the accumulator's place while that waits in registers: m <= ldw <= NP)
     if (a.pinv32 && a.m > a.ldw) a.pinv32 = nullptr;
+    const bool asked = a.pinv32 != nullptr;
     size_t smem = base + (a.pinv32 ? zbytes : 0);
     cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)std::max(smem, base));
@@ -1574,12 +1587,13 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_z, KFN, BD, smem);
         if (e != cudaSuccess) return e;
         if (per_sm_z < per_sm) {
-            a.pinv32 = nullptr;
+            a.z_rows = residual_z_rows(a.m, chain_acc_doubles<BD, EPT>());
+            if (!a.z_rows) a.pinv32 = nullptr;
             smem = base;
         }
     }
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    if (per_sm_out) *per_sm_out = per_sm;
+    if (per_sm_out) *per_sm_out = asked && !a.pinv32 ? -per_sm : per_sm;  // < 0: without the residual form
     if (a.P <= 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

@@ -78,6 +78,40 @@ const Cfg *find_cfg_for(const ChainArgs &a, int sms) {
     return best;
 }
 
+cudaError_t launch_cfg_of(const Cfg &c, const ChainArgs &a, cudaStream_t stream, int max_ctas, int *per_sm) {
+    if (c.bd <= 64) return launch_chain_cfg_small(c.bd, c.ept, a, stream, max_ctas, per_sm);
+    if (c.bd <= 128) return launch_chain_cfg_mid(c.bd, c.ept, a, stream, max_ctas, per_sm);
+    return launch_chain_cfg_large(c.bd, c.ept, a, stream, max_ctas, per_sm);
+}
+
+// The default for a model that reprojects through the residual in the kernel:
+// the first configuration, from its length's default on, in which z has room.
+// Reprojecting as N (N^T x) instead costs 4 n d FP64 operations, 11 ms of an SM
+// at 5063 x 7440 against a step's 23 K clocks.  The choice, and with it the form
+// and its turns, does not depend on the number of chains.
+cudaError_t find_cfg_residual(const ChainArgs &a, const Cfg **out) {
+    const int scratch = a.m > a.d ? a.m : a.d;
+    const Cfg *dflt = *out = find_cfg(a.n, 0, scratch);
+    if (!dflt) return cudaSuccess;
+    ChainArgs q = a;
+    q.P = 0;  // (asks for the residency only)
+    for (const Cfg *c = dflt; c != kLadder + sizeof(kLadder) / sizeof(kLadder[0]); ++c) {
+        if (c->bd * c->ept > a.np) continue;
+        if (c->bd == 256 && c->ept == 30 && scratch > kScratch256x30) continue;
+        int per_sm = 0;
+        const cudaError_t e = launch_cfg_of(*c, q, nullptr, 0, &per_sm);
+        if (e != cudaSuccess) return e;
+        if (per_sm > 0) {
+            *out = c;
+            break;
+        }
+    }
+    return cudaSuccess;
+}
+
+// Whether the kernel may reproject through the residual at its checks.
+bool residual_form(const ChainArgs &a) { return a.pinv32 && a.check_period != 0x7fffffff && !a.seg; }
+
 }  // namespace
 
 int chain_padded_length(int n, int threads_per_chain) {
@@ -120,8 +154,13 @@ bool chain_takes_threads(int n, int threads_per_chain) {
     return threads_per_chain == 0 || n <= most;
 }
 
-bool chain_config(int n, int threads_per_chain, int scratch, int *bd, int *ept) {
-    const Cfg *c = find_cfg(n, threads_per_chain, scratch);
+int chain_scratch_doubles(int bd, int ept) {
+    return bd == 256 && ept == 30 ? kScratch256x30 : bd * ept;
+}
+
+bool chain_config(const ChainArgs &a, int threads_per_chain, int *bd, int *ept) {
+    const Cfg *c = find_cfg(a.n, threads_per_chain, a.m > a.d ? a.m : a.d);
+    if (c && threads_per_chain == 0 && residual_form(a) && find_cfg_residual(a, &c) != cudaSuccess) return false;
     if (!c) return false;
     *bd = c->bd;
     *ept = c->ept;
@@ -137,7 +176,10 @@ cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_
 cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_t stream, int max_ctas,
                           int *per_sm) {
     const Cfg *c = find_cfg(a.n, threads_per_chain, a.m > a.d ? a.m : a.d);
-    if (threads_per_chain == 0 && a.P > 0) {
+    if (threads_per_chain == 0 && residual_form(a)) {
+        const cudaError_t e = find_cfg_residual(a, &c);
+        if (e != cudaSuccess) return e;
+    } else if (threads_per_chain == 0 && a.P > 0) {
         int dev = 0, sms = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -146,9 +188,7 @@ cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_
     }
     if (!c || c->bd * c->ept > a.np) return cudaErrorInvalidValue;
     if (a.P <= 0 && !per_sm) return cudaSuccess;
-    if (c->bd <= 64) return launch_chain_cfg_small(c->bd, c->ept, a, stream, max_ctas, per_sm);
-    if (c->bd <= 128) return launch_chain_cfg_mid(c->bd, c->ept, a, stream, max_ctas, per_sm);
-    return launch_chain_cfg_large(c->bd, c->ept, a, stream, max_ctas, per_sm);
+    return launch_cfg_of(*c, a, stream, max_ctas, per_sm);
 }
 
 }  // namespace achr

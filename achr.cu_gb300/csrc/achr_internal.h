@@ -63,6 +63,7 @@ struct ChainArgs {
     // Residual-form reprojection x <- x - S^T (S S^T)^+ S x: the pseudo-inverse
     // in FP32 (m x m, device row order) and the CSC of S; pinv32 NULL: N (N^T x).
     const float *pinv32;
+    int z_rows;                 // 0: z has shared memory of its own; else the rows of z held at a time beside r
     const int *csc_ptr;
     const int *csc_row;
     const double *csc_val;
@@ -163,7 +164,8 @@ inline void set_merged_bound(ChainArgs &a, double u_tol, double dnorm_max) {
 
 // Launch the persistent chain kernel; threads_per_chain = 0 picks the default
 // configuration for n.  max_ctas > 0 caps the grid; per_sm (if non-NULL)
-// receives the resident CTAs per SM of the configuration.  a.np is the length
+// receives the resident CTAs per SM of the configuration (negative: too many to
+// leave room for the residual-form reprojection that `a` asks for).  a.np is the length
 // the per-reaction arrays were padded to (>= the configuration's BD * EPT).
 cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_t stream, int max_ctas = 0,
                           int *per_sm = nullptr);
@@ -171,9 +173,15 @@ cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_
 // Configuration ladder: threads per chain and padded element count for n
 // reactions (threads_per_chain = 0: default); 0 if no configuration fits.
 int chain_block_size(int n, int threads_per_chain);
-// Configuration (threads, elements per thread) the model of n reactions runs with.
-// for a reprojection scratch of `scratch` doubles (the larger of m and d).
-bool chain_config(int n, int threads_per_chain, int scratch, int *bd, int *ept);
+// Configuration (threads, elements per thread) a batch runs the model with.
+int chain_scratch_doubles(int bd, int ept);  // the accumulator's share of shared memory
+// Rows of z = (S S^T)^+ r that fit beside r (m float pairs) in `scratch` doubles; 0
+// where that would take more than eight turns.
+inline int residual_z_rows(int m, int scratch) {
+    const int rows = 2 * (scratch - m);
+    return rows <= 0 || (long long)rows * 8 < m ? 0 : rows < m ? rows : m;
+}
+bool chain_config(const ChainArgs &a, int threads_per_chain, int *bd, int *ept);
 // Whether a caller may ask for this many threads per chain at n reactions (the
 // defaults and the autotuner also use longer configurations of a thread count).
 bool chain_takes_threads(int n, int threads_per_chain);

@@ -65,3 +65,19 @@ def test_long_scratch_takes_another_configuration(pkg):
     (x0, st0), (x1, st1) = pts
     assert np.array_equal(x0, x1)
     assert st0["reprojections"] == st1["reprojections"]
+
+
+@pytest.mark.parametrize("n", [1059, 3072, 6000, 7440])  # the larger: z takes turns beside the residual
+@pytest.mark.parametrize("form", [1, 2])
+def test_reprojection_independent_of_configuration(pkg, oracle_mod, n, form):
+    model, N, warm = _block_model(pkg, n // 3, seed=n)
+    warm = warm + 1e-7 * np.random.default_rng(n).standard_normal(warm.shape)  # every check reprojects
+    T = 22
+    with pkg.Sampler(model, warm, reproject_form=form) as s:
+        s.set_null_space(N)
+        base, st = s.sample(16, T, seed=9)
+        for P in (200, 700):
+            assert np.array_equal(s.sample(P, T, seed=9)[0][:, :16], base)
+    ref, rst = oracle_mod.sample(model, warm, N, 9, 16, T)
+    assert st["reprojections"] == rst["reprojections"] > 0
+    assert np.abs(base - ref).max() <= 1e-10 * max(1.0, np.abs(ref).max())
