@@ -291,6 +291,60 @@ achr_status null_space_svd_s(int n, int m, const std::vector<double> &denseS, st
     return ACHR_OK;
 }
 
+// Largest |G_ij - I_ij| over columns j0 .. j0 + cols - 1 of a Gram matrix (d x cols, column-major).
+__global__ void gram_error_kernel(int d, int cols, int j0, const double *__restrict__ G, unsigned long long *maxbits) {
+    unsigned long long mx = 0;
+    const long long cnt = (long long)d * cols;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += (long long)gridDim.x * blockDim.x) {
+        const double e = G[t] - (t % d == j0 + t / d ? 1.0 : 0.0);
+        mx = max(mx, (unsigned long long)__double_as_longlong(e) & 0x7FFFFFFFFFFFFFFFull);
+    }
+    if (mx) atomicMax(maxbits, mx);
+}
+
+// Whether the context's basis is an orthonormal basis of null(S), so that N (N^T x) is the projector
+// x - S^T (S S^T)^+ S x that the deferred and the residual form are built from: as many columns as S's
+// own, N^T N = I and S N = 0, both to kBasisTol (a basis from an FP64 factorisation meets them to
+// 1e-11 or better wherever those forms are used at all).
+constexpr double kBasisTol = 1e-10;
+achr_status spans_null_space(const achr_ctx *ctx, bool &spans) {
+    spans = ctx->m == 0;
+    const int n = ctx->n, d = ctx->d;
+    if (ctx->m == 0 || d != ctx->d_null) return ACHR_OK;
+    if (d == 0) {
+        spans = true;
+        return ACHR_OK;
+    }
+    double smax = 0.0;
+    for (double v : ctx->h_val) smax = std::max(smax, std::fabs(v));
+    const int chunk = std::min(d, 1024);  // columns of the Gram matrix at a time
+    DevBuf<unsigned long long> bits;      // [0] max|S N|, [1] max|N^T N - I|, as non-negative doubles
+    DevBuf<double> G;
+    ACHR_CUDA_TRY(bits.alloc(2));
+    ACHR_CUDA_TRY(G.alloc((size_t)d * chunk));
+    ACHR_CUDA_TRY(cudaMemset(bits.p, 0, 2 * sizeof(unsigned long long)));
+    warmup_residual_kernel<<<d, 128>>>(ctx->m, n, ctx->N.p, ctx->rowptr.p, ctx->colidx.p, ctx->val.p, bits.p);
+    ACHR_CUDA_TRY(cudaGetLastError());
+    cublasHandle_t cb = nullptr;
+    if (cublasCreate(&cb) != CUBLAS_STATUS_SUCCESS) return fail(ACHR_ERR_CUDA, "cublasCreate failed");
+    const double one = 1.0, zero = 0.0;
+    cublasStatus_t bs = CUBLAS_STATUS_SUCCESS;
+    for (int j0 = 0; j0 < d && bs == CUBLAS_STATUS_SUCCESS; j0 += chunk) {
+        const int cols = std::min(chunk, d - j0);
+        bs = cublasDgemm(cb, CUBLAS_OP_T, CUBLAS_OP_N, d, cols, n, &one, ctx->N.p, n, ctx->N.p + (size_t)j0 * n, n, &zero,
+                         G.p, d);
+        gram_error_kernel<<<256, 256>>>(d, cols, j0, G.p, bits.p + 1);
+    }
+    cublasDestroy(cb);
+    if (bs != CUBLAS_STATUS_SUCCESS) return fail(ACHR_ERR_CUDA, "cublasDgemm (N^T N) failed");
+    ACHR_CUDA_TRY(cudaGetLastError());
+    double err[2];
+    static_assert(sizeof err == 2 * sizeof(unsigned long long), "read back as bits");
+    ACHR_CUDA_TRY(cudaMemcpy(err, bits.p, sizeof err, cudaMemcpyDeviceToHost));
+    spans = err[0] <= kBasisTol * smax && err[1] <= kBasisTol;  // (a NaN is no)
+    return ACHR_OK;
+}
+
 achr_status upload_null_space(achr_ctx *ctx, const double *N, int d) {
     ctx->d = d;
     ACHR_CUDA_TRY(ctx->N.upload(N, (size_t)ctx->n * (size_t)(d > 0 ? d : 0)));
@@ -593,6 +647,7 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
             denseS[(size_t)ctx->h_colidx[q] * m + r] = ctx->h_val[q];
     std::vector<double> Nh;
     int d = 0;
+    bool augmented = false;    // the basis is of S with more rows
     achr::RowSpace row_space;  // from the null space's eigen-decomposition, for the reprojection operator
     DevBuf<double> eigenvectors;
     if (m == 0) {
@@ -613,6 +668,7 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
         double kappa_aug = 1.0;
         st = null_space_sts(n, ma, Sa, Nh, d, kappa_aug);
         if (st != ACHR_OK) return st;
+        augmented = !fixed.empty();
         ctx->kappa_sst = INFINITY;  // the deferred projector (built from S alone) would not match this basis
     } else {
         st = (opt.null_space == ACHR_NULL_SVD_S) ? null_space_svd_s(n, m, denseS, Nh, d, ctx->kappa_sst)
@@ -622,6 +678,9 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     }
     st = upload_null_space(ctx, Nh.data(), d);
     if (st != ACHR_OK) return st;
+    // (d = n with constraints: the rule found no null vector and keeps every column)
+    ctx->basis_spans = m == 0 || (!augmented && d < n);
+    ctx->d_null = ctx->basis_spans ? d : -1;
     const achr::RowSpace *rows = row_space.V ? &row_space : nullptr;
     // Large models reproject a chain through (S S^T)^+ on the residual (about
     // m^2 FP32 operations) instead of N (N^T x) (4 n d FP64 operations).
@@ -654,7 +713,9 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
 
 achr_status achr_set_null_space(achr_ctx *ctx, const double *N, int32_t d) {
     if (!ctx || (!N && d > 0) || d < 0 || d > ctx->n) return fail(ACHR_ERR_INVALID, "bad null-space arguments");
+    ctx->basis_spans = false;
     achr_status st = upload_null_space(ctx, N, d);
+    if (st == ACHR_OK) st = spans_null_space(ctx, ctx->basis_spans);
     if (st != ACHR_OK || ctx->opt.mode != ACHR_MODE_FEASIBLE) return st;
     return prepare_warmup_and_centre(ctx);  // re-project the warmup points onto the new basis
 }
@@ -759,7 +820,7 @@ ChainArgs chain_args(const achr_ctx *ctx, uint64_t seed, uint64_t chain_offset, 
     a.row_ptr = ctx->rowptr.p;
     a.col_idx = ctx->colidx.p;
     a.val = ctx->val.p;
-    a.pinv32 = ctx->pinv32.p;
+    a.pinv32 = ctx->basis_spans || ctx->opt.reproject_form == 2 ? ctx->pinv32.p : nullptr;
     a.csc_ptr = ctx->csc_ptr.p;
     a.csc_row = ctx->csc_row.p;
     a.csc_val = ctx->csc_val.p;

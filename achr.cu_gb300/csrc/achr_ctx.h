@@ -94,6 +94,10 @@ struct achr_ctx {
     int n = 0, m = 0, W = 0, d = 0, ldw = 0, np = 0;
     float bound_err = 0.0f;
     bool bound_exact = false;  // every bound finite and exact in FP32
+    // N is an orthonormal basis of null(S) (a caller's may be another), so that the automatic choice may
+    // reproject through S instead; dimension of null(S) (-1: not known)
+    bool basis_spans = true;
+    int d_null = -1;
     // sqrt(sum_i max(lb_i^2, ub_i^2)): every point and centre of a chain lies in
     // the box, so ||w - c|| <= 2 box_norm (inf when a bound is infinite)
     double box_norm = 0.0;

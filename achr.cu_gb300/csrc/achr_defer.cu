@@ -776,7 +776,8 @@ bool defer_selected(const achr_ctx *ctx) {
     // converge too slowly to be worth it, and far beyond they diverge.
     if (ctx->kappa_sst > kDeferMaxKappa) return false;
     if (o.reproject_form == 3) return true;
-    if (o.reproject_form != 0 || ctx->n_dirs > 0) return false;
+    // The passes project onto null(S), whatever basis a caller has set.
+    if (o.reproject_form != 0 || ctx->n_dirs > 0 || !ctx->basis_spans) return false;
     return ctx->warmup_residual > o.residual_tol / 8.0;
 }
 

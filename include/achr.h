@@ -86,7 +86,9 @@ typedef struct {
                                     check then reprojects), n_rxns x null_dim >= 2.5e5 or chains x
                                     n_rxns x null_dim >= 2e7, and form 3's conditions hold; otherwise
                                     in the chain kernel, as 2 when
-                                    n_rxns x null_dim >= 4e6, else as 1,
+                                    n_rxns x null_dim >= 4e6, else as 1; always as 1 where the basis in
+                                    use is not an orthonormal basis of null(S) (a caller's subspace,
+                                    ACHR_NULL_FIXED with blocked reactions),
                                  1: N (N^T x) in FP64 in the chain kernel,
                                  2: x - S^T (S S^T)^+ S x in the chain kernel, the pseudo-inverse product
                                     in FP32 on the residual (equal in exact arithmetic; m^2 FP32 instead
@@ -161,7 +163,10 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
 
 /* Replace the context's null-space basis with a caller-supplied one (n x d,
  * column-major, host memory).  The reference computes it internally
- * (ACHRCuda.cu:698-704); this lets a caller pin N across implementations.
+ * (ACHRCuda.cu:698-704); this lets a caller pin N across implementations, or
+ * reproject onto another space: reproject_form 0 and 1 reproject onto N's span
+ * (0 through S only where N is an orthonormal basis of null(S), to 1e-10),
+ * 2 and 3, asked for by name, onto null(S).
  * In ACHR_MODE_FEASIBLE the warmup points are projected onto the new basis
  * and the centre is recomputed. */
 achr_status achr_set_null_space(achr_ctx *ctx, const double *N, int32_t d);
