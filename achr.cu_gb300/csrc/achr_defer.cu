@@ -96,7 +96,11 @@ struct DeferState {
     std::vector<cudaEvent_t> ev;
     int ev_used = 0;
     double chains_per_sweep = 0.0;
+    // Recorded behind the last run: the buffers above hold one run at a time, so the next run,
+    // which may come on another stream, waits for it.
+    cudaEvent_t done = nullptr;
     ~DeferState() {
+        if (done) cudaEventDestroy(done);
         for (cudaEvent_t e : ev) cudaEventDestroy(e);
     }
 };
@@ -753,6 +757,8 @@ achr_status ensure_defer(achr_ctx *ctx, int chains, int segments) {
         DEFER_TRY(D->dxh.alloc(c * (size_t)D->ld));
         DEFER_TRY(D->dxl.alloc(c * (size_t)D->ld));
         DEFER_TRY(D->r0.alloc(c));
+        // (the memsets run on the default stream, which a non-blocking stream does not wait for)
+        DEFER_TRY(cudaStreamSynchronize(nullptr));
         D->cap = chains;
     }
     if (D->any_cap < segments) {
@@ -834,6 +840,22 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
     const int segments = segments_of(a_in);
     DeferState &D = *ctx->defer;
     const ReprojState &R = *ctx->reproj;
+    // One run at a time in the buffers.  A captured run has no event of its own (a graph may not wait
+    // for work outside its capture): its replays are ordered against other runs by the program.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DEFER_TRY(cudaStreamIsCapturing(s, &capture));
+    struct Turn {
+        cudaEvent_t done;
+        cudaStream_t s;
+        ~Turn() {
+            if (done) cudaEventRecord(done, s);
+        }
+    } turn{nullptr, s};
+    if (capture == cudaStreamCaptureStatusNone) {
+        if (D.done) DEFER_TRY(cudaStreamWaitEvent(s, D.done, 0));
+        else DEFER_TRY(cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming));
+        turn.done = D.done;
+    }
     D.ev_used = 0;
     D.chains_per_sweep = (double)P / (double)((P + cap - 1) / cap);
     auto mark = [&]() -> cudaError_t {  // record the next timing event on the stream
