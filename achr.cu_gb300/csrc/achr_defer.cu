@@ -56,7 +56,9 @@
 #include <vector>
 
 #include "achr_ctx.h"
+#include "achr_defer_rule.h"
 #include "achr_float.cuh"
+#include "achr_kept.h"
 
 extern "C" void achr_io_set_error(const char *msg);
 
@@ -73,12 +75,9 @@ struct SlicedEll {
     DevBuf<float> vh, vl;
 };
 
-struct DeferState {
-    int cap = 0;             // chains the buffers hold
-    long long ld = 0;        // leading dimension of the chain-major state (n rounded up to even)
-    int ldz = 0;             // leading dimension of Z and r (m rounded up to a multiple of 4)
-    int kpad = 0;            // K of the GEMM: m rounded up to a multiple of 64
-    bool exact32 = false;    // every coefficient of S is exact in FP32 (all lo parts zero)
+// A run's buffers.
+struct DeferBufs {
+    int cap = 0;             // chains they hold
     DevBuf<double> x, A;     // cap x ld: points and centre accumulators between launches
     DevBuf<unsigned> flags;  // cap: SEG_* bits
     DevBuf<unsigned short> Rh, Rl;  // cap x kpad BF16 bits: S x of the chains that reproject
@@ -87,10 +86,19 @@ struct DeferState {
     DevBuf<float> r;         // cap x ldz: r after each pass, FP32
     DevBuf<float> dxh, dxl;  // cap x ld: the passes' summed correction S^T z, double-float
     DevBuf<float> r0;        // cap: max|S x| of the chain when its check fired
+};
+
+struct DeferState {
+    long long ld = 0;        // leading dimension of the chain-major state (n rounded up to even)
+    int ldz = 0;             // leading dimension of Z and r (m rounded up to a multiple of 4)
+    int kpad = 0;            // K of the GEMM: m rounded up to a multiple of 64
+    bool exact32 = false;    // every coefficient of S is exact in FP32 (all lo parts zero)
+    Kept<DeferBufs> bufs;
     SlicedEll cols, rows;    // S^T and S; rows of S (and the row indices of S^T) in the device row order
     DevBuf<__nv_bfloat16> Bh, Bl;  // m x kpad: (S S^T)^+ split into hi + lo, rows and columns in the device row order
-    DevBuf<unsigned long long> any;  // one word per launch and pass: some chain needs that pass
-    int any_cap = 0;
+    Kept<DevBuf<unsigned long long>> any;  // one word per launch and pass: some chain needs that pass
+    int cap() const { return bufs.get() ? bufs.get()->cap : 0; }
+    int any_cap() const { return any.get() ? (int)any.get()->count : 0; }
     // Timing of the last run (only when requested): an event before and after every
     // chain-kernel launch, and one at the end.
     std::vector<cudaEvent_t> ev;
@@ -740,31 +748,36 @@ achr_status ensure_defer(achr_ctx *ctx, int chains, int segments) {
         if (st != ACHR_OK) return st;
         D = ctx->defer = nd.release();
     }
-    if (D->cap < chains) {
-        D->cap = 0;
+    if (D->cap() < chains) {
+        D->bufs.retire();
+        std::unique_ptr<DeferBufs> nb(new (std::nothrow) DeferBufs());
+        if (!nb) return set_err(ACHR_ERR_NOMEM, "allocation failed");
         const size_t c = (size_t)chains;
-        DEFER_TRY(D->x.alloc(c * (size_t)D->ld));
-        DEFER_TRY(D->A.alloc(c * (size_t)D->ld));
-        DEFER_TRY(D->flags.alloc(c));
-        DEFER_TRY(D->Rh.alloc(c * (size_t)D->kpad));
-        DEFER_TRY(D->Rl.alloc(c * (size_t)D->kpad));
+        DEFER_TRY(nb->x.alloc(c * (size_t)D->ld));
+        DEFER_TRY(nb->A.alloc(c * (size_t)D->ld));
+        DEFER_TRY(nb->flags.alloc(c));
+        DEFER_TRY(nb->Rh.alloc(c * (size_t)D->kpad));
+        DEFER_TRY(nb->Rl.alloc(c * (size_t)D->kpad));
         // the K padding of R (rows m..kpad) is never written and must be zero
-        DEFER_TRY(cudaMemset(D->Rh.p, 0, sizeof(unsigned short) * c * (size_t)D->kpad));
-        DEFER_TRY(cudaMemset(D->Rl.p, 0, sizeof(unsigned short) * c * (size_t)D->kpad));
-        DEFER_TRY(D->rd.alloc(c * (size_t)D->ldz));
-        DEFER_TRY(D->Z.alloc(c * (size_t)D->ldz));
-        DEFER_TRY(D->r.alloc(c * (size_t)D->ldz));
-        DEFER_TRY(D->dxh.alloc(c * (size_t)D->ld));
-        DEFER_TRY(D->dxl.alloc(c * (size_t)D->ld));
-        DEFER_TRY(D->r0.alloc(c));
+        DEFER_TRY(cudaMemset(nb->Rh.p, 0, sizeof(unsigned short) * c * (size_t)D->kpad));
+        DEFER_TRY(cudaMemset(nb->Rl.p, 0, sizeof(unsigned short) * c * (size_t)D->kpad));
+        DEFER_TRY(nb->rd.alloc(c * (size_t)D->ldz));
+        DEFER_TRY(nb->Z.alloc(c * (size_t)D->ldz));
+        DEFER_TRY(nb->r.alloc(c * (size_t)D->ldz));
+        DEFER_TRY(nb->dxh.alloc(c * (size_t)D->ld));
+        DEFER_TRY(nb->dxl.alloc(c * (size_t)D->ld));
+        DEFER_TRY(nb->r0.alloc(c));
         // (the memsets run on the default stream, which a non-blocking stream does not wait for)
         DEFER_TRY(cudaStreamSynchronize(nullptr));
-        D->cap = chains;
+        nb->cap = chains;
+        D->bufs.replace(std::move(nb));
     }
-    if (D->any_cap < segments) {
-        D->any_cap = 0;
-        DEFER_TRY(D->any.alloc((size_t)segments));
-        D->any_cap = segments;
+    if (D->any_cap() < segments) {
+        D->any.retire();
+        std::unique_ptr<DevBuf<unsigned long long>> na(new (std::nothrow) DevBuf<unsigned long long>());
+        if (!na) return set_err(ACHR_ERR_NOMEM, "allocation failed");
+        DEFER_TRY(na->alloc((size_t)segments));
+        D->any.replace(std::move(na));
     }
     return ACHR_OK;
 }
@@ -787,16 +800,6 @@ bool defer_selected(const achr_ctx *ctx) {
     return ctx->warmup_residual > o.residual_tol / 8.0;
 }
 
-// Reprojecting P chains in the chain kernel takes P 4 n d FP64 operations at every
-// check, deferring it about 0.1 ms of launches and passes, so the line lies at a
-// work of P n d.  Measured per 50 steps (five checks), in the kernel / deferred:
-//   n = 95, d = 20:    P = 1000 0.23 / 0.64 ms, 5000 0.75 / 1.18
-//   n = 200, d = 43:   P = 1000 0.49 / 0.82,    5000 1.85 / 1.58   (P n d = 8.6e6, 4.3e7)
-//   n = 400, d = 84:   P = 1000 1.08 / 0.87,    5000 5.19 / 2.23   (3.4e7, 1.7e8)
-//   n = 1060, d = 159: P = 1000 3.92 / 1.61,    5000 19.9 / 5.62
-// Models of n d >= 2.5e5 are always deferred.
-constexpr double kDeferWork = 2.0e7, kDeferModel = 2.5e5;
-
 namespace {
 
 int segments_of(const ChainArgs &a) { return (a.step0 + a.T) / a.check_period - a.step0 / a.check_period + 3; }
@@ -810,21 +813,18 @@ achr_status prepare(achr_ctx *ctx, const ChainArgs &a) {
 }  // namespace
 
 bool defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream) {
-    if (a.P <= 0 || a.T <= 0 || !defer_selected(ctx)) return false;
-    const double nd = (double)ctx->n * (double)ctx->d;
-    if (ctx->opt.reproject_form == 3 || nd >= kDeferModel) return true;
-    if ((double)a.P * nd < kDeferWork) return false;
-    // A model that could as well reproject in the kernel does so where the buffers
-    // cannot be had: their memory is short, or the stream is being captured (a
-    // capture allows no allocation).
-    const DeferState *D = ctx->defer;
-    if (D && ctx->reproj && D->cap >= std::min(a.P, kDeferChunk) && D->any_cap >= segments_of(a) * (kMaxPasses + 1))
-        return true;
+    if (a.P <= 0 || a.T <= 0) return false;
+    const DeferUse use = defer_use(defer_selected(ctx), ctx->opt.reproject_form == 3, (double)a.P,
+                                   (double)ctx->n * (double)ctx->d);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        (void)cudaGetLastError();
-        return false;
+    bool capturing = false;
+    if (use == DeferUse::kMay) {
+        capturing = cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+        if (capturing) (void)cudaGetLastError();
     }
+    if (!defer_run(use, capturing)) return false;
+    if (use == DeferUse::kAlways) return true;
+    // A model that could as well reproject in the kernel does so where memory for the buffers is short.
     if (prepare(ctx, a) == ACHR_OK) return true;
     (void)cudaGetLastError();
     return false;
@@ -839,6 +839,8 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
     const int cap = std::min(P, kDeferChunk);
     const int segments = segments_of(a_in);
     DeferState &D = *ctx->defer;
+    DeferBufs &U = *D.bufs.get();
+    unsigned long long *const any = D.any.get()->p;
     const ReprojState &R = *ctx->reproj;
     // One run at a time in the buffers.  A captured run has no event of its own (a graph may not wait
     // for work outside its capture): its replays are ordered against other runs by the program.
@@ -851,7 +853,10 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
             if (done) cudaEventRecord(done, s);
         }
     } turn{nullptr, s};
-    if (capture == cudaStreamCaptureStatusNone) {
+    if (capture != cudaStreamCaptureStatusNone) {
+        D.bufs.captured();
+        D.any.captured();
+    } else {
         if (D.done) DEFER_TRY(cudaStreamWaitEvent(s, D.done, 0));
         else DEFER_TRY(cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming));
         turn.done = D.done;
@@ -888,8 +893,8 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
     ctx->last_launches = 0;
     for (int c0 = 0; c0 < P; c0 += cap) {
         const int pc = std::min(cap, P - c0);
-        DEFER_TRY(cudaMemsetAsync(D.flags.p, 0, sizeof(unsigned) * (size_t)pc, s));
-        DEFER_TRY(cudaMemsetAsync(D.any.p, 0, sizeof(unsigned long long) * (size_t)segments * (kMaxPasses + 1), s));
+        DEFER_TRY(cudaMemsetAsync(U.flags.p, 0, sizeof(unsigned) * (size_t)pc, s));
+        DEFER_TRY(cudaMemsetAsync(any, 0, sizeof(unsigned long long) * (size_t)segments * (kMaxPasses + 1), s));
         ChainArgs a = a_in;
         a.P = pc;
         a.chain_offset = a_in.chain_offset + (unsigned long long)c0;
@@ -899,17 +904,17 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
         if (a_in.A_out) a.A_out = a_in.A_out + c0;
         a.pinv32 = nullptr;     // no reprojection inside the chain kernel
         a.seg = 1;
-        a.seg_x = D.x.p;
-        a.seg_A = D.A.p;
+        a.seg_x = U.x.p;
+        a.seg_A = U.A.p;
         a.ld_seg = D.ld;
-        a.seg_flags = D.flags.p;
-        a.seg_Rh = D.Rh.p;
-        a.seg_Rl = D.Rl.p;
+        a.seg_flags = U.flags.p;
+        a.seg_Rh = U.Rh.p;
+        a.seg_Rl = U.Rl.p;
         a.kpad = D.kpad;
-        a.seg_rd = D.rd.p;
+        a.seg_rd = U.rd.p;
         a.ld_r = D.ldz;
-        a.seg_dxh = D.dxh.p;
-        a.seg_dxl = D.dxl.p;
+        a.seg_dxh = U.dxh.p;
+        a.seg_dxl = U.dxl.p;
         const int pass_grid = (int)std::min<long long>((long long)sms * per_sm, (pc + pl.cpb - 1) / pl.cpb);
         const int pass1_grid = (int)std::min<long long>((long long)sms * per_sm1, (pc + pl.cpb1 - 1) / pl.cpb1);
         PassArgs pa{};
@@ -919,15 +924,15 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
         pa.P = pc;
         pa.ld = D.ld;
         pa.ldz = D.ldz;
-        pa.flags = D.flags.p;
-        pa.Z = D.Z.p;
-        pa.rd = D.rd.p;
-        pa.r = D.r.p;
-        pa.dxh = D.dxh.p;
-        pa.dxl = D.dxl.p;
-        pa.r0 = D.r0.p;
-        pa.Rh = reinterpret_cast<__nv_bfloat16 *>(D.Rh.p);
-        pa.Rl = reinterpret_cast<__nv_bfloat16 *>(D.Rl.p);
+        pa.flags = U.flags.p;
+        pa.Z = U.Z.p;
+        pa.rd = U.rd.p;
+        pa.r = U.r.p;
+        pa.dxh = U.dxh.p;
+        pa.dxl = U.dxl.p;
+        pa.r0 = U.r0.p;
+        pa.Rh = reinterpret_cast<__nv_bfloat16 *>(U.Rh.p);
+        pa.Rl = reinterpret_cast<__nv_bfloat16 *>(U.Rl.p);
         pa.cols = view(D.cols);
         pa.rows = view(D.rows);
         pa.fine_tol = (float)fine_tol;
@@ -943,7 +948,7 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
             a.step0 = s0;
             a.T = ends_on_check ? c - s0 + 1 : E - s0;
             a.seg_final = ends_on_check ? 0 : 1;
-            unsigned long long *gate = D.any.p + (size_t)seg * (kMaxPasses + 1);
+            unsigned long long *gate = any + (size_t)seg * (kMaxPasses + 1);
             a.seg_any = gate;  // pass 0 is needed when some chain's check fired
             DEFER_TRY(mark());
             DEFER_TRY(launch_chains(a, threads_per_chain, s));
@@ -952,8 +957,8 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
             ++ctx->last_launches;
             if (!ends_on_check) break;
             for (int pass = 0; pass < passes; ++pass) {
-                TcGemm g{pc, R.m, R.kpad, 3, D.Rh.p, D.Rl.p, (long long)R.kpad, D.Bh.p, D.Bl.p, (long long)R.kpad,
-                         D.Z.p, (long long)D.ldz};
+                TcGemm g{pc, R.m, R.kpad, 3, U.Rh.p, U.Rl.p, (long long)R.kpad, D.Bh.p, D.Bl.p, (long long)R.kpad,
+                         U.Z.p, (long long)D.ldz};
                 g.gate = gate + pass;  // skipped when no chain needs this pass
                 g.gate_max = 0;
                 if (const char *why = tc_gemm_check(g)) return set_err(ACHR_ERR_INVALID, why);
@@ -973,7 +978,7 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
                 a.step0 = E;
                 a.T = 0;
                 a.seg_final = 1;
-                a.seg_any = D.any.p + (size_t)seg * (kMaxPasses + 1);
+                a.seg_any = any + (size_t)seg * (kMaxPasses + 1);
                 DEFER_TRY(mark());
                 DEFER_TRY(launch_chains(a, threads_per_chain, s));
                 DEFER_TRY(mark());
