@@ -756,7 +756,13 @@ achr_status achr_sample_device(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
     }
     // Reprojections either inside the chain kernel, or deferred to a batched
     // tensor-core pass between segmented launches (achr_defer.cu).
-    const bool deferred = achr::defer_chosen(ctx, a, s);
+    bool deferred = false;
+    achr_status dst = achr::defer_chosen(ctx, a, s, &deferred);
+    if (dst != ACHR_OK) {
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+        return dst;
+    }
     if (ctx->opt.reproject_form == 3 && !deferred && n_points > 0 && n_steps > 0 && ctx->opt.check_period > 0 &&
         ctx->m > 0) {
         if (e0) cudaEventDestroy(e0);
@@ -766,7 +772,6 @@ achr_status achr_sample_device(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
                     "of S S^T of at most 2e4 (its BF16-split passes converge only then)");
     }
     cudaError_t e = cudaSuccess;
-    achr_status dst = ACHR_OK;
     if (deferred) dst = achr::defer_sample(ctx, a, ctx->opt.threads_per_chain, s, stats != nullptr);
     else e = achr::launch_chains(a, ctx->opt.threads_per_chain, s);
     if (e != cudaSuccess || dst != ACHR_OK) {
@@ -933,11 +938,11 @@ achr_status achr_sample_resume(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
         ACHR_CUDA_TRY(cudaEventCreate(&e1));
         ACHR_CUDA_TRY(cudaEventRecord(e0, s));
     }
-    const bool deferred = achr::defer_chosen(ctx, a, s);
+    bool deferred = false;
+    achr_status dst = achr::defer_chosen(ctx, a, s, &deferred);
     cudaError_t e = cudaSuccess;
-    achr_status dst = ACHR_OK;
     if (deferred) dst = achr::defer_sample(ctx, a, ctx->opt.threads_per_chain, s, stats != nullptr);
-    else e = achr::launch_chains(a, ctx->opt.threads_per_chain, s);
+    else if (dst == ACHR_OK) e = achr::launch_chains(a, ctx->opt.threads_per_chain, s);
     if (e != cudaSuccess || dst != ACHR_OK) {
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);

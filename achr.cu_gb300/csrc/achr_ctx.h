@@ -83,11 +83,11 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a, int threads_per_chai
 // After the stream of a timed defer_sample has completed: device time of its
 // chain-kernel launches and of its batched passes, and the chains per sweep.
 achr_status defer_times(achr_ctx *ctx, double *chain_ms, double *pass_ms, double *chains_per_sweep);
-// Whether sampling with these options may take the deferred path, and whether a
-// run of n_points chains described by `a` on `stream` does (deferred sampling's
+// Whether sampling with these options may take the deferred path, and whether the
+// run described by `a` on `stream` does (achr_defer_rule.h; deferred sampling's
 // buffers are then ready, or will be built by defer_sample).
 bool defer_selected(const achr_ctx *ctx);
-bool defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream);
+achr_status defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream, bool *deferred);
 }  // namespace achr
 
 struct achr_ctx {
@@ -121,6 +121,7 @@ struct achr_ctx {
     achr::DevBuf<float> pinv32;            // (S S^T)^+ in FP32, device row order, m x m (empty: not built)
     achr::DevBuf<unsigned long long> counters;
     achr::ReprojState *reproj = nullptr;  // batched reprojection operator, built on first use
+    int defer_short_from = 0;  // chains from which the deferred buffers could not be had (0: none so far)
     achr::DeferState *defer = nullptr;    // buffers of segmented sampling, built on first use
     double warmup_residual = 0.0;         // max |S w|_inf over the warmup points (as sampled)
     double kappa_sst = 1.0;               // condition number of S S^T on its range (from the null-space set-up)

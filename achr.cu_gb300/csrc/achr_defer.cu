@@ -812,22 +812,33 @@ achr_status prepare(achr_ctx *ctx, const ChainArgs &a) {
 
 }  // namespace
 
-bool defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream) {
-    if (a.P <= 0 || a.T <= 0) return false;
+achr_status defer_chosen(achr_ctx *ctx, const ChainArgs &a, cudaStream_t stream, bool *deferred) {
+    *deferred = false;
+    if (a.P <= 0 || a.T <= 0) return ACHR_OK;
     const DeferUse use = defer_use(defer_selected(ctx), ctx->opt.reproject_form == 3, (double)a.P,
                                    (double)ctx->n * (double)ctx->d);
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     bool capturing = false;
     if (use == DeferUse::kMay) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         capturing = cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
         if (capturing) (void)cudaGetLastError();
     }
-    if (!defer_run(use, capturing)) return false;
-    if (use == DeferUse::kAlways) return true;
-    // A model that could as well reproject in the kernel does so where memory for the buffers is short.
-    if (prepare(ctx, a) == ACHR_OK) return true;
-    (void)cudaGetLastError();
-    return false;
+    achr_status st = ACHR_OK;
+    const DeferChoice c = defer_choose(use, capturing, std::min(a.P, kDeferChunk), ctx->defer_short_from, [&] {
+        (void)cudaGetLastError();
+        try {
+            st = prepare(ctx, a);
+        } catch (const std::bad_alloc &) {
+            st = set_err(ACHR_ERR_NOMEM, "allocation failed");
+        }
+        if (st == ACHR_OK) return DeferBuffers::kReady;
+        if (cudaGetLastError() != cudaErrorMemoryAllocation && st != ACHR_ERR_NOMEM) return DeferBuffers::kFailed;
+        defer_free(ctx->defer);  // (whatever of it was had: the kernel needs none of it)
+        ctx->defer = nullptr;
+        return DeferBuffers::kNoMemory;
+    });
+    *deferred = c.deferred;
+    return c.failed ? st : ACHR_OK;
 }
 
 achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_chain, cudaStream_t s, bool timed) {

@@ -26,11 +26,27 @@ inline DeferUse defer_use(bool selected, bool asked, double chains, double nd) {
     return chains * nd >= kDeferWork ? DeferUse::kMay : DeferUse::kKernel;
 }
 
-// Whether the run is deferred.  A captured run that need not be stays in the kernel, whether or not
-// buffers exist: its graph then holds no buffer that the context may replace, and what a capture gives
-// does not depend on the calls before it.
-inline bool defer_run(DeferUse use, bool capturing) {
-    return use == DeferUse::kAlways || (use == DeferUse::kMay && !capturing);
+enum class DeferBuffers { kReady, kNoMemory, kFailed };
+
+struct DeferChoice {
+    bool deferred, failed;
+};
+
+// Whether a run of `chains` chains is deferred.  A captured run that need not be stays in the kernel,
+// whether or not buffers exist: its graph then holds no buffer that the context may replace, and what a
+// capture gives does not depend on the calls before it.  Where there is no memory for the buffers
+// (prepare) a run that need not be deferred stays in the kernel too, and so does every later run of the
+// context of that size or more (short_from, 0 at first): a run continued in segments keeps its form, and
+// memory is not asked for at every call.  Any other failure is the call's.
+template <class Prepare>
+DeferChoice defer_choose(DeferUse use, bool capturing, int chains, int &short_from, Prepare prepare) {
+    if (use == DeferUse::kAlways) return {true, false};
+    if (use == DeferUse::kKernel || capturing || (short_from > 0 && chains >= short_from)) return {false, false};
+    switch (prepare()) {
+        case DeferBuffers::kReady: return {true, false};
+        case DeferBuffers::kNoMemory: short_from = chains; return {false, false};
+        default: return {false, true};
+    }
 }
 
 }  // namespace achr

@@ -14,7 +14,25 @@ WRAPPER = r"""
 #include "achr_defer_rule.h"
 #include "achr_kept.h"
 extern "C" int rule(int selected, int asked, double chains, double nd, int capturing) {
-    return achr::defer_run(achr::defer_use(selected, asked, chains, nd), capturing);
+    int short_from = 0;
+    return achr::defer_choose(achr::defer_use(selected, asked, chains, nd), capturing, (int)chains, short_from,
+                              [] { return achr::DeferBuffers::kReady; }).deferred;
+}
+// A context's runs one after another: chains of each, and what asking for its buffers would give ('r' ready,
+// 'm' no memory, 'x' another failure).  What each did: 'd' deferred, 'k' in the kernel, 'e' an error; in
+// upper case if the buffers were asked for.
+extern "C" void runs(int n, const int *chains, const char *buffers, char *did) {
+    int short_from = 0;
+    for (int i = 0; i < n; ++i) {
+        bool asked = false;
+        const achr::DeferChoice c = achr::defer_choose(achr::DeferUse::kMay, false, chains[i], short_from, [&] {
+            asked = true;
+            return buffers[i] == 'r'   ? achr::DeferBuffers::kReady
+                   : buffers[i] == 'm' ? achr::DeferBuffers::kNoMemory
+                                       : achr::DeferBuffers::kFailed;
+        });
+        did[i] = (c.failed ? 'e' : c.deferred ? 'd' : 'k') - (asked ? 32 : 0);
+    }
 }
 static int alive;
 struct Buf {
@@ -51,6 +69,7 @@ def lib(tmp_path_factory):
                     "-o", str(d / "librule.so")], check=True)
     so = C.CDLL(str(d / "librule.so"))
     so.rule.argtypes = [C.c_int, C.c_int, C.c_double, C.c_double, C.c_int]
+    so.runs.argtypes = [C.c_int, C.POINTER(C.c_int), C.c_char_p, C.c_char_p]
     so.kept.argtypes = [C.c_char_p]
     return so
 
@@ -64,6 +83,19 @@ def lib(tmp_path_factory):
 ])
 def test_line(lib, selected, asked, chains, nd, capturing, deferred):
     assert lib.rule(selected, asked, chains, nd, capturing) == deferred
+
+
+@pytest.mark.parametrize("chains,buffers,did", [
+    ([100, 100], "rr", "DD"),
+    ([100, 100, 100], "mrr", "Kkk"),            # short once: every later run of that size stays in the kernel
+    ([100, 200, 50, 100], "mrrr", "KkDk"),      # and the larger ones; smaller ones are asked for
+    ([100, 50, 70, 20], "mmrr", "KKkD"),
+    ([100, 100], "xr", "ED"),                   # any other failure is the call's, and not remembered
+])
+def test_memory_short(lib, chains, buffers, did):
+    out = C.create_string_buffer(len(chains) + 1)
+    lib.runs(len(chains), (C.c_int * len(chains))(*chains), buffers.encode(), out)
+    assert out.value.decode() == did
 
 
 @pytest.mark.parametrize("steps,left", [("", 0), ("g", 1), ("gg", 1), ("ggg", 1), ("c", 0), ("gc", 1), ("gcg", 2),
