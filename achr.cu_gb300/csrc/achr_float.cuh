@@ -19,7 +19,8 @@ __device__ __forceinline__ float f64_to_f32_rz(double v) {
     return __uint_as_float((hi & 0x80000000u) | mag);
 }
 
-// FP64 -> FP32 rounding to nearest (ties away from zero), otherwise like f64_to_f32_rz.
+// FP64 -> FP32 rounding to nearest (ties away from zero), otherwise like f64_to_f32_rz; not for NaN
+// (its fraction's carry can reach the sign).
 __device__ __forceinline__ float f64_to_f32_near(double v) {
     return f64_to_f32_rz(__longlong_as_double(__double_as_longlong(v) + (1ll << 28)));
 }
@@ -62,6 +63,21 @@ __device__ __forceinline__ void split_bf16_bits(float f, unsigned short &hi, uns
     const unsigned r = __float_as_uint(f - __uint_as_float(hu));
     const unsigned ru = (r + 0x7FFFu + ((r >> 16) & 1u)) & 0xFFFF0000u;
     lo = (unsigned short)(ru >> 16);
+}
+
+// BF16 bits of v (hi) and of the remainder v - hi (lo), as the conversions would give them for any v:
+// beyond BF16's range hi is infinite and lo the opposite infinity, of an infinite v hi is infinite and lo
+// NaN, of NaN both are NaN, so that a product with hi and lo is NaN and not a finite or infinite value.
+__device__ __forceinline__ void split_bf16_any(double v, unsigned short &hi, unsigned short &lo) {
+    const unsigned top = (unsigned)__double2hiint(v) & 0x7FFFFFFFu;
+    if (top < 0x47EFFFFFu) {  // below 2^128 (1 - 2^-20)
+        split_bf16_bits(f64_to_f32_near(v), hi, lo);
+        return;
+    }
+    const unsigned sign = ((unsigned)__double2hiint(v) >> 16) & 0x8000u;
+    const bool finite = top < 0x7FF00000u, nan = !finite && (top > 0x7FF00000u || __double2loint(v) != 0);
+    hi = (unsigned short)(nan ? 0x7FFFu : sign | 0x7F80u);
+    lo = (unsigned short)(finite ? (sign ^ 0x8000u) | 0x7F80u : 0x7FFFu);
 }
 
 // Error-free transformations on FP32 (IEEE round-to-nearest; nvcc neither

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32)
 #pragma unroll
             for (int u = 0; u < kSplitLoads; ++u) {
                 unsigned short h, l;
-                split_bf16_bits(f64_to_f32_near(mu ? x[u] - m[u] : x[u]), h, l);
+                split_bf16_any(mu ? x[u] - m[u] : x[u], h, l);
                 stage[warp][0][lane * kSplitStride + r + u] = h;
                 stage[warp][1][lane * kSplitStride + r + u] = l;
             }
