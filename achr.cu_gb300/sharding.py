@@ -2,8 +2,12 @@
 
 Chains are independent and every random draw is keyed by (seed, chain id, step,
 attempt), so a rank that samples chain ids [offset, offset + count) produces
-exactly the columns a single process would produce for those ids.  The data
-path therefore has no collective; the only collectives are the barrier around
+the columns a single process would produce for those ids: bit for bit when both
+reproject the same way, as they do unless reproject_form is 0 and the warmup
+points carry a residual (a %f CSV).  There the library defers the reprojections
+of a call from chains x n_rxns x null_dim = 2e7 on, so a rank's smaller call may
+take another form than the whole, and its points then differ by rounding; name
+the form (1 or 3) where the split must not show.  The data path therefore has no collective; the only collectives are the barrier around
 the timed region and the maximum of the per-rank times (the job is as slow as
 its slowest rank).  The reference runs one process on one GPU (its chains are
 ACHRcu/ACHRCuda.cu:741's grid over nPoints); this is the weak-scaling split of

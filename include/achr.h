@@ -88,7 +88,14 @@ typedef struct {
                                     in the chain kernel, as 2 when
                                     n_rxns x null_dim >= 4e6, else as 1; always as 1 where the basis in
                                     use is not an orthonormal basis of null(S) (a caller's subspace,
-                                    ACHR_NULL_FIXED with blocked reactions),
+                                    ACHR_NULL_FIXED with blocked reactions).  Below n_rxns x null_dim =
+                                    2.5e5 a run on such warmup points is thus deferred or not by its number
+                                    of chains, and it is not while its stream is being captured, nor once
+                                    the context has been short of memory for as many chains; the forms
+                                    agree to rounding, not bit for bit, so name 1 or 3 where a chain's
+                                    points must not depend on how chains are split over calls.  Deferred
+                                    runs of one context take turns; their buffers, about 24 n_rxns +
+                                    20 n_mets bytes per chain, stay with it,
                                  1: N (N^T x) in FP64 in the chain kernel,
                                  2: x - S^T (S S^T)^+ S x in the chain kernel, the pseudo-inverse product
                                     in FP32 on the residual (equal in exact arithmetic; m^2 FP32 instead
@@ -205,7 +212,7 @@ achr_status achr_sample_device(achr_ctx *ctx, uint64_t seed, uint64_t chain_offs
  * both as the state after step0 steps and overwrites them with the state
  * after step0 + n_steps.  Running T1 then T2 steps this way gives the same
  * points as one launch of T1 + T2 steps (the random stream is keyed by the
- * global step index), except in ACHR_MODE_FEASIBLE, where every segment ends
+ * global step index; with reproject_form 0 under the conditions stated there), except in ACHR_MODE_FEASIBLE, where every segment ends
  * with the feasibility projection.  Queued on `stream`; stats synchronise. */
 achr_status achr_sample_resume(achr_ctx *ctx, uint64_t seed, uint64_t chain_offset, int32_t n_points, int32_t step0,
                                int32_t n_steps, int32_t resume, double *d_points, double *d_centre_acc, int64_t ld,
@@ -401,7 +408,8 @@ typedef struct {
  * first.  Model k runs n_points[k] chains of n_steps into d_points_out[k]
  * (device, n_k x P_k, leading dimension ld_out[k]); its chain ids start at the
  * sum of the earlier models' n_points, so achr_sample_device on model k alone
- * with that chain_offset gives the same points.  Synchronises `stream`;
+ * with that chain_offset gives the same points (where it reprojects in the chain
+ * kernel as well; batched launches always do, see reproject_form).  Synchronises `stream`;
  * per-model finish times (ms from the launch) go to model_ms_out[k] if
  * non-NULL. */
 achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int32_t *n_points, int32_t n_steps,
