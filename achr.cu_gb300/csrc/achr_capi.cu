@@ -986,7 +986,8 @@ void achr_destroy(achr_ctx *ctx) {
 
 namespace {
 
-// Autotuning results per (default padded length, device): threads per chain.
+// Autotuning results per (default padded length, long scratch or not, residual form or not; device):
+// threads per chain.
 std::mutex g_tune_mutex;
 std::map<std::pair<int, int>, int> g_tune_cache;
 // Guided self-scheduling of the batched work queues: an item holds the work
@@ -1011,11 +1012,21 @@ achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out) {
     if (!ctx) return fail(ACHR_ERR_INVALID, "ctx is NULL");
     int dev = 0;
     ACHR_CUDA_TRY(cudaGetDevice(&dev));
-    // A context that reprojects through the residual in the kernel takes only
-    // configurations that leave it room (the others would fall back to N (N^T x)).
-    ChainArgs probe = chain_args(ctx, 0, 0, 0, 0, nullptr, 0);
+    // Candidates are the thread counts this context can launch with: the configuration must hold its
+    // reprojection's scratch (max(m, d) doubles) and, where the context reprojects through the residual
+    // in the kernel, leave that form room (it would fall back to N (N^T x)).
+    const ChainArgs probe = chain_args(ctx, 0, 0, 0, 0, nullptr, 0);
     const bool residual = probe.pinv32 && ctx->opt.check_period > 0;
-    const std::pair<int, int> key(2 * achr::chain_padded_length(ctx->n, 0) + (residual ? 1 : 0), dev);
+    auto takes = [&](int threads) {
+        int per_sm = 0;
+        const cudaError_t e = achr::launch_chains(probe, threads, nullptr, 0, &per_sm);
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return e == cudaSuccess && (!residual || per_sm > 0);
+    };
+    const int scratch = std::max(probe.m, probe.d);
+    const bool long_scratch = scratch > achr::chain_scratch_doubles(256, 30);
+    const std::pair<int, int> key(4 * achr::chain_padded_length(ctx->n, 0) + (long_scratch ? 2 : 0) + (residual ? 1 : 0),
+                                  dev);
     int cand[8];
     int nc = 0;
     {
@@ -1026,14 +1037,13 @@ achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out) {
             nc = 1;
         }
     }
+    // (a model of the same length may have had another scratch)
+    if (nc == 1 && !takes(cand[0])) nc = 0;
     if (nc == 0) {
-        nc = achr::chain_candidates(ctx->n, ctx->np, cand, 8);
+        nc = achr::chain_candidates(ctx->n, ctx->np, scratch, cand, 8);
         int kept = 0;
-        for (int c = 0; c < nc && residual; ++c) {
-            int per_sm = 0;
-            ACHR_CUDA_TRY(achr::launch_chains(probe, cand[c], nullptr, 0, &per_sm));
-            if (per_sm > 0) cand[kept++] = cand[c];
-        }
+        for (int c = 0; c < nc && residual; ++c)
+            if (takes(cand[c])) cand[kept++] = cand[c];
         if (kept > 0) nc = kept;
     }
     if (nc == 0) return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration to tune");

@@ -130,12 +130,13 @@ int chain_alloc_length(int n) {
     return np * 2 > 16384 ? np : np * 2;
 }
 
-int chain_candidates(int n, int max_np, int *bds, int cap) {
+int chain_candidates(int n, int max_np, int scratch, int *bds, int cap) {
     const int np0 = chain_padded_length(n, 0);
     int k = 0;
     for (const Cfg &c : kLadder) {
         const int np = c.bd * c.ept;
         if (np < n || np > max_np || np > 2 * np0) continue;
+        if (c.bd == 256 && c.ept == 30 && scratch > kScratch256x30) continue;
         bool dup = false;
         for (int j = 0; j < k; ++j) dup |= bds[j] == c.bd;
         if (dup || chain_padded_length(n, c.bd) != np) continue;

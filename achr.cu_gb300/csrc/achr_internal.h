@@ -191,8 +191,9 @@ int chain_padded_length(int n, int threads_per_chain);
 // Length to pad per-reaction arrays to: twice the default padded length (so
 // every autotuning candidate fits), at most 16384.
 int chain_alloc_length(int n);
-// Threads-per-chain values worth timing for n (padded length within max_np).
-int chain_candidates(int n, int max_np, int *bds, int cap);
+// Threads-per-chain values worth timing for n (padded length within max_np), of
+// the configurations that hold a reprojection's scratch (max(m, d) doubles).
+int chain_candidates(int n, int max_np, int scratch, int *bds, int cap);
 
 // Tensor-core GEMM (achr_tc_gemm.cu): C (M x N, FP32, row-major, ldc) =
 // A0 B0^T (nsplit 1) or A0 B0^T + A0 B1^T + A1 B0^T (nsplit 3); operands BF16

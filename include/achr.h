@@ -382,8 +382,8 @@ achr_status achr_gemm_bf16(int32_t M, int32_t N, int32_t K, int32_t nsplit, cons
 
 /* Time the chain kernel's candidate configurations (threads per chain x
  * reactions per thread) on a short run of this context and keep the fastest in
- * its options; the choice is cached per padded model size and device for the
- * rest of the process.  Writes the chosen threads per chain if non-NULL. */
+ * its options; the choice is cached per padded model size, kind of reprojection
+ * and device for the rest of the process.  Writes the chosen threads per chain if non-NULL. */
 achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out);
 
 typedef struct {
