@@ -10,6 +10,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <new>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -697,12 +698,15 @@ achr_status achr_create(const achr_model *model, const double *warmup, int32_t n
     ACHR_CUDA_TRY(ctx->A0.alloc(np));
     st = prepare_warmup_and_centre(ctx);
     if (st != ACHR_OK) return st;
-    // Sampling on these warmup points will need the reprojection operator: build it
-    // while the eigenvectors are here (on first use it takes a decomposition of its own,
-    // which for a small model is milliseconds).
+    // Sampling on these warmup points will need the reprojection operator (a small model's where a run is
+    // long enough to be deferred): build it while the eigenvectors are here, 5 to 7 % of this call; on
+    // first use it takes a decomposition of its own, which for a small model is milliseconds.  Only an
+    // early start: a context is complete without it, and a run that needs it builds it or says why not.
     if (rows && achr::defer_selected(ctx) && (double)n * (double)d >= 1.0e4) {
-        st = achr::build_operator(ctx, false, rows);
-        if (st != ACHR_OK) return st;
+        try {
+            if (achr::build_operator(ctx, false, rows) != ACHR_OK) (void)cudaGetLastError();
+        } catch (const std::bad_alloc &) {
+        }
     }
 
     owned = nullptr;  // release from the guard

@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -422,15 +423,11 @@ achr_status build_reproj(achr_ctx *ctx, ReprojState &R, bool want_pinv32, const 
 
 achr_status ensure_reproj(achr_ctx *ctx) {
     if (ctx->reproj) return ACHR_OK;
-    ReprojState *R = new (std::nothrow) ReprojState();
+    std::unique_ptr<ReprojState> R(new (std::nothrow) ReprojState());
     if (!R) return set_err(ACHR_ERR_NOMEM, "allocation failed");
     const achr_status st = build_reproj(ctx, *R, false, nullptr);
-    if (st != ACHR_OK) {
-        delete R;
-        return st;
-    }
-    ctx->reproj = R;
-    return ACHR_OK;
+    if (st == ACHR_OK) ctx->reproj = R.release();
+    return st;
 }
 
 namespace {
@@ -464,15 +461,12 @@ dim3 residual_grid(int P, int kpad) {
 achr_status build_operator(achr_ctx *ctx, bool want_pinv32, const RowSpace *eig) {
     if (ctx->reproj && (!want_pinv32 || ctx->pinv32.p)) return ACHR_OK;
     if ((int)ctx->h_row_order.size() != ctx->m) return set_err(ACHR_ERR_INVALID, "row order missing");
-    ReprojState *R = new (std::nothrow) ReprojState();
+    std::unique_ptr<ReprojState> R(new (std::nothrow) ReprojState());
     if (!R) return set_err(ACHR_ERR_NOMEM, "allocation failed");
     const achr_status st = build_reproj(ctx, *R, want_pinv32, eig);
-    if (st != ACHR_OK) {
-        delete R;
-        return st;
-    }
+    if (st != ACHR_OK) return st;
     reproj_free(ctx->reproj);
-    ctx->reproj = R;
+    ctx->reproj = R.release();
     return ACHR_OK;
 }
 
