@@ -52,6 +52,8 @@ ACHR_DIV_HD float div_rcp(float x) {  // relative error below 2^-21 suffices
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+#elif defined(ACHR_DIV_RCP)  // (another one, for a test of the bound)
+    return ACHR_DIV_RCP(x);
 #else
     return 1.0f / x;
 #endif
