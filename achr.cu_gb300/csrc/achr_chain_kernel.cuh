@@ -1558,6 +1558,15 @@ __global__ void __launch_bounds__(BD, (chain_min_ctas<BD, EPT>())) achr_chain_qu
     if (threadIdx.x == 0 && q.cta_ns) q.cta_ns[blockIdx.x] = global_ns();
 }
 
+// Lets a kernel be launched with `need` bytes of dynamic shared memory.  The limit belongs to the
+// function, not to the launch: set to a launch's own need it fails another thread's launch that needs
+// more, so it is always the same one (what a CTA may have, less 1 KB for static arrays).
+inline cudaError_t allow_smem(const void *kernel, size_t need) {
+    constexpr size_t kMost = 226 * 1024;
+    if (need > kMost) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
+}
+
 // Occupancy-sized persistent launch of one configuration.  max_ctas > 0 caps
 // the grid.
 template <int BD, int EPT, bool SEG>
@@ -1576,8 +1585,7 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
     if (a.pinv32 && a.m > a.ldw) a.pinv32 = nullptr;
     const bool asked = a.pinv32 != nullptr;
     size_t smem = base + (a.pinv32 ? zbytes : 0);
-    cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::max(smem, base));
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(KFN), std::max(smem, base));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KFN, BD, base);
@@ -1614,7 +1622,7 @@ template <int BD, int EPT>
 cudaError_t launch_queue_cfg(const ChainQueue &q, cudaStream_t stream, int grid, int *per_sm_out) {
     auto *const KFN = achr_chain_queue_kernel<BD, EPT>;
     const size_t smem = chain_smem_bytes_cfg<BD, EPT>() + q.extra_smem;
-    cudaError_t e = cudaFuncSetAttribute(KFN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(KFN), smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KFN, BD, smem);

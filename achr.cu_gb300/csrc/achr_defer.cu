@@ -893,8 +893,9 @@ achr_status defer_sample(achr_ctx *ctx, const ChainArgs &a_in, int threads_per_c
     const PassPlan pl = plan_passes(D.ld, D.ldz, D.exact32);
     if (pl.smem1 > kPassSmemMax || pl.smem > kPassSmemMax)
         return set_err(ACHR_ERR_UNSUPPORTED, "model too large for the batched reprojection's shared memory");
-    DEFER_TRY(cudaFuncSetAttribute(pl.pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-    DEFER_TRY(cudaFuncSetAttribute(pl.pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem1));
+    // (one limit for every model: it belongs to the function, and another thread may be between these and its launch)
+    DEFER_TRY(cudaFuncSetAttribute(pl.pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemMax));
+    DEFER_TRY(cudaFuncSetAttribute(pl.pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemMax));
     DEFER_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pl.pass, kPassThreads, pl.smem));
     DEFER_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm1, pl.pass1, kPassThreads, pl.smem1));
     if (per_sm < 1 || per_sm1 < 1)
