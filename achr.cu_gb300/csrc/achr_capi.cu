@@ -719,7 +719,11 @@ achr_status achr_set_null_space(achr_ctx *ctx, const double *N, int32_t d) {
     if (!ctx || (!N && d > 0) || d < 0 || d > ctx->n) return fail(ACHR_ERR_INVALID, "bad null-space arguments");
     ctx->basis_spans = false;
     achr_status st = upload_null_space(ctx, N, d);
-    if (st == ACHR_OK) st = spans_null_space(ctx, ctx->basis_spans);
+    // (without memory for the check the basis is not shown to span null(S): N (N^T x) is right for any)
+    if (st == ACHR_OK && spans_null_space(ctx, ctx->basis_spans) != ACHR_OK) {
+        (void)cudaGetLastError();
+        ctx->basis_spans = false;
+    }
     if (st != ACHR_OK || ctx->opt.mode != ACHR_MODE_FEASIBLE) return st;
     return prepare_warmup_and_centre(ctx);  // re-project the warmup points onto the new basis
 }
