@@ -25,6 +25,17 @@ __device__ __forceinline__ float f64_to_f32_near(double v) {
     return f64_to_f32_rz(__longlong_as_double(__double_as_longlong(v) + (1ll << 28)));
 }
 
+// The same for any v, NaN giving an infinity: its exponent is looked at before the rounding.
+__device__ __forceinline__ float f64_to_f32_near_any(double v) {
+    const long long b = __double_as_longlong(v) + (1ll << 28);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32), lo = (unsigned)b, was = (unsigned)__double2hiint(v);
+    const int fe = (int)((hi >> 20) & 0x7FFu) - 896;
+    unsigned mag = ((unsigned)fe << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+    mag = (fe <= 0) ? 0u : mag;
+    mag = (fe >= 255 || (was & 0x7FF00000u) == 0x7FF00000u) ? 0x7F800000u : mag;
+    return __uint_as_float((was & 0x80000000u) | mag);
+}
+
 // Order-preserving integer key of a double (sign-magnitude -> two's
 // complement; -0 and +0 share key 0).  a < b  <=>  key(a) < key(b) for non-NaN.
 __device__ __forceinline__ long long order_key(double v) {
@@ -65,15 +76,14 @@ __device__ __forceinline__ void split_bf16_bits(float f, unsigned short &hi, uns
     lo = (unsigned short)(ru >> 16);
 }
 
-// BF16 bits of v (hi) and of the remainder v - hi (lo), as the conversions would give them for any v:
-// beyond BF16's range hi is infinite and lo the opposite infinity, of an infinite v hi is infinite and lo
-// NaN, of NaN both are NaN, so that a product with hi and lo is NaN and not a finite or infinite value.
-__device__ __forceinline__ void split_bf16_any(double v, unsigned short &hi, unsigned short &lo) {
+// High word of the smallest magnitude whose split is not that of the conversions, about 2^128 (1 - 2^-20):
+// from there BF16 rounds to infinity, and an infinity or NaN comes out as an infinity and -0, or as 0.
+constexpr unsigned kSplitTop = 0x47EFFFFFu;
+
+// The split of such a value as the conversions give it: hi infinite and lo the opposite infinity; of an
+// infinity hi infinite and lo NaN; of NaN both NaN.  A product with hi and lo is NaN.
+__device__ __forceinline__ void split_bf16_top(double v, unsigned short &hi, unsigned short &lo) {
     const unsigned top = (unsigned)__double2hiint(v) & 0x7FFFFFFFu;
-    if (top < 0x47EFFFFFu) {  // below 2^128 (1 - 2^-20)
-        split_bf16_bits(f64_to_f32_near(v), hi, lo);
-        return;
-    }
     const unsigned sign = ((unsigned)__double2hiint(v) >> 16) & 0x8000u;
     const bool finite = top < 0x7FF00000u, nan = !finite && (top > 0x7FF00000u || __double2loint(v) != 0);
     hi = (unsigned short)(nan ? 0x7FFFu : sign | 0x7F80u);

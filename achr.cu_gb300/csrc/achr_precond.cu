@@ -271,12 +271,25 @@ __global__ void __launch_bounds__(kSplitWarps * 32)
                 m[u] = mu ? __ldg(mu + ii) : 0.0;
                 if (i >= n) x[u] = m[u] = 0.0;
             }
+            unsigned top = 0;  // largest magnitude (high words): one branch for the eight
 #pragma unroll
             for (int u = 0; u < kSplitLoads; ++u) {
                 unsigned short h, l;
-                split_bf16_any(mu ? x[u] - m[u] : x[u], h, l);
+                if (mu) x[u] -= m[u];
+                top = max(top, (unsigned)__double2hiint(x[u]) & 0x7FFFFFFFu);
+                split_bf16_bits(f64_to_f32_near(x[u]), h, l);
                 stage[warp][0][lane * kSplitStride + r + u] = h;
                 stage[warp][1][lane * kSplitStride + r + u] = l;
+            }
+            if (top >= kSplitTop) {
+#pragma unroll
+                for (int u = 0; u < kSplitLoads; ++u) {
+                    unsigned short h, l;
+                    if (((unsigned)__double2hiint(x[u]) & 0x7FFFFFFFu) < kSplitTop) continue;
+                    split_bf16_top(x[u], h, l);
+                    stage[warp][0][lane * kSplitStride + r + u] = h;
+                    stage[warp][1][lane * kSplitStride + r + u] = l;
+                }
             }
         }
         __syncwarp();

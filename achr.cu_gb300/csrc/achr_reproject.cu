@@ -131,8 +131,10 @@ __global__ void __launch_bounds__(kResWarps * 32)
             }
             if (live) mx = max(mx, abs_bits64(acc));
             if (SPLIT) {
+                // (a residual beyond BF16's range, infinite or NaN: hi is infinite, every z of the chain infinite
+                // or NaN, and the correction, whose error terms subtract infinities, NaN)
                 unsigned short h, l;
-                split_bf16_any(acc, h, l);
+                split_bf16_bits(f64_to_f32_near_any(acc), h, l);
                 sh[lane * kStageStride + r] = h;
                 sl[lane * kStageStride + r] = l;
             }
@@ -208,15 +210,8 @@ __global__ void __launch_bounds__(kCorrWarps * 32)
         double *xp = X + (long long)j * ldx + p;
         const double xo = *xp;
         double d;
-        if (fabsf(ah) + fabsf(al) < INFINITY) {
-            d = f32_to_f64_exact(ah) + f32_to_f64_exact(al);
-        } else {  // NaN, or beyond FP32's range on the way: the sum in FP64
-            d = 0.0;
-            for (int q = __ldg(cp + j); q < q1; ++q) {
-                const double v = EXACT32 ? (double)__ldg(ch + q) : (double)__ldg(ch + q) + (double)__ldg(cl + q);
-                d = fma(v, (double)__ldg(zp + (long long)__ldg(ri + q) * ldz), d);
-            }
-        }
+        if (fabsf(ah) + fabsf(al) < INFINITY) d = f32_to_f64_exact(ah) + f32_to_f64_exact(al);
+        else d = (double)ah + (double)al;  // NaN, or beyond FP32's range: NaN
         const double xc = xo - d;
         const double xn = abs_bits64(xc) > 0x7FF0000000000000ull ? xc : clip_exact(xc, lbub[j]);
         *xp = xn;
