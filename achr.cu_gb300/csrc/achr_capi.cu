@@ -58,7 +58,6 @@ void f32_bound(double v, float &f, float &err) {
     err = ef;
 }
 
-using achr::f32_down;
 using achr::f32_up;
 
 // Writes the global nanosecond timer (used to time each model's branch of a
@@ -431,8 +430,8 @@ achr_status deferred_stats(achr_ctx *ctx, bool deferred, achr_stats *stats) {
 achr_status read_counters(achr_ctx *ctx, achr_stats *stats, float ms) {
     unsigned long long c[achr::CNT_SLOTS];
     ACHR_CUDA_TRY(cudaMemcpy(c, ctx->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
-    if (c[achr::CNT_ERROR] & achr::ERR_TMA_TIMEOUT)
-        return fail(ACHR_ERR_TIMEOUT, "a warmup-column copy did not complete within its wait limit");
+    if (c[achr::CNT_ERROR] & achr::ERR_WAIT_TIMEOUT)
+        return fail(ACHR_ERR_TIMEOUT, "the chain kernel's bounded wait ran out");
     if (c[achr::CNT_ERROR] & achr::ERR_TC_TIMEOUT)
         return fail(ACHR_ERR_TIMEOUT, "a tensor-core pipeline wait of the batched reprojection expired");
     if (c[achr::CNT_ERROR] & achr::ERR_DEFER_DIVERGED)
@@ -824,7 +823,6 @@ ChainArgs chain_args(const achr_ctx *ctx, uint64_t seed, uint64_t chain_offset, 
     a.bound_err = ctx->bound_err;
     a.bound_exact = ctx->bound_exact ? 1 : 0;
     a.dtol_hi = f32_up(ctx->opt.d_tol) * (1.0f + 9.5367431640625e-07f);
-    a.dtol_lo = f32_down(ctx->opt.d_tol) * (1.0f - 9.5367431640625e-07f);
     a.utol32 = (float)ctx->opt.u_tol;
     a.mmt32 = (float)ctx->opt.max_min_tol;
     set_merged_bound(a, ctx->opt.u_tol, ctx->opt.bracket_pass == 1 ? INFINITY

@@ -68,7 +68,7 @@ constexpr float kDCert = 1.5777218104420236e-30f;      // 2^-99: no smaller |d| 
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bounded mbarrier wait: 2 s
 constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 
-// The same for the hot loops, in six integer operations: the magnitude is
+// FP64 -> FP32 for the hot loops, in six integer operations: the magnitude is
 // clamped to [2^LO_EXP, 2^128 (1 - 2^-20)) in its FP64 form (three spare low
 // bits of a clamped value are below the error bound), then the exponent is
 // re-biased with one addition.  |v - f| <= 2^-23 |f| inside the range; below
@@ -1497,7 +1497,7 @@ __device__ __forceinline__ bool chain_run(const ChainArgs &a, int p_begin, int p
         if (*exact_count) atomicAdd(c + CNT_EXACT, (unsigned long long)*exact_count);
         if (worst[0]) atomicMax(c + CNT_MAXRES_BITS, worst[0]);
         if (worst[1]) atomicMax(c + CNT_MAXVIOL_BITS, worst[1]);
-        if (failed) atomicOr(c + CNT_ERROR, ERR_TMA_TIMEOUT);
+        if (failed) atomicOr(c + CNT_ERROR, ERR_WAIT_TIMEOUT);
     }
     return failed;
 }
@@ -1520,8 +1520,9 @@ __global__ void __launch_bounds__(BD, (chain_min_ctas<BD, EPT>())) achr_chain_ke
 // Many models of one configuration in one persistent launch: each CTA takes
 // the next (model, first chain, end chain) item of a device work queue until
 // the queue is empty.  The host orders the items longest model first, with
-// tiles that shrink towards the end of the queue, and sets the residual-form
-// reprojection off (its shared memory is not part of this launch).  When a
+// tiles that shrink towards the end of the queue, and gives each model's
+// residual-form reprojection room for z beside the header (extra_smem) or in
+// turns (z_rows), or sets the form off.  When a
 // model's last chain is done, its finish time (globaltimer, ns) goes to
 // done_ns[model].
 template <int BD, int EPT>

@@ -25,7 +25,7 @@ enum CounterSlot {
 };
 
 enum DeviceError : unsigned long long {
-    ERR_TMA_TIMEOUT = 1ull,
+    ERR_WAIT_TIMEOUT = 1ull,  // the chain kernel's bounded wait ran out (the failure test), or a warmup index out of range
     ERR_TC_TIMEOUT = 2ull,  // a tensor-core GEMM pipeline wait expired
     ERR_DEFER_DIVERGED = 4ull,  // a deferred reprojection ended with max|S x| > residual_tol
 };
@@ -43,7 +43,7 @@ struct ChainArgs {
     const float2 *bnd;          // np: (lb, ub) rounded to FP32, infinite bounds as -+3e38; padding (-1, 1)
     int bound_exact;            // 1: every bound is finite and exact in FP32, so bnd holds the bounds themselves
     float bound_err;            // max |lb - float(lb)|, |ub - float(ub)| over finite bounds, rounded up
-    float dtol_hi, dtol_lo;     // FP32 brackets of d_tol (1 +- 2^-20)
+    float dtol_hi;              // d_tol in FP32, rounded up (1 + 2^-20)
     float utol32, mmt32;        // u_tol and max_min_tol in FP32
     // merged_ab = 1: the FP32 ratio-test brackets are formed in the same pass as
     // d, before the block knows ||d||, with the candidacy threshold bounded by
@@ -129,15 +129,10 @@ enum SegFlag : unsigned {
     SEG_CORR = 32u,     // the next launch subtracts the passes' accumulated correction from the point
 };
 
-// FP32 rounding of a double toward +inf / -inf (host side).
+// FP32 rounding of a double toward +inf (host side).
 inline float f32_up(double v) {
     float f = (float)v;
     if ((double)f < v) f = nextafterf(f, __builtin_huge_valf());
-    return f;
-}
-inline float f32_down(double v) {
-    float f = (float)v;
-    if ((double)f > v) f = nextafterf(f, -__builtin_huge_valf());
     return f;
 }
 

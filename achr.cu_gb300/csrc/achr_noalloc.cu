@@ -297,7 +297,6 @@ extern "C" achr_status achr_sample_noalloc(const achr_device_model *m, const ach
     a.bnd = sv.bnd;
     a.bound_err = berr;
     a.dtol_hi = achr::f32_up(opt.d_tol) * (1.0f + 9.5367431640625e-07f);
-    a.dtol_lo = achr::f32_down(opt.d_tol) * (1.0f - 9.5367431640625e-07f);
     a.utol32 = (float)opt.u_tol;
     a.mmt32 = (float)opt.max_min_tol;
     // Brackets formed with the direction when the box bounds ||d|| (every point
@@ -340,8 +339,8 @@ extern "C" achr_status achr_sample_noalloc(const achr_device_model *m, const ach
     unsigned long long c[achr::CNT_SLOTS];
     NOALLOC_TRY(cudaMemcpyAsync(c, sv.counters, sizeof c, cudaMemcpyDeviceToHost, s));
     NOALLOC_TRY(cudaStreamSynchronize(s));
-    if (c[achr::CNT_ERROR] & achr::ERR_TMA_TIMEOUT)
-        return fail(ACHR_ERR_TIMEOUT, "a warmup-column copy did not complete within its wait limit");
+    if (c[achr::CNT_ERROR] & achr::ERR_WAIT_TIMEOUT)
+        return fail(ACHR_ERR_TIMEOUT, "the chain kernel's bounded wait ran out");
     if (!stats) return ACHR_OK;
     std::memset(stats, 0, sizeof *stats);
     stats->accepted = (int64_t)c[achr::CNT_ACCEPTED];

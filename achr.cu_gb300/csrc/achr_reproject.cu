@@ -13,9 +13,10 @@
 //   2. z = B r as one tensor-core GEMM over all chains, with B split the same
 //      way and the three leading split products (Bh rh + Bh rl + Bl rh)
 //      accumulated in FP32 (achr_tc_gemm.cu);
-//   3. x <- clip(x - S^T z) in FP64 sparse, the same clip the reference applies
-//      after reprojecting (correctBounds, :193-206, :347-350), and the chain's
-//      centre accumulator follows the point.
+//   3. x <- clip(x - S^T z), the sparse sum in double-float on the FP32 pipes
+//      (z itself is FP32) and the subtraction in FP64, the same clip the
+//      reference applies after reprojecting (correctBounds, :193-206,
+//      :347-350); the chain's centre accumulator follows the point.
 //
 // The low-precision GEMM only ever sees the residual, so its relative error
 // (about 2^-16 times the condition number of S S^T on its range) multiplies
@@ -308,8 +309,8 @@ achr_status build_reproj(achr_ctx *ctx, ReprojState &R, bool want_pinv32, const 
     REPROJ_TRY(R.ch.upload(ch.data(), ch.size()));
     REPROJ_TRY(R.cl.upload(cl.data(), cl.size()));
 
-    // B = (S S^T)^+ from the eigen-decomposition of S S^T, eigenvalues below
-    // m * lambda_max * 2.2204e-16 dropped (the reference's null-space cutoff
+    // B = (S S^T)^+, from `eig` or from the eigen-decomposition of S S^T, eigenvalues
+    // below m * lambda_max * 2.2204e-16 dropped (the reference's null-space cutoff
     // rule, ACHRCuda.cu:478-487, applied to S S^T).
     DevBuf<double> B;
     cublasHandle_t cb = nullptr;
@@ -531,7 +532,7 @@ achr_status achr_reproject_batch(achr_ctx *ctx, int32_t n_points, double *d_poin
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> gemm_ev;
     std::vector<double> chunk_flops((size_t)nchunks, 0.0);
     // Round r, chunk c: residual + split, then (gated on that chunk's residual
-    // exceeding residual_tol) the tensor-core GEMM and the FP64 correction.
+    // exceeding residual_tol) the tensor-core GEMM and the correction.
     for (int r = 0; r < max_rounds; ++r) {
         for (int c = 0; c < nchunks; ++c) {
             const int c0 = c * chunk;

@@ -455,15 +455,12 @@ __global__ void __launch_bounds__(512)
     }
     __syncthreads();
     // log det M = 2 sum log L_kk, in the order of 1024 strided sums
-    float ld = 0.0f;
     for (int v = tid; v < 1024; v += nt) {
         float x = 0.0f;
         for (int k = v; k < r; k += 1024) x += logf(Lw[(long long)k * r + k]);
         for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
         if ((v & 31) == 0) red[v >> 5] = x;
-        ld = x;
     }
-    (void)ld;
     __syncthreads();
     if (tid == 0) {
         float t = 0.0f;

@@ -94,8 +94,9 @@ typedef struct {
                                     the context has been short of memory for as many chains; the forms
                                     agree to rounding, not bit for bit, so name 1 or 3 where a chain's
                                     points must not depend on how chains are split over calls.  Deferred
-                                    runs of one context take turns; their buffers, about 24 n_rxns +
-                                    20 n_mets bytes per chain, stay with it,
+                                    runs of one context take turns (replays of a captured one are for the
+                                    program to order); their buffers, about 24 n_rxns + 20 n_mets bytes
+                                    per chain, stay with it,
                                  1: N (N^T x) in FP64 in the chain kernel,
                                  2: x - S^T (S S^T)^+ S x in the chain kernel, the pseudo-inverse product
                                     in FP32 on the residual (equal in exact arithmetic; m^2 FP32 instead
@@ -350,9 +351,12 @@ typedef struct achr_reproj_stats {
  * d_centre_acc is non-NULL, same layout) move with the points.  Up to
  * max_rounds (1..16) passes; a block of chains whose max |S x| is already
  * within opt.residual_tol is left as it is.  Equals the reference's N (N^T x) followed by its clip; the
- * residual S x and the update are FP64, the dense (S S^T)^+ product runs on
- * the tensor cores as three BF16 split products with FP32 accumulation.  The
- * operator is built on the first call (FP64 eigen-decomposition of S S^T).
+ * residual S x is FP64, the dense (S S^T)^+ product runs on the tensor cores
+ * as three BF16 split products with FP32 accumulation, and S^T times that FP32
+ * product is summed in double-float (about 48 bits) and subtracted in FP64.
+ * The operator is built with the context where its runs will want it, else on
+ * the first call (FP64 eigen-decomposition of S^T S or S S^T).  A point with a
+ * NaN or an infinity leaves NaN, its chain alone.
  * Synchronises `stream`. */
 achr_status achr_reproject_batch(achr_ctx *ctx, int32_t n_points, double *d_points, double *d_centre_acc,
                                  int64_t ld, int32_t max_rounds, void *stream, achr_reproj_stats *stats);
@@ -471,7 +475,7 @@ typedef struct {
  * N (N^T x) in FP64 (reproject_form 2 or 3 gives ACHR_ERR_UNSUPPORTED); in
  * ACHR_MODE_FEASIBLE only the final projection of emitted points is applied
  * (the warmup points are used as given).  Synchronises the stream and reports
- * an expired column wait as ACHR_ERR_TIMEOUT; stats->kernel_ms is 0. */
+ * an expired wait as ACHR_ERR_TIMEOUT; stats->kernel_ms is 0. */
 achr_status achr_sample_noalloc(const achr_device_model *model, const achr_options *opt, uint64_t seed,
                                 uint64_t chain_offset, int32_t n_points, int32_t n_steps, double *d_points_out,
                                 int64_t ld_out, void *stream, achr_stats *stats);
