@@ -1024,13 +1024,13 @@ achr_status achr_autotune(achr_ctx *ctx, int32_t *threads_per_chain_out) {
     const ChainArgs probe = chain_args(ctx, 0, 0, 0, 0, nullptr, 0);
     const bool residual = probe.pinv32 && ctx->opt.check_period > 0;
     auto takes = [&](int threads) {
-        int per_sm = 0;
-        const cudaError_t e = achr::launch_chains(probe, threads, nullptr, 0, &per_sm);
+        achr::ChainFit fit;
+        const cudaError_t e = achr::launch_chains(probe, threads, nullptr, 0, &fit);
         if (e != cudaSuccess) (void)cudaGetLastError();
-        return e == cudaSuccess && (!residual || per_sm > 0);
+        return e == cudaSuccess && (!residual || fit.turn > 0);
     };
     const int scratch = std::max(probe.m, probe.d);
-    const bool long_scratch = scratch > achr::chain_scratch_doubles(256, 30);
+    const bool long_scratch = scratch > achr::kScratch256x30;
     const std::pair<int, int> key(4 * achr::chain_padded_length(ctx->n, 0) + (long_scratch ? 2 : 0) + (residual ? 1 : 0),
                                   dev);
     int cand[8];
@@ -1159,7 +1159,7 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
                 extra = 0;
                 for (int k : G.models) {  // z takes turns beside the residual, or the form is off
                     ChainArgs &a = args[(size_t)k];
-                    a.z_rows = achr::residual_z_rows(a.m, achr::chain_scratch_doubles(G.bd, G.ept));
+                    a.z_rows = achr::residual_z_rows(a.m, achr::cfg_scratch({G.bd, G.ept, false}));
                     if (!a.z_rows) a.pinv32 = nullptr;
                 }
             }

@@ -3,15 +3,15 @@
 
 namespace achr {
 
-cudaError_t launch_chain_cfg_mid(int bd, int ept, const ChainArgs &a, cudaStream_t s, int max_ctas, int *per_sm) {
+cudaError_t launch_chain_cfg_mid(int bd, int ept, const ChainArgs &a, cudaStream_t s, int max_ctas, ChainFit *fit) {
     switch (bd * 100 + ept) {
-        case 128 * 100 + 4: return launch_cfg<128, 4>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 8: return launch_cfg<128, 8>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 12: return launch_cfg<128, 12>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 16: return launch_cfg<128, 16>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 20: return launch_cfg<128, 20>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 24: return launch_cfg<128, 24>(a, s, max_ctas, per_sm);
-        case 128 * 100 + 32: return launch_cfg<128, 32>(a, s, max_ctas, per_sm);
+        case 128 * 100 + 4: return launch_cfg<128, 4>(a, s, max_ctas, fit);
+        case 128 * 100 + 8: return launch_cfg<128, 8>(a, s, max_ctas, fit);
+        case 128 * 100 + 12: return launch_cfg<128, 12>(a, s, max_ctas, fit);
+        case 128 * 100 + 16: return launch_cfg<128, 16>(a, s, max_ctas, fit);
+        case 128 * 100 + 20: return launch_cfg<128, 20>(a, s, max_ctas, fit);
+        case 128 * 100 + 24: return launch_cfg<128, 24>(a, s, max_ctas, fit);
+        case 128 * 100 + 32: return launch_cfg<128, 32>(a, s, max_ctas, fit);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -1571,9 +1571,10 @@ inline cudaError_t allow_smem(const void *kernel, size_t need) {
 // Occupancy-sized persistent launch of one configuration.  max_ctas > 0 caps
 // the grid.
 template <int BD, int EPT, bool SEG>
-cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int max_ctas, int *per_sm_out) {
+cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int max_ctas, ChainFit *fit) {
     auto *const KFN = achr_chain_kernel<BD, EPT, SEG>;
     ChainArgs a = a_in;
+    const int turn = a.z_rows;  // > 0: the rows of z per turn that this launch has to take
     a.z_rows = 0;
     const size_t base = chain_smem_bytes_cfg<BD, EPT>();
     // The residual-form reprojection keeps z (m floats) in shared memory and
@@ -1584,7 +1585,6 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
     const size_t zbytes = ((size_t)a.m * sizeof(float) + 15) & ~(size_t)15;
     // (its residual takes the accumulator's place while that waits in registers: m <= ldw <= NP)
     if (a.pinv32 && a.m > a.ldw) a.pinv32 = nullptr;
-    const bool asked = a.pinv32 != nullptr;
     size_t smem = base + (a.pinv32 ? zbytes : 0);
     cudaError_t e = allow_smem(reinterpret_cast<const void *>(KFN), std::max(smem, base));
     if (e != cudaSuccess) return e;
@@ -1595,14 +1595,30 @@ cudaError_t launch_cfg_kernel(const ChainArgs &a_in, cudaStream_t stream, int ma
         int per_sm_z = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_z, KFN, BD, smem);
         if (e != cudaSuccess) return e;
-        if (per_sm_z < per_sm) {
+        if (per_sm_z < per_sm || (turn > 0 && turn < a.m)) {
             a.z_rows = residual_z_rows(a.m, chain_acc_doubles<BD, EPT>());
-            if (!a.z_rows) a.pinv32 = nullptr;
-            smem = base;
+            if (turn > 0) {
+                if (a.z_rows >= turn) {
+                    a.z_rows = turn;
+                } else if (turn == a.m && per_sm_z > 0) {  // all of z at once, in memory of its own
+                    a.z_rows = 0;
+                    per_sm = per_sm_z;
+                } else {
+                    return cudaErrorInvalidConfiguration;  // (the caller's rule has ruled it out)
+                }
+            }
+            if (a.z_rows) smem = base;
+            else if (turn == 0) {
+                a.pinv32 = nullptr;
+                smem = base;
+            }
         }
     }
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    if (per_sm_out) *per_sm_out = asked && !a.pinv32 ? -per_sm : per_sm;  // < 0: without the residual form
+    if (fit) {
+        fit->per_sm = per_sm;
+        fit->turn = a.pinv32 ? (a.z_rows ? a.z_rows : a.m) : 0;
+    }
     if (a.P <= 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -1643,9 +1659,9 @@ cudaError_t launch_queue_cfg(const ChainQueue &q, cudaStream_t stream, int grid,
 // Occupancy-sized persistent launch of one configuration (segmented launches
 // take the kernel's segmented instantiation).
 template <int BD, int EPT>
-cudaError_t launch_cfg(const ChainArgs &a, cudaStream_t stream, int max_ctas, int *per_sm_out) {
-    return a.seg ? launch_cfg_kernel<BD, EPT, true>(a, stream, max_ctas, per_sm_out)
-                 : launch_cfg_kernel<BD, EPT, false>(a, stream, max_ctas, per_sm_out);
+cudaError_t launch_cfg(const ChainArgs &a, cudaStream_t stream, int max_ctas, ChainFit *fit) {
+    return a.seg ? launch_cfg_kernel<BD, EPT, true>(a, stream, max_ctas, fit)
+                 : launch_cfg_kernel<BD, EPT, false>(a, stream, max_ctas, fit);
 }
 
 }  // namespace achr

@@ -5,6 +5,8 @@
 
 #include <cmath>
 
+#include "achr_chain_rule.h"
+
 namespace achr {
 
 // Counters kept in device memory while a sampling launch runs.
@@ -158,34 +160,26 @@ inline void set_merged_bound(ChainArgs &a, double u_tol, double dnorm_max) {
 }
 
 // Launch the persistent chain kernel; threads_per_chain = 0 picks the default
-// configuration for n.  max_ctas > 0 caps the grid; per_sm (if non-NULL)
-// receives the resident CTAs per SM of the configuration (negative: too many to
-// leave room for the residual-form reprojection that `a` asks for).  a.np is the length
-// the per-reaction arrays were padded to (>= the configuration's BD * EPT).
+// configuration for n, or for few chains one with more threads (achr_chain_rule.h).
+// max_ctas > 0 caps the grid.  a.np is the length the per-reaction arrays were padded
+// to (>= the configuration's BD * EPT); a.z_rows is the launch's own.
+struct ChainFit {
+    int per_sm = 0;  // resident CTAs per SM of the configuration
+    int turn = 0;    // rows of z per turn of the residual-form reprojection; 0: not asked for, or no room for it
+};
 cudaError_t launch_chains(const ChainArgs &a, int threads_per_chain, cudaStream_t stream, int max_ctas = 0,
-                          int *per_sm = nullptr);
+                          ChainFit *fit = nullptr);
 
 // Configuration ladder: threads per chain and padded element count for n
 // reactions (threads_per_chain = 0: default); 0 if no configuration fits.
 int chain_block_size(int n, int threads_per_chain);
 // Configuration (threads, elements per thread) a batch runs the model with.
-int chain_scratch_doubles(int bd, int ept);  // the accumulator's share of shared memory
-// Rows of z = (S S^T)^+ r that fit beside r (m float pairs) in `scratch` doubles; 0
-// where that would take more than eight turns.
-inline int residual_z_rows(int m, int scratch) {
-    const int rows = 2 * (scratch - m);
-    return rows <= 0 || (long long)rows * 8 < m ? 0 : rows < m ? rows : m;
-}
 bool chain_config(const ChainArgs &a, int threads_per_chain, int *bd, int *ept);
 // Whether a caller may ask for this many threads per chain at n reactions (the
 // defaults and the autotuner also use longer configurations of a thread count).
 bool chain_takes_threads(int n, int threads_per_chain);
 // Persistent work-queue launch of the configuration (bd, ept); see ChainQueue.
 cudaError_t launch_chain_queue(int bd, int ept, const ChainQueue &q, cudaStream_t stream, int grid, int *per_sm);
-int chain_padded_length(int n, int threads_per_chain);
-// Length to pad per-reaction arrays to: twice the default padded length (so
-// every autotuning candidate fits), at most 16384.
-int chain_alloc_length(int n);
 // Threads-per-chain values worth timing for n (padded length within max_np), of
 // the configurations that hold a reprojection's scratch (max(m, d) doubles).
 int chain_candidates(int n, int max_np, int scratch, int *bds, int cap);
