@@ -228,7 +228,9 @@ extern "C" achr_status achr_sample_noalloc(const achr_device_model *m, const ach
         return fail(ACHR_ERR_UNSUPPORTED,
                     "achr_sample_noalloc reprojects as N (N^T x) in FP64; the residual and deferred forms "
                     "(reproject_form 2 and 3) need a pseudo-inverse of S S^T and buffers that only a context builds");
-    const int np = achr::chain_padded_length(n, opt.threads_per_chain);
+    // room for the configurations that a launch of few chains takes (as a context has), or the asked one's length
+    const int np = opt.threads_per_chain == 0 ? achr::chain_alloc_length(n, kMaxRxns)
+                                              : achr::chain_padded_length(n, opt.threads_per_chain);
     if (np == 0 || np > kMaxRxns || !achr::chain_takes_threads(n, opt.threads_per_chain))
         return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for this size");
     const int prep_blocks = (np + kPrepThreads - 1) / kPrepThreads;

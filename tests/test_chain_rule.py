@@ -63,3 +63,12 @@ def test_any_size(lib):
                         if c != d:
                             assert c // 100 > d // 100 and per_sm * (c // 3200) <= 16
                             assert turn == 0 or turn == m or lib.room(c, m) >= turn
+
+
+def test_room_without_allocation(lib):
+    """achr_sample_noalloc's arrays hold 8192 reactions at most: what fits them is what a context would take."""
+    for n in [*range(1, 8193, 41), 1060, 2500, 7680, 8192]:
+        for per_sm in (1, 2, 4):
+            want = lib.few(n, lib.alloc(n, 16384), 0, 0, 0, per_sm)
+            assert _np(want) > 8192 or lib.few(n, lib.alloc(n, 8192), 0, 0, 0, per_sm) == want
+    assert lib.few(1060, lib.alloc(1060, 8192), 0, 0, 0, 1) == 51204
