@@ -1098,6 +1098,9 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
     std::vector<ChainArgs> args((size_t)n_models);
     std::vector<double> chain_time((size_t)n_models);
     std::vector<int> cfg_key((size_t)n_models);
+    long long chains = 0;
+    for (int k = 0; k < n_models; ++k) chains += std::max(n_points[k], 0);
+    const int chains_per_sm = (int)std::min((chains + sms - 1) / sms, 1ll << 20);
     uint64_t off = 0;
     for (int k = 0; k < n_models; ++k) {
         achr_ctx *c = ctxs[k];
@@ -1106,7 +1109,7 @@ achr_status achr_sample_batch(achr_ctx *const *ctxs, int32_t n_models, const int
         int bd = 0, ept = 0;
         // disjoint chain ids: model k uses ids off .. off + P_k - 1
         args[(size_t)k] = chain_args(c, seed, off, n_points[k], n_steps, d_points_out[k], ld_out[k]);
-        if (!achr::chain_config(args[(size_t)k], c->opt.threads_per_chain, &bd, &ept) || bd * ept > c->np)
+        if (!achr::chain_config(args[(size_t)k], c->opt.threads_per_chain, chains_per_sm, &bd, &ept) || bd * ept > c->np)
             return fail(ACHR_ERR_UNSUPPORTED, "no chain-kernel configuration for batch entry " + std::to_string(k));
         cfg_key[(size_t)k] = bd * 100 + ept;
         off += (uint64_t)n_points[k];

@@ -80,10 +80,14 @@ bool chain_takes_threads(int n, int threads_per_chain) {
     return threads_per_chain == 0 || n <= most;
 }
 
-bool chain_config(const ChainArgs &a, int threads_per_chain, int *bd, int *ept) {
-    const ChainCfg *c = find_cfg(a.n, threads_per_chain, a.m > a.d ? a.m : a.d);
+bool chain_config(const ChainArgs &a, int threads_per_chain, int chains_per_sm, int *bd, int *ept) {
+    const int scratch = a.m > a.d ? a.m : a.d;
+    const ChainCfg *c = find_cfg(a.n, threads_per_chain, scratch);
     int turn = 0;
-    if (c && threads_per_chain == 0 && residual_form(a) && find_cfg_residual(a, &c, &turn) != cudaSuccess) return false;
+    if (c && threads_per_chain == 0) {
+        if (!residual_form(a)) c = few_chains_cfg(c, a.n, a.np, a.m, scratch, 0, chains_per_sm);
+        else if (find_cfg_residual(a, &c, &turn) != cudaSuccess) return false;
+    }
     if (!c) return false;
     *bd = c->bd;
     *ept = c->ept;
