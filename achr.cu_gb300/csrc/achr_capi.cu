@@ -827,7 +827,7 @@ ChainArgs chain_args(const achr_ctx *ctx, uint64_t seed, uint64_t chain_offset, 
     a.mmt32 = (float)ctx->opt.max_min_tol;
     set_merged_bound(a, ctx->opt.u_tol, ctx->opt.bracket_pass == 1 ? INFINITY
                                         : ctx->n_dirs > 0           ? ctx->dir_norm_max
-                                                                    : 2.0 * ctx->box_norm);
+                                                                    : achr::box_dnorm_max(ctx->box_norm, ctx->opt.u_tol, ctx->n));
     a.row_ptr = ctx->rowptr.p;
     a.col_idx = ctx->colidx.p;
     a.val = ctx->val.p;

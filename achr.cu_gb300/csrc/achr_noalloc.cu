@@ -304,7 +304,7 @@ extern "C" achr_status achr_sample_noalloc(const achr_device_model *m, const ach
     // Brackets formed with the direction when the box bounds ||d|| (every point
     // and centre lies in it: ||w - c|| <= 2 sqrt(sum max(lb^2, ub^2))), as the
     // allocating path does; infinite bounds or bracket_pass = 1 keep a separate pass.
-    achr::set_merged_bound(a, opt.u_tol, opt.bracket_pass == 1 ? INFINITY : 2.0 * std::sqrt(box_sq));
+    achr::set_merged_bound(a, opt.u_tol, opt.bracket_pass == 1 ? INFINITY : achr::box_dnorm_max(std::sqrt(box_sq), opt.u_tol, n));
     // The residual check reads the caller's CSR rows directly (the allocating
     // path reads a sliced-ELL copy it builds; the sums are the same).
     a.row_ptr = m->row_ptr;

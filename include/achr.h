@@ -128,8 +128,9 @@ typedef struct {
     int32_t bracket_pass;     /* FP32 ratio-test brackets (ACHRCuda.cu:266-281): 0: formed in the same pass
                                  as the direction, before its norm is known, with the candidacy threshold
                                  bounded through the box (or the longest hit-and-run direction); a step
-                                 whose threshold exceeds the bound, or a model with an infinite bound,
-                                 uses a separate pass.  1: always a separate pass.  Results are equal. */
+                                 whose threshold exceeds the bound, a model with an infinite bound, or one
+                                 with u_tol sqrt(n_rxns) > 1.5e-4 (no directions), uses a separate pass.
+                                 1: always a separate pass.  Results are equal. */
     int32_t reprojection_passes; /* most passes of one deferred reprojection, 1..8 (0: 8); a chain still
                                     above residual_tol after the last pass is an ACHR_ERR_NUMERIC */
 } achr_options;
