@@ -11,6 +11,9 @@ namespace achr {
 //   n = 400, d = 84:   P = 1000 1.08 / 0.87,    5000 5.19 / 2.23   (3.4e7, 1.7e8)
 //   n = 1060, d = 159: P = 1000 3.92 / 1.61,    5000 19.9 / 5.62
 // Models of n d >= 2.5e5 are always deferred.
+// Neither side of the line is the less exact one by being deferred: against a projection refined in
+// 128-bit floating point a deferred point's rms error is 2e-14 to 4e-14 for 95 to 1060 reactions,
+// N (N^T x) in the kernel 6e-14 to 6e-13.
 constexpr double kDeferWork = 2.0e7, kDeferModel = 2.5e5;
 
 enum class DeferUse {
